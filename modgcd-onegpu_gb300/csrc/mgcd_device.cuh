@@ -1,10 +1,9 @@
 // mgcd_device.cuh -- device arithmetic of the modular GCD kernels (sm_103a).
 //
 // Per-modulus arithmetic is done in Montgomery form with R = 2^32 (REDC), and modular
-// inverses by the extended Euclidean algorithm with float-reciprocal quotient estimates
-// followed by an exact integer correction.  Everything here is bit-exact integer math;
-// floats only ever produce a quotient estimate that is corrected, and every inverse is
-// checked (x * x^-1 == 1) before it is used.
+// inverses by the extended Euclidean algorithm with float-reciprocal quotient estimates.
+// Every result is bit-exact: floats hold integers exactly or only choose a quotient, and
+// every inverse is checked (x * x^-1 == 1) before it is used.
 #pragma once
 #include <cstdint>
 
@@ -82,80 +81,113 @@ static __device__ __noinline__ uint32_t inv_mod_slow(uint32_t x, uint32_t q)
   return (uint32_t)(s0 < 0 ? s0 + q : s0);
 }
 
-// Quotient estimates of inv_mod's Euclid steps (also run by the certification kernel).
-// Phase A (2^22 <= r1 < r0 < 2^32): nearest integer to r0 / r1 from a float reciprocal.
-__device__ __forceinline__ uint32_t inv_quot_a(uint32_t r0, uint32_t r1)
-{
-  return __float2uint_rn(__fmul_rn(__uint2float_rn(r0), rcp_approx(__uint2float_rn(r1))));
-}
-
-// Phase C (r1 < r0 < 2^22, both exact in float): Q = rint(f0 * rcp(f1)) read from the
-// mantissa of Q + 1.5 * 2^23; returns the float whose low mantissa bits hold Q.
+// Quotient estimate of the inverse's Euclid steps (also run by the certification kernel):
+// Q = rint(f0 / f1), |Q| < 2^22, read from the mantissa of f0 * rcp(f1) + 1.5 * 2^23; returns
+// the float whose low mantissa bits hold Q.
 constexpr float INV_MAGIC = 12582912.0f;     // 1.5 * 2^23
-constexpr uint32_t INV_MAGIC_BITS = 0x4B400000u;
-__device__ __forceinline__ float inv_quot_c(float f0, float f1)
+__device__ __forceinline__ float inv_quot(float f0, float f1)
 {
   return __fmaf_rn(f0, rcp_approx(f1), INV_MAGIC);
 }
 
-// x^{-1} mod q for 0 < x < q, q an odd prime < 2^32.
-//
-// Extended Euclid on (r0, r1) = (q, x) with nearest-integer quotients (remainders of
-// either sign, their magnitudes kept; about 13 steps for 32-bit operands instead of 19),
-// tracking the cofactor s_k modulo 2^32 with s_k * x == r_k (mod q):
-//   phase A (r1 >= 2^22): operands rounded to float, quotient < 2^10, estimate within
-//            2^-11 of r0/r1, so the rounded quotient is within 1 of it and |r| < r1;
-//   phase B (r0 >= 2^22 > r1): one exact integer division at the transition;
-//   phase C (|r0|, |r1| < 2^22): operands exact in float, quotient below 2^22 in magnitude
-//            and within 1/2 of r0/r1 before rounding, remainder exact by FMA (an integer
-//            below 2^22 in magnitude); remainders and quotients keep their signs.
-// The bounds assume rcp.approx.ftz.f32's documented error (1 ulp).  At the end |s| < q,
-// so s is either the 32-bit value read as unsigned or that minus 2^32 (possible only for
-// q > 2^31); the candidate whose product with x is 1 is taken, and if neither is (never
-// observed), the integer-only routine recomputes it, so no float error can reach a result.
+// One Euclid step (f0, s0) -= Q (f1, s1) where `on`; the caller alternates the roles.
+__device__ __forceinline__ void inv_step(float& f0, float f1, float& s0, float s1, bool on)
+{
+  const float nq = INV_MAGIC - inv_quot(f0, f1);
+  if (on) {
+    f0 = __fmaf_rn(nq, f1, f0);
+    s0 = __fmaf_rn(nq, s1, s0);
+  }
+}
+
+// Euclid steps on (f0, f1) with cofactors (s0, s1) while both remainders are above `lim` in
+// magnitude (a lane that is done keeps its values through the rest of a trip: predicated
+// steps, two to a branch).
+__device__ __forceinline__ void inv_steps(float& f0, float& f1, float& s0, float& s1, float lim)
+{
+  bool on = fabsf(f0) > lim && fabsf(f1) > lim;
+#pragma unroll 1
+  while (on) {
+    inv_step(f0, f1, s0, s1, on);
+    on = fabsf(f0) > lim;
+    inv_step(f1, f0, s1, s0, on);
+    on = on && fabsf(f1) > lim;
+  }
+}
+
+// s with s x == +-1 (mod q), as a signed value modulo 2^32, for 0 < x < q, q an odd prime:
+// extended Euclid on (q, x) with nearest-integer quotients (remainders of either sign; about
+// 13 steps for 32-bit operands, 10.7 for 27, 8.7 for 22), every step in floats.
+//   1. On the operands rounded to float (f = r + e).  A remainder is a multiple of its
+//      divisor's ulp and below it in magnitude, so each step is exact: it is the Euclid of
+//      the rounded operands, and its steps are a unimodular map of the true ones.  The
+//      cofactors s stay below q / lim in magnitude, so a true remainder is within
+//      2^-24 q (2 q / lim) of its float: it stops once the smaller one is below lim.
+//   2. The two remainders r = S x - A q exactly, modulo 2^32, A = rint((S x - f) / q) (S x =
+//      r + A q: the estimate is off by |e| / q plus rounding, far below 1/2), and one step on
+//      them in integers, since the larger one may be far above lim: Q from the float of the
+//      larger, so |r2| <= |r1| / 2 + |e| + 2^-22 q.
+//   3. The rest exactly: r1, r2 < 2^22 (LIM22: lim = 2^22, q < 2^32; 2^18, q < 2^30), so
+//      remainders and cofactors are exact in float.  Only r2's cofactor B is carried; r1's is
+//      A = (1 - B r2) / r1, exact to the nearest integer below 2^20 and put right by one
+//      integer step above.
+// Moduli below 2^22 are exact in float from the start and need only 3.
+// What bounds it: instruction issue (87 % of the issue slots in a full SM).  Against the
+// version with integer remainders above 2^22 and integer cofactors, in a loop of dependent
+// inverses: 483 -> 303 issue slots per warp and 2,033 -> 1,458 cycles latency at 32 bits,
+// 314 -> 258 and 1,395 -> 1,198 at 27, 241 -> 172 and 1,101 -> 844 at 22.
+template <bool LIM22>
+__device__ __forceinline__ uint32_t inv_euclid(uint32_t x, uint32_t q)
+{
+  const float fq = __uint2float_rn(q), fx = __uint2float_rn(x);
+  float g0 = fq, g1 = fx, b0 = 0.0f, b1 = 1.0f;
+  if (!LIM22 && q < (1u << 22)) {
+    inv_steps(g0, g1, b0, b1, 1.0f);
+    const bool z = fabsf(g0) == 1.0f;
+    return (uint32_t)__float2int_rn((z ? g0 : g1) * (z ? b0 : b1));
+  }
+  constexpr float lim = LIM22 ? 4194304.0f : 262144.0f;
+  inv_steps(g0, g1, b0, b1, lim);
+  const bool sw = fabsf(g0) < fabsf(g1);
+  const float fb = sw ? g1 : g0, fs = sw ? g0 : g1, sb = sw ? b1 : b0, ss = sw ? b0 : b1;
+  const float iq = rcp_approx(fq);
+  const uint32_t S0 = (uint32_t)__float2int_rn(sb), S1 = (uint32_t)__float2int_rn(ss);
+  const uint32_t A0 = (uint32_t)__float2int_rn(__fmaf_rn(sb, fx, -fb) * iq);
+  const uint32_t A1 = (uint32_t)__float2int_rn(__fmaf_rn(ss, fx, -fs) * iq);
+  const uint32_t r1 = S1 * x - A1 * q;
+  g0 = __int2float_rn((int32_t)r1);
+  const uint32_t Q = (uint32_t)__float2int_rn(fb * rcp_approx(g0));
+  const uint32_t r2 = S0 * x - A0 * q - Q * r1;
+  const uint32_t S2 = S0 - Q * S1;
+  g1 = __int2float_rn((int32_t)r2);
+  b0 = 0.0f;
+  b1 = 1.0f;
+  inv_steps(g0, g1, b0, b1, 1.0f);
+  const bool z = fabsf(g0) == 1.0f;
+  const float b = (z ? g0 : g1) * (z ? b0 : b1);
+  const float i1 = rcp_approx(__int2float_rn((int32_t)r1));
+  const uint32_t B = (uint32_t)__float2int_rn(b);
+  uint32_t A = (uint32_t)__float2int_rn(__fmaf_rn(-b, __int2float_rn((int32_t)r2), 1.0f) * i1);
+  if (LIM22) A -= (uint32_t)__float2int_rn(__int2float_rn((int32_t)(A * r1 + B * r2 - 1u)) * i1);
+  return A * S1 + B * S2;
+}
+
+// x^{-1} mod q for 0 < x < q, q an odd prime < 2^32 (inv_euclid).  |s| < q, so s is either
+// the 32-bit value read as unsigned or that minus 2^32 (possible only for q > 2^31); the
+// candidate whose product with x is 1 is taken, and if neither is (never observed), the
+// integer-only routine recomputes it, so no float error can reach a result.
 __device__ __forceinline__ uint32_t inv_mod(uint32_t x, uint32_t q, uint32_t qinv)
 {
-  uint32_t r0 = q, r1 = x, s0 = 0, s1 = 1;
-  while (r1 >= (1u << 22)) {
-    const uint32_t Q = inv_quot_a(r0, r1);
-    const uint64_t m = (uint64_t)Q * r1;
-    const bool neg = m > r0;
-    const uint32_t d = r0 - (uint32_t)m;        // r0 - Q r1 modulo 2^32, |r0 - Q r1| < r1
-    const uint32_t s = s0 - Q * s1;
-    r0 = r1; s0 = s1;
-    r1 = neg ? 0u - d : d;
-    s1 = neg ? 0u - s : s;
-  }
-  if (r1 > 1u) {
-    if (r0 >= (1u << 22)) {
-      const uint32_t Q = r0 / r1;
-      const uint32_t r = r0 - Q * r1;
-      const uint32_t s = s0 - Q * s1;
-      r0 = r1; r1 = r; s0 = s1; s1 = s;
-    }
-    // remainders keep their sign here (quotients of either sign, read from the mantissa
-    // as two's complement), so s_k x == r_k holds without a sign fix per step
-    float f0 = (float)r0, f1 = (float)r1;
-    int guard = 64;
-    while (fabsf(f1) > 1.0f && --guard) {
-      const float qm = inv_quot_c(f0, f1);
-      const float rem = __fmaf_rn(INV_MAGIC - qm, f1, f0);   // r0 - Q r1, exact
-      const uint32_t Q = __float_as_uint(qm) - INV_MAGIC_BITS;
-      const uint32_t s = s0 - Q * s1;
-      f0 = f1; s0 = s1;
-      f1 = rem; s1 = s;
-    }
-    if (f1 < 0.0f) s1 = 0u - s1;                   // s1 x == -1
-  }
+  const uint32_t s = inv_euclid<true>(x, q);
   // inv * x == 1 (mod q)  <=>  redc(inv * x) == redc(1)
   const uint32_t one = redc(1ull, q, qinv);
   if (q < 0x80000000u) {
-    const uint32_t inv = (int32_t)s1 < 0 ? s1 + q : s1;
+    const uint32_t inv = (int32_t)s < 0 ? s + q : s;
     if (redc((uint64_t)inv * x, q, qinv) == one) return inv;
   } else {
-    // candidates s1 mod q and (s1 - 2^32) mod q = that - (2^32 - q); redc of the second's
+    // candidates s mod q and (s - 2^32) mod q = that - (2^32 - q); redc of the second's
     // product with x is the first's minus x
-    const uint32_t inv = s1 >= q ? s1 - q : s1;
+    const uint32_t inv = s >= q ? s - q : s;
     const uint32_t c = redc((uint64_t)inv * x, q, qinv);
     if (c == one) return inv;
     if (mod_sub(c, x, q) == one) return mod_sub(inv, 0u - q, q);
@@ -163,67 +195,14 @@ __device__ __forceinline__ uint32_t inv_mod(uint32_t x, uint32_t q, uint32_t qin
   return inv_mod_slow(x, q);
 }
 
-// Phase A quotient of inv_mod_narrow (2^22 <= r1 < r0 < 2^30, so Q < 2^8): the nearest
-// integer to rn(r0) * rcp(rn(r1)), read from the mantissa (one rounding) instead of a
-// float-to-integer conversion; g0, g1 are the operands already converted.
-__device__ __forceinline__ uint32_t inv_quot_an(float g0, float g1)
-{
-  return __float_as_uint(__fmaf_rn(g0, rcp_approx(g1), INV_MAGIC)) - INV_MAGIC_BITS;
-}
-
-// x^{-1} mod q for 0 < x < q < 2^30 (the moduli of widths up to 30 bits): inv_mod's Euclid
-// with cheaper steps where the narrower operands allow them.
-//   phase A (r1 >= 2^22): quotient estimate as inv_quot_an, each remainder converted once;
-//            |r0 - Q r1| < r1 < 2^30, so the remainder and its sign come from 32-bit
-//            wrapping arithmetic read as signed;
-//   phase B (r0 >= 2^22 > r1): a float quotient estimate instead of an integer division.
-//            Its error is below (r0 / r1) 2^-22 + 1/2 (operand rounding 2^-24, reciprocal
-//            2^-23, product 2^-24), so the exact signed remainder r0 - Q r1 is below
-//            2^8 + r1 / 2 < 2^22 in magnitude: exact in float, as phase C requires (its
-//            first step may then see |r0| < |r1|, a quotient of 0 or +-1);
-//   phase C: inv_mod's, two steps per loop trip with the roles of the registers
-//            alternating, at most 64 steps (never reached: 22-bit operands take ~32 at most).
-// The result is checked as inv_mod's is, with the same integer-only fallback.
+// x^{-1} mod q for 0 < x < q < 2^30 (the moduli of widths up to 30 bits): the rounded
+// operands' errors are smaller, so the first part of inv_euclid goes down to 2^18.  The
+// result is checked as inv_mod's is, with the same integer-only fallback.
 __device__ __forceinline__ uint32_t inv_mod_narrow(uint32_t x, uint32_t q, uint32_t qinv)
 {
-  uint32_t r0 = q, r1 = x, s0 = 0, s1 = 1;
-  float g0 = __uint2float_rn(r0), g1 = __uint2float_rn(r1);
-  while (r1 >= (1u << 22)) {
-    const uint32_t Q = inv_quot_an(g0, g1);
-    const uint32_t d = r0 - Q * r1;
-    const uint32_t s = s0 - Q * s1;
-    const bool neg = (int32_t)d < 0;
-    r0 = r1; s0 = s1; g0 = g1;
-    r1 = neg ? 0u - d : d;
-    s1 = neg ? 0u - s : s;
-    g1 = __uint2float_rn(r1);
-  }
-  if (r1 > 1u) {
-    int32_t i0 = (int32_t)r0, i1 = (int32_t)r1;
-    if (r0 >= (1u << 22)) {
-      const uint32_t Q = __float2uint_rn(__fmul_rn(g0, rcp_approx(g1)));
-      const int32_t r = (int32_t)(r0 - Q * r1);
-      const uint32_t s = s0 - Q * s1;
-      i0 = i1; i1 = r; s0 = s1; s1 = s;
-    }
-    float f0 = (float)i0, f1 = (float)i1;
-    for (int trips = 32; trips > 0 && fabsf(f1) > 1.0f; --trips) {
-      {
-        const float qm = inv_quot_c(f0, f1);
-        f0 = __fmaf_rn(INV_MAGIC - qm, f1, f0);
-        s0 = s0 - (__float_as_uint(qm) - INV_MAGIC_BITS) * s1;
-      }
-      if (!(fabsf(f0) > 1.0f)) { f1 = f0; s1 = s0; break; }
-      {
-        const float qm = inv_quot_c(f1, f0);
-        f1 = __fmaf_rn(INV_MAGIC - qm, f0, f1);
-        s1 = s1 - (__float_as_uint(qm) - INV_MAGIC_BITS) * s0;
-      }
-    }
-    if (f1 < 0.0f) s1 = 0u - s1;                   // s1 x == -1
-  }
+  const uint32_t s = inv_euclid<false>(x, q);
   const uint32_t one = redc(1ull, q, qinv);
-  const uint32_t inv = (int32_t)s1 < 0 ? s1 + q : s1;
+  const uint32_t inv = (int32_t)s < 0 ? s + q : s;
   if (redc((uint64_t)inv * x, q, qinv) == one) return inv;
   return inv_mod_slow(x, q);
 }
