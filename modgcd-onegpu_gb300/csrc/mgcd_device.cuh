@@ -68,17 +68,21 @@ __device__ __forceinline__ float rcp_approx(float y)
   return r;
 }
 
-// Exact inverse by integer-only extended Euclid (64-bit division); the fallback that
-// runs only if the fast routine's self-check ever fails.
-static __device__ __noinline__ uint32_t inv_mod_slow(uint32_t x, uint32_t q)
+// Exact inverse by integer-only extended Euclid; the fallback that runs only if the fast
+// routine's self-check ever fails.  Cofactors as magnitudes (at most q), signs alternating.
+// Inline: a call here made the kernels keep their state in callee-saved registers.
+__device__ __forceinline__ uint32_t inv_mod_slow(uint32_t x, uint32_t q)
 {
-  int64_t r0 = q, r1 = x, s0 = 0, s1 = 1;
-  while (r1 != 0) {
-    const int64_t Q = r0 / r1;
-    int64_t t = r0 - Q * r1; r0 = r1; r1 = t;
-    t = s0 - Q * s1; s0 = s1; s1 = t;
+  uint32_t r0 = q, r1 = x, s0 = 0u, s1 = 1u;
+  bool neg = true;                                // sign of s0
+#pragma unroll 1
+  while (r1 != 0u) {
+    const uint32_t Q = r0 / r1, r = r0 - Q * r1, s = s0 + Q * s1;
+    r0 = r1; r1 = r;
+    s0 = s1; s1 = s;
+    neg = !neg;
   }
-  return (uint32_t)(s0 < 0 ? s0 + q : s0);
+  return neg ? q - s0 : s0;
 }
 
 // Quotient estimate of the inverse's Euclid steps (also run by the certification kernel):
