@@ -444,6 +444,10 @@ int mgcd::plan_batch(mgcd_context* c, Plan& P, size_t np, const uint32_t* limbs,
   return MGCD_OK;
 }
 
+// Threads of a CTA that owns `per` moduli of a single pair: one modulus per thread and a
+// warp more for the pair's bookkeeping (run_pair), while they fit.
+static int single_threads(uint32_t per) { return (int)std::min<uint32_t>(1024, (per + 31) / 32 * 32 + 32); }
+
 // Groups the pairs `subset` (indices into descs) into size-class buckets (batches) or
 // single-pair launches (plain); appends the processing order to P.order and returns the
 // scratch words needed.  `latency`: the few pairs rerun after a scaled batch -- one
@@ -459,7 +463,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
     std::vector<uint32_t> v(subset);
     std::sort(v.begin(), v.end(), [&](uint32_t x, uint32_t y) { return descs[x].nq > descs[y].nq; });
     Bucket bk;
-    bk.threads = 512;
+    bk.threads = single_threads(512);
     bk.k = 1;
     bk.cls = CLUSTER_CLASS;
     bk.first = (uint32_t)P.order.size();
@@ -510,7 +514,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       for (size_t i = 0; i < v.size(); ++i) v[i] = key[i].second;
     }
     Bucket bk;
-    bk.threads = plain ? 256 : c->cfg[b].threads;
+    bk.threads = plain ? single_threads(plain_cta_max) : c->cfg[b].threads;
     bk.k = plain ? 1 : c->cfg[b].k;
     bk.csize = 0;
     bk.cls = b;
@@ -669,10 +673,9 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
       // 19.0 ms at 11,264; at 8,192 moduli the 512-thread cluster wins, 13.0 vs 14.0 ms)
       const int ctas = (int)std::min<uint32_t>(MAX_CLUSTER, (d.nq + 255) / 256);
       const uint32_t per = (d.nq + ctas - 1) / ctas;
-      const int threads = per <= 256 ? 256 : per <= 512 ? 512 : 1024;
       g.per_cta = per;
       g.sync = nullptr;
-      if (launch_cluster(g, threads, ctas, grid_smem_bytes(per), P.stream) != cudaSuccess) return MGCD_ERR_GRID;
+      if (launch_cluster(g, single_threads(per), ctas, grid_smem_bytes(per), P.stream) != cudaSuccess) return MGCD_ERR_GRID;
       ++P.launches;
       continue;
     }
@@ -681,7 +684,7 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
       constexpr int CS = 8;
       int nclu = c->sms / CS;
       uint32_t per = std::max<uint32_t>(32, (d.nq + nclu * CS - 1) / (nclu * CS));
-      const int threads = per <= 256 ? 256 : per <= 512 ? 512 : 1024;
+      const int threads = single_threads(per);
       int maxc = 0;
       if (cgrid_max_clusters(threads, CS, grid_smem_bytes(per), &maxc) != cudaSuccess || maxc < 1) return MGCD_ERR_GRID;
       if (maxc < nclu) {
@@ -694,7 +697,7 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
       g.sync = P.d_gsync.as<GridSync>();
       CK(launch_gridsync_init(g.sync, c->wait_timeout_ns, c->withhold_cta, P.stream));
       ++P.launches;
-      const int thr = per <= 256 ? 256 : per <= 512 ? 512 : 1024;
+      const int thr = single_threads(per);
       cudaError_t e = launch_cgrid(g, thr, CS, nclu, grid_smem_bytes(per), P.stream);
       if (e == cudaErrorCooperativeLaunchTooLarge) return MGCD_ERR_GRID;
       if (e != cudaSuccess) return MGCD_ERR_CUDA;
@@ -702,9 +705,9 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
       continue;
     }
     // cooperative grid: at most one CTA per SM and at least 256 moduli per CTA (fewer CTAs in
-    // each exchange); or the reference's shape: 256-thread CTAs, 256 moduli
+    // each exchange); or the reference's shape: 256-thread CTAs, 256 moduli each
     uint32_t per = ref_shape ? 256u : std::max<uint32_t>(256, (d.nq + c->sms - 1) / c->sms);
-    const int threads = (ref_shape || per <= 256) ? 256 : per <= 512 ? 512 : GRID_THREADS;
+    const int threads = ref_shape ? 256 : single_threads(per);
     int bps = 0;
     if (grid_max_blocks_per_sm(threads, grid_smem_bytes(per), &bps) != cudaSuccess || bps < 1) return MGCD_ERR_GRID;
     uint32_t grid = (d.nq + per - 1) / per;

@@ -175,7 +175,6 @@ cudaError_t launch_cgrid(const GridArgs& a, int threads, int csize, int clusters
 cudaError_t launch_gridsync_init(GridSync* gs, unsigned long long timeout_ns, uint32_t withhold, cudaStream_t s);
 
 size_t grid_smem_bytes(uint32_t per_cta);
-constexpr int GRID_THREADS = 1024;   // CTA size of the grid path (256 for the reference's shape)
 constexpr int MAX_CLUSTER = 16;      // largest thread-block cluster (non-portable size)
 cudaError_t grid_max_blocks_per_sm(int threads, size_t smem, int* blocks);
 cudaError_t launch_grid(const GridArgs& a, int threads, int grid, size_t smem, cudaStream_t s);

@@ -105,10 +105,9 @@ __device__ __forceinline__ void stream_done(const BatchArgs& a, uint32_t k)
   st_release_sys_u32(&a.ring->done[k % STREAM_RING], k + 1u);
 }
 
-// Persistent batched kernel: each CTA repeatedly takes the next pair of the queue (pairs
-// ordered largest first) and computes its gcd alone.
-template <int T>
-__global__ void __launch_bounds__(T) batch_kernel(const BatchArgs a)
+// Persistent batched kernel: each CTA (of any size up to 1,024 threads) repeatedly takes the
+// next pair of the queue (pairs ordered largest first) and computes its gcd alone.
+__global__ void __launch_bounds__(1024) batch_kernel(const BatchArgs a)
 {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ RedSmem rs;
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(T) batch_kernel(const BatchArgs a)
   uint32_t* v0 = scr + a.nq_max;
   int2* hist = reinterpret_cast<int2*>(scr + 2 * (size_t)a.nq_max);
   cta_begin(a);
-  uint32_t taken = 0;
+  uint32_t taken = 0, epoch = 0;
   for (;;) {
     if (threadIdx.x == 0) next = atomicAdd(a.queue, 1u);
     __syncthreads();
@@ -134,7 +133,7 @@ __global__ void __launch_bounds__(T) batch_kernel(const BatchArgs a)
     ++taken;
     const uint32_t pi = a.order[k];
     const PairDesc d = a.pairs[pi];
-    run_pair<T, SYNC_CTA>(a.limbs, d, a.mods, a.L, 0u, d.nq, st, acc2, stg, rs, u0, v0, hist, nullptr,
+    run_pair<0, SYNC_CTA>(a.limbs, d, a.mods, a.L, 0u, d.nq, st, acc2, stg, rs, u0, v0, hist, nullptr, epoch,
                        a.digits, a.count + pi, a.iters + pi, a.status + pi, a.inv);
     __syncthreads();
   }
@@ -150,36 +149,6 @@ __global__ void __launch_bounds__(T) batch_kernel(const BatchArgs a)
 // Set-up (residues) and finish (certification, replay, recovery) run pair by pair: when a
 // pair's loop ends, the CTA finishes it and loads the next pair of the queue into that
 // slot while the other slots keep their state, so the slots stay occupied.
-
-template <int K>
-struct SlotSmem {
-  unsigned long long key[2][K][32];  // per-warp minima per slot, double-buffered
-  PairDesc d[K];
-  uint32_t pi[K];                    // pair index of each slot (~0: empty)
-  long long lu[K], lv[K];            // certification bounds (bound_step)
-};
-
-template <int T, int K>
-__device__ __forceinline__ void block_min_keys(uint32_t (&kh)[K], uint32_t (&kl)[K], SlotSmem<K>& ss,
-                                               uint32_t& parity)
-{
-  constexpr int NW = T / 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int s = 0; s < K; ++s) {
-    warp_min_key(kh[s], kl[s]);
-    if (lane == 0) ss.key[parity][s][w] = ((unsigned long long)kh[s] << 32) | kl[s];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int s = 0; s < K; ++s) {
-    const unsigned long long k = (lane < NW) ? ss.key[parity][s][lane] : ~0ull;
-    kh[s] = (uint32_t)(k >> 32);
-    kl[s] = (uint32_t)k;
-    warp_min_key(kh[s], kl[s]);
-  }
-  parity ^= 1u;
-}
 
 // Per-slot loop state of batchk_kernel in shared memory.  Warp s owns slot s's entries
 // during the pivot step; every thread reads them only after a barrier that follows the
@@ -661,7 +630,7 @@ __global__ void __launch_bounds__(T) batchk_kernel(const BatchArgs a)
         uint32_t* u0 = scr + (size_t)s * 4 * NQS;
         finish_pair<T, SYNC_CTA>(a.mods, ss.d[s], L, 0u, ss.d[s].nq, tS + (size_t)s * NQS, rs, rparity, repoch, nullptr,
                               u0, u0 + NQS, reinterpret_cast<const int2*>(u0 + 2 * (size_t)NQS), it, ss.rem[s],
-                              ss.lu[s], ss.lv[s], a.digits, a.count + pi, a.status + pi, a.inv, smem, acc2,
+                              ss.lu[s], ss.lv[s], 0u, a.digits, a.count + pi, a.status + pi, a.inv, smem, acc2,
                               a.phases ? &phs[PH_REPLAY] : nullptr);
       }
       if (RING && threadIdx.x == 0) stream_done(a, ss.seq[s]);   // results written by this thread
@@ -823,39 +792,55 @@ __global__ void __launch_bounds__(T) batchk_kernel(const BatchArgs a)
 // The cluster analogue of batchk_kernel for pairs larger than one CTA (size class 3).  A
 // cluster of C CTAs holds K pairs; CTA r owns global moduli [r * per, (r + 1) * per) of every
 // pair (per = ceil(nq_max / C), the same slice for all slots, so a thread's K updates share
-// one modulus and one inverse).  Pivot keys: each CTA reduces its K minima (one
-// __syncthreads), warp 0 stores them into every CTA of the cluster (DSMEM), one cluster
-// barrier, then every warp reduces the C values per slot.  Queue pops are made by CTA 0 and
-// broadcast the same way.  Set-up and finish of one slot run the cluster single-pair code
+// one modulus and one inverse).  Pivot keys: after the warp minima and one __syncthreads, warp
+// s reduces slot s's and exchanges it with the other CTAs (cluster_min_key, the K slots in
+// parallel).  Queue pops are made by CTA 0 and broadcast through DSMEM.  Set-up and finish of one slot run the cluster single-pair code
 // on the CTA's slice while the other slots wait.
 
 template <int K>
+struct SlotSmem {
+  unsigned long long key[K][32];     // per-warp minima per slot
+  PairDesc d[K];
+  uint32_t pi[K];                    // pair index of each slot (~0: empty)
+  long long lu[K], lv[K];            // certification bounds (bound_step)
+};
+
+template <int K>
 struct ClusterSlotKeys {
-  unsigned long long key[2][K][MAX_CLUSTER];   // per slot: each CTA's minimum, double-buffered
+  unsigned long long key[2][K][MAX_CLUSTER];   // per slot: each CTA's tagged minimum, double-buffered
+  unsigned long long res[2][K];                // per slot: the cluster's minimum
   uint32_t next;                               // queue index broadcast by CTA 0
   uint32_t nloc[K];                            // this CTA's moduli of each slot's pair
 };
 
+// The K slots' minima over the cluster, in every thread; false if a wait expired.
 template <int T, int K>
-__device__ __forceinline__ void cluster_min_keys(uint32_t (&kh)[K], uint32_t (&kl)[K], SlotSmem<K>& ss,
-                                                 ClusterSlotKeys<K>& ck, uint32_t& kparity, uint32_t& cparity)
+__device__ __forceinline__ bool cluster_min_keys(uint32_t (&kh)[K], uint32_t (&kl)[K], SlotSmem<K>& ss,
+                                                 ClusterSlotKeys<K>& ck, ClusterSmem& cs, uint32_t& epoch)
 {
-  block_min_keys<T, K>(kh, kl, ss, kparity);
-  const uint32_t lane = threadIdx.x & 31u, me = cluster_rank(), nc = cluster_size();
-  if (threadIdx.x < 32u && lane < nc) {
-#pragma unroll
-    for (int s = 0; s < K; ++s)
-      st_cluster_u64(&ck.key[cparity][s][me], lane, ((unsigned long long)kh[s] << 32) | kl[s]);
-  }
-  cluster_sync_all();
+  static_assert(T / 32 >= K, "one warp per slot");
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, b = epoch & 1u;
 #pragma unroll
   for (int s = 0; s < K; ++s) {
-    const unsigned long long k = lane < nc ? ck.key[cparity][s][lane] : ~0ull;
-    kh[s] = (uint32_t)(k >> 32);
-    kl[s] = (uint32_t)k;
     warp_min_key(kh[s], kl[s]);
+    if (lane == 0) ss.key[s][w] = ((unsigned long long)kh[s] << 32) | kl[s];
   }
-  cparity ^= 1u;
+  __syncthreads();
+  if (w < K) {
+    const unsigned long long k = lane < T / 32 ? ss.key[w][lane] : ~0ull;
+    uint32_t h = (uint32_t)(k >> 32), l = (uint32_t)k;
+    warp_min_key(h, l);
+    cluster_min_key(h, l, ck.key[b][w], cs, key_tag(epoch));
+    if (lane == 0) ck.res[b][w] = ((unsigned long long)h << 32) | l;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < K; ++s) {
+    kh[s] = (uint32_t)(ck.res[b][s] >> 32);
+    kl[s] = (uint32_t)ck.res[b][s];
+  }
+  epoch += 1u;
+  return cs.dead == 0u;
 }
 
 template <int T, int K>
@@ -879,9 +864,8 @@ __global__ void __launch_bounds__(T) cluster_batchk_kernel(const BatchArgs a)
   const uint32_t NQS = a.nq_max;
   const int L = a.L;
   GridSync* const gcs = reinterpret_cast<GridSync*>(&cs);
-  // parities of the double-buffered exchanges: slot keys in the CTA (ss) and across the
-  // cluster (ck), single keys in the CTA (rs) and across the cluster (cs)
-  uint32_t kparity = 0, cparity = 0, bparity = 0, rparity = 0, repoch = 0;
+  // exchange counts: slot keys (ck), single keys (rs in the CTA, cs across the cluster)
+  uint32_t kepoch = 0, rparity = 0, repoch = 0;
   uint32_t valid = 0, active = 0, redux = 0;
   int rem[K], ubits[K], vbits[K];
   uint32_t iters[K], p[K], kh[K], kl[K];
@@ -889,7 +873,8 @@ __global__ void __launch_bounds__(T) cluster_batchk_kernel(const BatchArgs a)
   cta_begin(a);
   uint32_t taken = 0;
 
-  cluster_sync_all();
+  for (uint32_t i = threadIdx.x; i < 2u * K * MAX_CLUSTER; i += T) (&ck.key[0][0][0])[i] = 0ull;
+  cluster_exchange_init(cs);
   // Takes the next pair of the queue into slot s.  A CTA whose operands could not be staged
   // contributes the key (0, 0) (no modulus produces it), so the whole cluster answers that
   // pair with ST_TIMEOUT and takes the next one together.
@@ -940,8 +925,7 @@ __global__ void __launch_bounds__(T) cluster_batchk_kernel(const BatchArgs a)
         ss.lv[s] = bound_init(a.limbs + d.v_off, d.v_len);
       }
       if (!ok) h0 = l0 = 0u;
-      block_min_key<T>(h0, l0, rs, bparity);
-      cluster_min_key<T>(h0, l0, cs, rparity, [] {});
+      if (!reduce_min<T, SYNC_CLUSTER>(h0, l0, rs, rparity, gcs, repoch)) h0 = l0 = 0u;
       if (h0 != 0u || l0 != 0u) break;
       if (r == 0 && threadIdx.x == 0) {
         a.status[ss.pi[s]] = ST_TIMEOUT;
@@ -981,7 +965,7 @@ __global__ void __launch_bounds__(T) cluster_batchk_kernel(const BatchArgs a)
         uint32_t* u0 = scr + (size_t)s * 4 * NQS;
         finish_pair<T, SYNC_CLUSTER>(a.mods, ss.d[s], L, j0, ck.nloc[s], tS + (size_t)s * per, rs, rparity, repoch,
                                      gcs, u0 + j0, u0 + NQS + j0, reinterpret_cast<const int2*>(u0 + 2 * (size_t)NQS),
-                                     it, pick(rem, s), ss.lu[s], ss.lv[s], a.digits, a.count + pi, a.status + pi,
+                                     it, pick(rem, s), ss.lu[s], ss.lv[s], 0u, a.digits, a.count + pi, a.status + pi,
                                      a.inv, smem, acc2);
       }
       cluster_sync_all();                             // the slot's scratch is free in every CTA
@@ -1038,7 +1022,13 @@ __global__ void __launch_bounds__(T) cluster_batchk_kernel(const BatchArgs a)
         if (key_less(h, l, kh[s], kl[s])) { kh[s] = h; kl[s] = l; }
       }
     }
-    cluster_min_keys<T, K>(kh, kl, ss, ck, kparity, cparity);
+    if (!cluster_min_keys<T, K>(kh, kl, ss, ck, cs, kepoch)) {
+      if (r == 0 && threadIdx.x < K && ((valid >> threadIdx.x) & 1u)) {
+        a.status[ss.pi[threadIdx.x]] = ST_TIMEOUT;
+        a.count[ss.pi[threadIdx.x]] = 0;
+      }
+      break;
+    }
 #pragma unroll
     for (int s = 0; s < K; ++s)
       if ((active >> s) & 1u) key_pair(kh[s], kl[s], p[s], b[s]);
@@ -1047,10 +1037,9 @@ __global__ void __launch_bounds__(T) cluster_batchk_kernel(const BatchArgs a)
   cta_end(a, taken);
 }
 
-// One pair over a cooperative grid of GRID_THREADS-thread CTAs; CTA c owns moduli
-// [c * per_cta, min(nq, (c + 1) * per_cta)).
-template <int T>
-__global__ void __launch_bounds__(T) grid_kernel(const GridArgs a)
+// One pair over a cooperative grid of CTAs (of any size up to 1,024 threads); CTA c owns
+// moduli [c * per_cta, min(nq, (c + 1) * per_cta)).
+__global__ void __launch_bounds__(1024) grid_kernel(const GridArgs a)
 {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ RedSmem rs;
@@ -1066,15 +1055,15 @@ __global__ void __launch_bounds__(T) grid_kernel(const GridArgs a)
   uint32_t* u0 = a.scratch + j0;
   uint32_t* v0 = a.scratch + nq + j0;
   int2* hist = reinterpret_cast<int2*>(a.scratch + 2 * (size_t)nq);
-  run_pair<T, SYNC_GRID>(a.limbs, a.pair, a.mods, a.L, j0, nloc, st, acc2, stg, rs, u0, v0, hist,
-                               a.sync, a.digits, a.count, a.iters, a.status, a.inv);
+  uint32_t epoch = 0;
+  run_pair<0, SYNC_GRID>(a.limbs, a.pair, a.mods, a.L, j0, nloc, st, acc2, stg, rs, u0, v0, hist,
+                               a.sync, epoch, a.digits, a.count, a.iters, a.status, a.inv);
 }
 
 // One pair over a thread-block cluster (up to 16 CTAs, one per SM); CTA r owns moduli
 // [r * per_cta, min(nq, (r + 1) * per_cta)).  Pivot keys travel through distributed shared
-// memory; each reduction is one hardware cluster barrier (no global-memory round trip).
-template <int T>
-__global__ void __launch_bounds__(T) cluster_kernel(const GridArgs a)
+// memory (cluster_min_key; no global-memory round trip).
+__global__ void __launch_bounds__(1024) cluster_kernel(const GridArgs a)
 {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ RedSmem rs;
@@ -1091,9 +1080,10 @@ __global__ void __launch_bounds__(T) cluster_kernel(const GridArgs a)
   uint32_t* u0 = a.scratch + j0;
   uint32_t* v0 = a.scratch + nq + j0;
   int2* hist = reinterpret_cast<int2*>(a.scratch + 2 * (size_t)nq);
-  cluster_sync_all();   // every CTA of the cluster is running before remote stores begin
-  run_pair<T, SYNC_CLUSTER>(a.limbs, a.pair, a.mods, a.L, j0, nloc, st, acc2, stg, rs, u0, v0, hist,
-                            reinterpret_cast<GridSync*>(&cs), a.digits, a.count, a.iters, a.status, a.inv);
+  cluster_exchange_init(cs);
+  uint32_t epoch = 0;
+  run_pair<0, SYNC_CLUSTER>(a.limbs, a.pair, a.mods, a.L, j0, nloc, st, acc2, stg, rs, u0, v0, hist,
+                            reinterpret_cast<GridSync*>(&cs), epoch, a.digits, a.count, a.iters, a.status, a.inv);
   cluster_sync_all();   // no CTA leaves while others may still address its shared memory
 }
 
@@ -1101,8 +1091,7 @@ __global__ void __launch_bounds__(T) cluster_kernel(const GridArgs a)
 // [b * per_cta, ...); pivot keys meet inside each cluster through DSMEM and only one
 // leader per cluster joins the global exchange (fewer atomics on one address than one per
 // CTA).
-template <int T>
-__global__ void __launch_bounds__(T) cgrid_kernel(const GridArgs a)
+__global__ void __launch_bounds__(1024) cgrid_kernel(const GridArgs a)
 {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ RedSmem rs;
@@ -1122,8 +1111,9 @@ __global__ void __launch_bounds__(T) cgrid_kernel(const GridArgs a)
   if (threadIdx.x == 0) cg.g = a.sync;
   __syncthreads();
   cluster_sync_all();   // every CTA of the cluster is running before remote stores begin
-  run_pair<T, SYNC_CGRID>(a.limbs, a.pair, a.mods, a.L, j0, nloc, st, acc2, stg, rs, u0, v0, hist,
-                          reinterpret_cast<GridSync*>(&cg), a.digits, a.count, a.iters, a.status, a.inv);
+  uint32_t epoch = 0;
+  run_pair<0, SYNC_CGRID>(a.limbs, a.pair, a.mods, a.L, j0, nloc, st, acc2, stg, rs, u0, v0, hist,
+                          reinterpret_cast<GridSync*>(&cg), epoch, a.digits, a.count, a.iters, a.status, a.inv);
   cluster_sync_all();   // no CTA leaves while others may still address its shared memory
 }
 
@@ -1132,8 +1122,7 @@ __global__ void __launch_bounds__(T) cgrid_kernel(const GridArgs a)
 // (pair moduli split into C contiguous ranges).  The queue is popped by CTA 0 of the
 // cluster, which writes the index into every CTA's shared memory.  Scratch per cluster:
 // u0[nq_max], v0[nq_max], hist[2 * nq_max].
-template <int T>
-__global__ void __launch_bounds__(T) cluster_batch_kernel(const BatchArgs a)
+__global__ void __launch_bounds__(1024) cluster_batch_kernel(const BatchArgs a)
 {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ RedSmem rs;
@@ -1149,8 +1138,8 @@ __global__ void __launch_bounds__(T) cluster_batch_kernel(const BatchArgs a)
   uint32_t* acc2 = st + per_max;
   uint32_t* scr = a.scratch + (size_t)(blockIdx.x / C) * a.scratch_words;
   cta_begin(a);
-  uint32_t taken = 0;
-  cluster_sync_all();
+  uint32_t taken = 0, epoch = 0;
+  cluster_exchange_init(cs);
   for (;;) {
     if (r == 0 && threadIdx.x < C) {
       const uint32_t k = __shfl_sync(0xFFFFFFFFu >> (32 - C), threadIdx.x == 0 ? atomicAdd(a.queue, 1u) : 0u, 0);
@@ -1168,8 +1157,8 @@ __global__ void __launch_bounds__(T) cluster_batch_kernel(const BatchArgs a)
     const uint32_t per = (d.nq + C - 1) / C;
     const uint32_t j0 = r * per;
     const uint32_t nloc = j0 >= d.nq ? 0u : (d.nq - j0 < per ? d.nq - j0 : per);
-    run_pair<T, SYNC_CLUSTER>(a.limbs, d, a.mods, a.L, j0, nloc, st, acc2, stg, rs, scr + j0, scr + d.nq + j0,
-                              reinterpret_cast<int2*>(scr + 2 * (size_t)d.nq), reinterpret_cast<GridSync*>(&cs),
+    run_pair<0, SYNC_CLUSTER>(a.limbs, d, a.mods, a.L, j0, nloc, st, acc2, stg, rs, scr + j0, scr + d.nq + j0,
+                              reinterpret_cast<int2*>(scr + 2 * (size_t)d.nq), reinterpret_cast<GridSync*>(&cs), epoch,
                               a.digits, a.count + pi, a.iters + pi, a.status + pi, a.inv);
     cluster_sync_all();   // every CTA is done with `next` and with the pair's scratch
   }
@@ -1279,14 +1268,7 @@ static const void* batchk_fn_for(int threads, int k)
 // narrow: the context's moduli are below 2^30 (width <= 30)
 static const void* batch_fn_for(int threads, int k, bool narrow)
 {
-  if (k == 1) {
-    switch (threads) {
-      case 256: return reinterpret_cast<const void*>(&batch_kernel<256>);
-      case 512: return reinterpret_cast<const void*>(&batch_kernel<512>);
-      case 1024: return reinterpret_cast<const void*>(&batch_kernel<1024>);
-      default: return nullptr;
-    }
-  }
+  if (k == 1) return reinterpret_cast<const void*>(&batch_kernel);
   return narrow ? batchk_fn_for<true>(threads, k) : batchk_fn_for<false>(threads, k);
 }
 
@@ -1346,26 +1328,6 @@ cudaError_t launch_batch(const BatchArgs& a, int threads, int k, int grid, size_
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-static const void* cluster_fn(int threads)
-{
-  switch (threads) {
-    case 256: return reinterpret_cast<const void*>(&cluster_kernel<256>);
-    case 512: return reinterpret_cast<const void*>(&cluster_kernel<512>);
-    case 1024: return reinterpret_cast<const void*>(&cluster_kernel<1024>);
-    default: return nullptr;
-  }
-}
-
-static const void* cluster_batch_fn(int threads)
-{
-  switch (threads) {
-    case 256: return reinterpret_cast<const void*>(&cluster_batch_kernel<256>);
-    case 512: return reinterpret_cast<const void*>(&cluster_batch_kernel<512>);
-    case 1024: return reinterpret_cast<const void*>(&cluster_batch_kernel<1024>);
-    default: return nullptr;
-  }
-}
-
 static cudaLaunchConfig_t cluster_config(int ctas, int threads, int csize, size_t smem, cudaStream_t s,
                                          cudaLaunchAttribute* attr)
 {
@@ -1393,7 +1355,7 @@ static cudaError_t prepare_cluster_fn(const void* fn, int csize, size_t smem)
 
 static const void* cluster_batch_fn_k(int threads, int k)
 {
-  if (k == 1) return cluster_batch_fn(threads);
+  if (k == 1) return reinterpret_cast<const void*>(&cluster_batch_kernel);
   if (k == 2) {
     switch (threads) {
       case 256: return reinterpret_cast<const void*>(&cluster_batchk_kernel<256, 2>);
@@ -1431,7 +1393,7 @@ cudaError_t cluster_batch_max_clusters(int threads, int k, int csize, size_t sme
 
 cudaError_t launch_cluster(const GridArgs& a, int threads, int ctas, size_t smem, cudaStream_t s)
 {
-  const void* fn = cluster_fn(threads);
+  const void* fn = reinterpret_cast<const void*>(&cluster_kernel);
   cudaError_t e = prepare_cluster_fn(fn, ctas, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
@@ -1457,19 +1419,9 @@ cudaError_t launch_cluster_batch(const BatchArgs& a, int threads, int k, int csi
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-static const void* cgrid_fn(int threads)
-{
-  switch (threads) {
-    case 256: return reinterpret_cast<const void*>(&cgrid_kernel<256>);
-    case 512: return reinterpret_cast<const void*>(&cgrid_kernel<512>);
-    case 1024: return reinterpret_cast<const void*>(&cgrid_kernel<1024>);
-    default: return nullptr;
-  }
-}
-
 cudaError_t cgrid_max_clusters(int threads, int csize, size_t smem, int* clusters)
 {
-  const void* fn = cgrid_fn(threads);
+  const void* fn = reinterpret_cast<const void*>(&cgrid_kernel);
   cudaError_t e = prepare_cluster_fn(fn, csize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
@@ -1479,7 +1431,7 @@ cudaError_t cgrid_max_clusters(int threads, int csize, size_t smem, int* cluster
 
 cudaError_t launch_cgrid(const GridArgs& a, int threads, int csize, int clusters, size_t smem, cudaStream_t s)
 {
-  const void* fn = cgrid_fn(threads);
+  const void* fn = reinterpret_cast<const void*>(&cgrid_kernel);
   cudaError_t e = prepare_cluster_fn(fn, csize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[2];
@@ -1496,20 +1448,9 @@ size_t grid_smem_bytes(uint32_t per_cta)
   return sizeof(uint32_t) * (2 * (size_t)per_cta + STAGE_SMEM_WORDS);
 }
 
-static const void* grid_fn(int threads)
-{
-  switch (threads) {
-    case 256: return reinterpret_cast<const void*>(&grid_kernel<256>);
-    case 512: return reinterpret_cast<const void*>(&grid_kernel<512>);
-    case 1024: return reinterpret_cast<const void*>(&grid_kernel<1024>);
-    default: return nullptr;
-  }
-}
-
 cudaError_t grid_max_blocks_per_sm(int threads, size_t smem, int* blocks)
 {
-  const void* fn = grid_fn(threads);
-  if (!fn) return cudaErrorInvalidValue;
+  const void* fn = reinterpret_cast<const void*>(&grid_kernel);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, fn, threads, smem);
@@ -1517,8 +1458,7 @@ cudaError_t grid_max_blocks_per_sm(int threads, size_t smem, int* blocks)
 
 cudaError_t launch_grid(const GridArgs& a, int threads, int grid, size_t smem, cudaStream_t s)
 {
-  const void* fn = grid_fn(threads);
-  if (!fn) return cudaErrorInvalidValue;
+  const void* fn = reinterpret_cast<const void*>(&grid_kernel);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<GridArgs*>(&a)};

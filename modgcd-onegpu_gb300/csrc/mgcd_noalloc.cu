@@ -96,8 +96,9 @@ __global__ void __launch_bounds__(NA_THREADS) noalloc_kernel(const NaArgs a)
   int2* hist = reinterpret_cast<int2*>(a.scratch + 2 * (size_t)NA_MAX_NQ);
   // caller-owned operand buffers carry no padding for widened bulk copies: plain loads
   const Stage stg{smem + 2 * NA_MAX_NQ, nullptr, nullptr, 0u};
+  uint32_t epoch = 0;
   run_pair<NA_THREADS, SYNC_CTA>(a.limbs, d, a.mods, NA_L, 0u, d.nq, smem, smem + NA_MAX_NQ, stg,
-                              rs, u0, v0, hist, nullptr, a.digits, a.count, &iters, a.status, InvTab{nullptr, 0u});
+                              rs, u0, v0, hist, nullptr, epoch, a.digits, a.count, &iters, a.status, InvTab{nullptr, 0u});
   if (threadIdx.x == 0) {
     const int32_t s = *a.status;
     *a.status = s == ST_OK ? MGCD_OK : (s == ST_REDUX || s == ST_INSUFFICIENT) ? MGCD_ERR_REDUX

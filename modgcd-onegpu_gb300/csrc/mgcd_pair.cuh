@@ -30,10 +30,12 @@ struct RedSmem {
   uint32_t cert;                  // the result could not be certified (more moduli needed)
 };
 
-// Cluster mode: every warp's minimum lands in every CTA of the cluster, so one cluster
-// barrier per reduction suffices.  Double-buffered by parity.
+// Cluster mode: each CTA's minimum lands in every CTA of the cluster as a tagged word that
+// the receiver polls in its own shared memory (cluster_min_key).  Double-buffered.
 struct ClusterSmem {
-  unsigned long long key[2][MAX_CLUSTER][32];
+  unsigned long long key[2][MAX_CLUSTER];  // zero before use (cluster_exchange_init)
+  unsigned long long bcast[2];             // the cluster-wide result, for the CTA's other warps
+  uint32_t dead;                           // a bounded wait expired: later exchanges fail at once
 };
 
 // Cluster-grid mode: the global exchange state and, per CTA, the cluster's slots.
@@ -63,17 +65,6 @@ __device__ __forceinline__ void cluster_sync_all()
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// The two halves of cluster_sync_all, for work that overlaps the wait.
-__device__ __forceinline__ void cluster_arrive()
-{
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void cluster_wait()
-{
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // Stores v at the same shared-memory offset as *local in CTA `rank` of this cluster.
 __device__ __forceinline__ void st_cluster_u64(unsigned long long* local, uint32_t rank, unsigned long long v)
 {
@@ -81,32 +72,6 @@ __device__ __forceinline__ void st_cluster_u64(unsigned long long* local, uint32
   uint32_t ra;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
   asm volatile("st.shared::cluster.u64 [%0], %1;" :: "r"(ra), "l"(v) : "memory");
-}
-
-// Minimum over the whole cluster: each warp's minimum is written into every CTA's
-// slots, one cluster barrier, then each warp reduces all slots locally.
-template <int T, class F>
-__device__ __forceinline__ void cluster_min_key(uint32_t& hi, uint32_t& lo, ClusterSmem& cs, uint32_t& parity,
-                                                F&& during)
-{
-  constexpr int NW = T / 32;
-  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint32_t me = cluster_rank(), nc = cluster_size();
-  warp_min_key(hi, lo);
-  const unsigned long long k = ((unsigned long long)hi << 32) | lo;
-  if (lane < nc) st_cluster_u64(&cs.key[parity][me][w], lane, k);   // lane r writes into CTA r
-  cluster_arrive();
-  during();
-  cluster_wait();
-  unsigned long long m = ~0ull;
-  for (uint32_t e = lane; e < nc * NW; e += 32) {
-    const unsigned long long x = cs.key[parity][e / NW][e % NW];
-    m = x < m ? x : m;
-  }
-  hi = (uint32_t)(m >> 32);
-  lo = (uint32_t)m;
-  warp_min_key(hi, lo);
-  parity ^= 1u;
 }
 
 static __device__ __forceinline__ unsigned long long globaltimer_ns()
@@ -154,15 +119,23 @@ __device__ __forceinline__ bool lead_cta()
   else return blockIdx.x == 0;   // the grid's first CTA (also in the cluster grid)
 }
 
+// Threads of the CTA: T where the kernel fixes it, else (T = 0) the launch's block size.
+template <int T>
+__device__ __forceinline__ uint32_t cta_threads()
+{
+  if constexpr (T > 0) return (uint32_t)T;
+  else return blockDim.x;
+}
+
 // Lexicographic (hi, lo) minimum over the CTA; every thread gets the result.
 // One __syncthreads; the two slot buffers alternate so the next call cannot overwrite
 // slots still being read.
 template <int T>
 __device__ __forceinline__ void block_min_key(uint32_t& hi, uint32_t& lo, RedSmem& rs, uint32_t& parity)
 {
-  constexpr int NW = T / 32;
+  const uint32_t NW = cta_threads<T>() / 32u;
   warp_min_key(hi, lo);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
   if (lane == 0) rs.key[parity][w] = ((unsigned long long)hi << 32) | lo;
   __syncthreads();
   const unsigned long long k = (lane < NW) ? rs.key[parity][lane] : ~0ull;
@@ -172,17 +145,7 @@ __device__ __forceinline__ void block_min_key(uint32_t& hi, uint32_t& lo, RedSme
   parity ^= 1u;
 }
 
-// Minimum over the CTA and, with several CTAs, over the cluster (DSMEM + cluster barrier),
-// the cooperative grid (leader exchange over tagged slots) or the cluster grid (atomic
-// minimum and arrival counter per cluster leader); the grid protocols are described at
-// GridSync.  Every wait is bounded by timeout_ns; returns false if one expired (the grid
-// then unwinds; the host sees ST_TIMEOUT).
-// `during()` is called by every thread while the CTA waits for the others (after its own
-// contribution is out), so per-iteration bookkeeping of one thread (BOUND_THREAD, not the
-// thread that carries the CTA's part of the exchange) overlaps the exchange.
-constexpr uint32_t BOUND_THREAD = 32;
-
-// 63-bit form of a key for the tagged grid exchange, in the same order: |value| keys stay
+// 63-bit form of a key for the tagged exchanges, in the same order: |value| keys stay
 // below 2^31 - 1, MOD_INFINITY (0x80000000) and "no key" (0xFFFFFFFF, 0xFFFFFFFF) share the
 // high word 2^31 - 1 and differ in the low word.  Bit 63 carries the exchange tag.
 constexpr unsigned long long KEY_TAG = 1ull << 63;
@@ -205,37 +168,98 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned l
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
 }
 
-template <int T, int MODE, bool PUB = false, class F>
-__device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& rs, uint32_t& parity,
-                                           GridSync* gs, uint32_t& epoch, F&& during)
+__device__ __forceinline__ unsigned long long key_tag(uint32_t epoch)
 {
-  if constexpr (MODE == SYNC_CLUSTER) {
-    ClusterSmem& cs = *reinterpret_cast<ClusterSmem*>(gs);
-    const uint32_t nc = cluster_size();
-    if (nc * (T / 32) <= 64) {
-      cluster_min_key<T>(hi, lo, cs, parity, during);
-      return true;
-    }
-    // Large clusters: the CTA's minimum first (one __syncthreads), then one key per CTA
-    // into every CTA (slot [me][0] of the buffer chosen by the exchange count), one cluster
-    // barrier, and a 16-entry reduction instead of one over every warp of the cluster.
+  return (unsigned long long)(((epoch >> 1) + 1u) & 1u) << 63;
+}
+
+// A grid poll looks at the error flag and the clock once in POLL_CHECK polls: on every one,
+// they made the two hops of an exchange ~370 cycles longer.
+constexpr uint32_t POLL_CHECK = 256u;
+struct PollClock {
+  uint32_t n = 0;
+  unsigned long long t0 = 0;
+  __device__ __forceinline__ bool due() { return (++n & (POLL_CHECK - 1u)) == 0u; }
+  __device__ __forceinline__ bool expired(unsigned long long limit_ns)
+  {
+    const unsigned long long t = globaltimer_ns();
+    if (t0 == 0ull) t0 = t;
+    return t - t0 > limit_ns;
+  }
+};
+constexpr uint32_t CLUSTER_POLLS = 1u << 25;   // bound of a cluster poll: ~0.5 s of polls
+
+// Once per kernel, before the first exchange: every CTA's slots are zero when any CTA of the
+// cluster stores into them.
+__device__ __forceinline__ void cluster_exchange_init(ClusterSmem& cs)
+{
+  if (threadIdx.x < 2u * MAX_CLUSTER) (&cs.key[0][0])[threadIdx.x] = 0ull;
+  if (threadIdx.x == 0) cs.dead = 0u;
+  __syncthreads();
+  cluster_sync_all();
+}
+
+// Warp 0, with the CTA's minimum in every lane: lane c stores it, tagged with the exchange
+// count, into this CTA's slot in CTA c, and polls CTA c's slot here; the minimum of all in
+// every lane.  A slot read in exchange e holds e's or e - 2's value (no CTA can be two
+// exchanges ahead of another), which the tag tells apart, so there is neither a cluster
+// barrier nor a fence.  What bounds it is one DSMEM hop, ~450 cycles: with the CTA's own
+// reduction 725-783 cycles per exchange (2-16 CTAs of 256 or 512 threads) against 950-1,630
+// with stores and a cluster barrier (barrier.cluster, release and acquire).  False (sticky)
+// if a wait expired.
+__device__ __forceinline__ bool cluster_min_key(uint32_t& hi, uint32_t& lo, unsigned long long (&slots)[MAX_CLUSTER],
+                                                ClusterSmem& cs, unsigned long long tag)
+{
+  const uint32_t lane = threadIdx.x & 31u, nc = cluster_size();
+  if (lane < nc) st_cluster_u64(&slots[cluster_rank()], lane, tag | pack_key(hi, lo));
+  const volatile unsigned long long* const mine = &slots[lane < nc ? lane : 0u];
+  bool ok = *reinterpret_cast<volatile uint32_t*>(&cs.dead) == 0u;
+  unsigned long long v = 0ull;
+  for (uint32_t n = 0; ok; ++n) {
+    v = *mine;
+    if (__all_sync(0xFFFFFFFFu, (v & KEY_TAG) == tag)) break;
+    if (n >= CLUSTER_POLLS) { cs.dead = 1u; ok = false; }
+  }
+  unpack_key(v & ~KEY_TAG, hi, lo);
+  warp_min_key(hi, lo);
+  return ok;
+}
+
+// Minimum over the CTA and, with several CTAs, over the cluster (cluster_min_key), the
+// cooperative grid (leader exchange over tagged slots) or the cluster grid (atomic minimum
+// and arrival counter per cluster leader); the grid protocols are described at GridSync.
+// Every wait is bounded; returns false if one expired (the pair then unwinds; the host sees
+// ST_TIMEOUT).  PUB: the exchange also publishes data written before it to every CTA.
+template <int T, int MODE, bool PUB = false>
+__device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& rs, uint32_t& parity,
+                                           GridSync* gs, uint32_t& epoch)
+{
+  if constexpr (MODE == SYNC_CTA) {
     block_min_key<T>(hi, lo, rs, parity);
-    const uint32_t cb = epoch & 1u, lane = threadIdx.x & 31u, me = cluster_rank();
-    if (threadIdx.x < 32u && lane < nc) st_cluster_u64(&cs.key[cb][me][0], lane, ((unsigned long long)hi << 32) | lo);
-    cluster_arrive();
-    during();
-    cluster_wait();
-    const unsigned long long k = lane < nc ? cs.key[cb][lane][0] : ~0ull;
-    hi = (uint32_t)(k >> 32);
-    lo = (uint32_t)k;
-    warp_min_key(hi, lo);
-    epoch += 1u;
     return true;
   }
-  if constexpr (MODE == SYNC_CTA) {
-    during();
-    block_min_key<T>(hi, lo, rs, parity);
-    return true;
+  if constexpr (MODE == SYNC_CLUSTER) {
+    ClusterSmem& cs = *reinterpret_cast<ClusterSmem*>(gs);
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, cb = epoch & 1u;
+    if constexpr (PUB) cluster_sync_all();           // release / acquire in the cluster
+    warp_min_key(hi, lo);
+    if (lane == 0) rs.key[parity][w] = ((unsigned long long)hi << 32) | lo;
+    __syncthreads();
+    if (w == 0) {
+      const unsigned long long k = lane < cta_threads<T>() / 32u ? rs.key[parity][lane] : ~0ull;
+      hi = (uint32_t)(k >> 32);
+      lo = (uint32_t)k;
+      warp_min_key(hi, lo);
+      cluster_min_key(hi, lo, cs.key[cb], cs, key_tag(epoch));
+      if (lane == 0) cs.bcast[cb] = ((unsigned long long)hi << 32) | lo;
+    }
+    __syncthreads();
+    const unsigned long long k = cs.bcast[cb];
+    hi = (uint32_t)(k >> 32);
+    lo = (uint32_t)k;
+    parity ^= 1u;
+    epoch += 1u;
+    return cs.dead == 0u;
   }
   block_min_key<T>(hi, lo, rs, parity);
   if constexpr (MODE == SYNC_CGRID) {
@@ -282,7 +306,6 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
         asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(ra), "r"(bad) : "memory");
       }
     }
-    during();
     cluster_sync_all();
     const unsigned long long k = cg.res[cb];
     const bool ok = cg.bad[cb] == 0u;
@@ -293,43 +316,38 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
   } else {
     // Leader exchange (GridSync): tagged slots, relaxed stores and loads, bounded polls.
     // PUB adds release fences before the stores and acquire fences after the polls, for
-    // exchanges that also publish data written before them.
+    // exchanges that also publish data written before them.  What bounds it: two hops through
+    // L2, each a store (~300 cycles) and the poll that sees it (295 cycles a round trip).
     const uint32_t b = epoch & 1u;
-    const unsigned long long tag = (unsigned long long)(((epoch >> 1) + 1u) & 1u) << 63;
+    const unsigned long long tag = key_tag(epoch);
     unsigned long long* const keys = gs->keys[b];
     unsigned long long k = pack_key(hi, lo);
     uint32_t bad = 0;
+    PollClock clk;
     if (blockIdx.x != 0) {
       if (threadIdx.x == 0) {
         if constexpr (PUB) __threadfence();
         if (blockIdx.x != gs->withhold_cta) st_relaxed_u64(keys + blockIdx.x, tag | k);
-        const unsigned long long t0 = globaltimer_ns();
         unsigned long long v;
-        for (;;) {
-          v = ld_relaxed_u64(&gs->bcast[b][0]);
-          if ((v & KEY_TAG) == tag) break;
+        while (((v = ld_relaxed_u64(&gs->bcast[b][0])) & KEY_TAG) != tag) {
+          if (!clk.due()) continue;
           if (ld_relaxed_u32(&gs->error)) { bad = 1; break; }
-          if (globaltimer_ns() - t0 > gs->timeout_ns) { atomicExch(&gs->error, 1u); bad = 1; break; }
+          if (clk.expired(gs->timeout_ns)) { atomicExch(&gs->error, 1u); bad = 1; break; }
         }
         if constexpr (PUB) __threadfence();
         rs.bcast = v & ~KEY_TAG;
         rs.bad = bad;
       }
-      during();
       __syncthreads();
       k = rs.bcast;
       bad = rs.bad;
     } else {
-      during();
       unsigned long long m = threadIdx.x == 0 ? k : ~0ull;
-      const unsigned long long t0 = globaltimer_ns();
-      for (uint32_t i = threadIdx.x == 0 ? T : threadIdx.x; i < gridDim.x && !bad; i += T) {
+      for (uint32_t i = threadIdx.x == 0 ? cta_threads<T>() : threadIdx.x; i < gridDim.x && !bad;
+           i += cta_threads<T>()) {
         unsigned long long v;
-        for (;;) {
-          v = ld_relaxed_u64(keys + i);
-          if ((v & KEY_TAG) == tag) break;
-          if (globaltimer_ns() - t0 > gs->timeout_ns) { atomicExch(&gs->error, 1u); bad = 1; break; }
-        }
+        while (((v = ld_relaxed_u64(keys + i)) & KEY_TAG) != tag)
+          if (clk.due() && clk.expired(gs->timeout_ns)) { atomicExch(&gs->error, 1u); bad = 1; break; }
         v &= ~KEY_TAG;
         m = v < m ? v : m;
       }
@@ -347,13 +365,6 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
     epoch += 1u;
     return bad == 0;
   }
-}
-
-template <int T, int MODE, bool PUB = false>
-__device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& rs, uint32_t& parity,
-                                           GridSync* gs, uint32_t& epoch)
-{
-  return reduce_min<T, MODE, PUB>(hi, lo, rs, parity, gs, epoch, [] {});
 }
 
 // ---- operand staging: bulk copies (the TMA engine, cp.async.bulk) into shared memory
@@ -463,7 +474,8 @@ template <int T>
 __device__ bool residues(const uint32_t* __restrict__ x, uint32_t n, const ModConst* __restrict__ mods,
                          uint32_t nloc, uint32_t* __restrict__ acc, Stage stg, bool narrow)
 {
-  for (uint32_t j = threadIdx.x; j < nloc; j += T) acc[j] = 0u;
+  const uint32_t TT = cta_threads<T>();
+  for (uint32_t j = threadIdx.x; j < nloc; j += TT) acc[j] = 0u;
   int nt = ((int)n + CHUNK - 1) / CHUNK;
   bool ok = true;
   if (stg.mbar == nullptr) {
@@ -474,13 +486,13 @@ __device__ bool residues(const uint32_t* __restrict__ x, uint32_t n, const ModCo
       __syncthreads();
       if (stg.coherent) {
         const volatile uint32_t* xv = x;
-        for (int i = lo + (int)threadIdx.x; i < hi; i += T) chunk[i - lo] = xv[i];
+        for (int i = lo + (int)threadIdx.x; i < hi; i += (int)TT) chunk[i - lo] = xv[i];
       } else {
-        for (int i = lo + (int)threadIdx.x; i < hi; i += T) chunk[i - lo] = __ldg(x + i);
+        for (int i = lo + (int)threadIdx.x; i < hi; i += (int)TT) chunk[i - lo] = __ldg(x + i);
       }
       __syncthreads();
       const int len = hi - lo;
-      for (uint32_t j = threadIdx.x; j < nloc; j += T) acc[j] = horner_tile(acc[j], chunk, len, mods[j], narrow);
+      for (uint32_t j = threadIdx.x; j < nloc; j += TT) acc[j] = horner_tile(acc[j], chunk, len, mods[j], narrow);
     }
   } else {
     __syncthreads();                   // the state word of the previous call is written
@@ -514,14 +526,14 @@ __device__ bool residues(const uint32_t* __restrict__ x, uint32_t n, const ModCo
       const uint32_t* const chunk =
           stg.buf + b * STAGE_WORDS + (uint32_t)(((uintptr_t)(x + lo) & 15) >> 2);
       const int len = hi - lo;
-      for (uint32_t j = threadIdx.x; j < nloc; j += T) acc[j] = horner_tile(acc[j], chunk, len, mods[j], narrow);
+      for (uint32_t j = threadIdx.x; j < nloc; j += TT) acc[j] = horner_tile(acc[j], chunk, len, mods[j], narrow);
       __syncthreads();                 // buffer b is free for tile t + 2
     }
     if (threadIdx.x == 0) *stg.state = phase;
   }
   if (stg.inject) ok = false;
   __syncthreads();
-  for (uint32_t j = threadIdx.x; j < nloc; j += T) {
+  for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
     const ModConst c = mods[j];
     acc[j] = redc((uint64_t)acc[j] * c.r2, c.q, c.qinv);
   }
@@ -533,7 +545,7 @@ template <int T, int MODE>
 __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d, int L, uint32_t j0, uint32_t nloc,
                             uint32_t* st, RedSmem& rs, uint32_t& parity, uint32_t& epoch, GridSync* gs,
                             const uint32_t* u0g, const uint32_t* v0g, const int2* hist, uint32_t iters, int remaining,
-                            long long lu, long long lv, mgcd_pair* digits, uint32_t* count, int32_t* status,
+                            long long lu, long long lv, uint32_t bound_thread, mgcd_pair* digits, uint32_t* count, int32_t* status,
                             InvTab inv, uint32_t* hbuf, uint32_t* ibuf, unsigned long long* prof_replay = nullptr);
 
 // The whole gcd of one pair by this CTA (GRID = false) or by the cooperative grid, the
@@ -544,23 +556,30 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
 // A CTA whose operands could not be staged contributes the key (0, 0), which no modulus
 // produces (it would need q = 1): the first exchange then stops every CTA of the pair
 // together and the pair is answered with ST_TIMEOUT.
+//   epoch      the exchange count, kept by the kernel from pair to pair
+// A single pair is one chain of iterations (inverse, then exchange), so nothing else is on
+// that chain: with at most one modulus per thread its state and constants stay in registers,
+// and the history and the certification bounds (logarithms, ~650 cycles) are the work of one
+// thread of the last warp at the start of the update, which the launches leave without moduli
+// where they can (a warp more than the moduli need).
 template <int T, int MODE>
 __device__ void run_pair(const uint32_t* __restrict__ limbs, const PairDesc& d, const ModConst* __restrict__ mods,
                          int L, uint32_t j0, uint32_t nloc, uint32_t* st, uint32_t* acc2, Stage stg,
-                         RedSmem& rs, uint32_t* u0g, uint32_t* v0g, int2* hist, GridSync* gs,
+                         RedSmem& rs, uint32_t* u0g, uint32_t* v0g, int2* hist, GridSync* gs, uint32_t& epoch,
                          mgcd_pair* digits, uint32_t* count, uint32_t* iters_out, int32_t* status,
                          InvTab inv)
 {
   const bool writer = threadIdx.x == 0 && lead_cta<MODE>();
+  const uint32_t TT = cta_threads<T>(), book = TT - 32u;   // book: the bookkeeping thread
   const ModConst* __restrict__ my = mods + j0;
-  uint32_t parity = 0, epoch = 0;
+  uint32_t parity = 0;
 
   // ---- MGCD2: residues
   const bool staged = residues<T>(limbs + d.u_off, d.u_len, my, nloc, st, stg, L <= 30);
   const bool ok = residues<T>(limbs + d.v_off, d.v_len, my, nloc, acc2, stg, L <= 30) && staged;
 
   uint32_t kh = 0xFFFFFFFFu, kl = 0xFFFFFFFFu;
-  for (uint32_t j = threadIdx.x; j < nloc; j += T) {
+  for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
     const ModConst c = my[j];
     const uint32_t u = st[j], v = acc2[j];
     u0g[j] = u;
@@ -588,25 +607,37 @@ __device__ void run_pair(const uint32_t* __restrict__ limbs, const PairDesc& d, 
   int remaining = (int)d.nq;
   int ubits = ((int)d.u_len + 1) * 32, vbits = ((int)d.v_len + 1) * 32;
   uint32_t iters = 0;
-  // Certification bounds (BOUND_THREAD of each CTA; every CTA computes the same values),
-  // stepped while the CTA waits in the exchange.
+  // Certification bounds (one thread of each CTA; every CTA computes the same values).
   long long lu = 0, lv = 0;
-  if (threadIdx.x == BOUND_THREAD) {
+  if (threadIdx.x == book) {
     lu = bound_init(limbs + d.u_off, d.u_len);
     lv = bound_init(limbs + d.v_off, d.v_len);
   }
+  const bool one = nloc <= TT, have = threadIdx.x < nloc;   // `one`: states in registers
+  const ModConst c1 = (one && have ? my : mods)[one && have ? threadIdx.x : 0u];
+  uint32_t t1 = one && have ? st[threadIdx.x] : T_RETIRED;
   while (b != MOD_INFINITY) {
-    if (writer) hist[iters] = make_int2((int)p, b);
+    if (threadIdx.x == book) {
+      if (lead_cta<MODE>()) hist[iters] = make_int2((int)p, b);
+      bound_step(lu, lv, p, b);
+    }
     ++iters;
     kh = 0xFFFFFFFFu;
     kl = 0xFFFFFFFFu;
-    for (uint32_t j = threadIdx.x; j < nloc; j += T) {
-      const ModConst c = my[j];
-      const uint32_t t = t_update(st[j], c.q, c.qinv, p, b, L <= 30);
-      st[j] = t;
-      uint32_t h, l;
-      t_key(t, c.q, h, l);
-      if (key_less(h, l, kh, kl)) { kh = h; kl = l; }
+    if (one) {
+      if (have) {
+        t1 = t_update(t1, c1.q, c1.qinv, p, b, L <= 30);
+        t_key(t1, c1.q, kh, kl);
+      }
+    } else {
+      for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
+        const ModConst c = my[j];
+        const uint32_t t = t_update(st[j], c.q, c.qinv, p, b, L <= 30);
+        st[j] = t;
+        uint32_t h, l;
+        t_key(t, c.q, h, l);
+        if (key_less(h, l, kh, kl)) { kh = h; kl = l; }
+      }
     }
     remaining -= 1;
     const uint32_t absb = b < 0 ? 0u - (uint32_t)b : (uint32_t)b;
@@ -617,18 +648,15 @@ __device__ void run_pair(const uint32_t* __restrict__ limbs, const PairDesc& d, 
       if (writer) { *status = ST_REDUX; *count = 0; }
       return;
     }
-    const uint32_t pp = p;
-    const int32_t bb = b;
-    if (!reduce_min<T, MODE>(kh, kl, rs, parity, gs, epoch, [&] {
-          if (threadIdx.x == BOUND_THREAD) bound_step(lu, lv, pp, bb);
-        })) {
+    if (!reduce_min<T, MODE>(kh, kl, rs, parity, gs, epoch)) {
       if (writer) *status = ST_TIMEOUT;
       return;
     }
     key_pair(kh, kl, p, b);
   }
+  if (one && have) st[threadIdx.x] = t1;
   if (writer) *iters_out = iters;
-  finish_pair<T, MODE>(mods, d, L, j0, nloc, st, rs, parity, epoch, gs, u0g, v0g, hist, iters, remaining, lu, lv,
+  finish_pair<T, MODE>(mods, d, L, j0, nloc, st, rs, parity, epoch, gs, u0g, v0g, hist, iters, remaining, lu, lv, book,
                        digits, count, status, inv, stg.buf, acc2);
 }
 
@@ -660,6 +688,7 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
   __shared__ mgcd_pair pdig[32];       // the panel's digits
   __shared__ uint32_t pn;              // panel size, then the digits it produced
   const bool writer = threadIdx.x == 0 && lead_cta<MODE>();
+  const uint32_t TT = cta_threads<T>();
   const ModConst* __restrict__ my = mods + j0;
   const uint32_t lane = threadIdx.x & 31u;
   mgcd_pair* const out = digits + d.out_off;
@@ -691,7 +720,7 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
       }
       __syncthreads();
       np = pn;
-      for (uint32_t e = threadIdx.x; e < np * np; e += T) {
+      for (uint32_t e = threadIdx.x; e < np * np; e += TT) {
         const uint32_t a = e / np, bb = e % np;
         uint32_t v = 0u;
         if (a != bb) {
@@ -751,7 +780,7 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
       // ---- 5. one reference round: the lowest nonzero modulus anywhere, or the end
       kh = 0xFFFFFFFFu;
       kl = 0xFFFFFFFFu;
-      for (uint32_t j = threadIdx.x; j < nloc; j += T) {
+      for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
         const uint32_t u = st[j];
         if (u != U_RETIRED && u != 0u) { kh = j0 + j; kl = (uint32_t)to_signed(u, my[j].q); break; }
       }
@@ -765,7 +794,7 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
       }
       const uint32_t p = mods[kh].q;
       const int32_t g = (int32_t)kl;
-      for (uint32_t j = threadIdx.x; j < nloc; j += T) {
+      for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
         uint32_t u = st[j];
         if (u == U_RETIRED) continue;
         const ModConst c = my[j];
@@ -785,7 +814,7 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
     }
     // ---- 4. the panel's digits on every other surviving modulus, as one composed map
     const uint32_t last = front ? pidx[np - 1u] : 0u;
-    for (uint32_t j = threadIdx.x; j < nloc; j += T) {
+    for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
       const uint32_t u = st[j];
       if (u == U_RETIRED || (front && j <= last)) continue;   // the panel lanes are done
       const ModConst c = my[j];
@@ -816,22 +845,23 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
 
 // After the reduction loop of one pair: certification, replay and recovery (MGCD4).
 // st holds the final t states of this CTA's moduli; `remaining` the surviving count;
-// lu, lv (meaningful in BOUND_THREAD) the size bounds of the final u and v.
+// lu, lv (meaningful in bound_thread) the size bounds of the final u and v.
 template <int T, int MODE>
 __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d, int L, uint32_t j0, uint32_t nloc,
                             uint32_t* st, RedSmem& rs, uint32_t& parity, uint32_t& epoch, GridSync* gs,
                             const uint32_t* u0g, const uint32_t* v0g, const int2* hist, uint32_t iters, int remaining,
-                            long long lu, long long lv, mgcd_pair* digits, uint32_t* count, int32_t* status,
+                            long long lu, long long lv, uint32_t bound_thread, mgcd_pair* digits, uint32_t* count, int32_t* status,
                             InvTab inv, uint32_t* hbuf, uint32_t* ibuf, unsigned long long* prof_replay)
 {
   const bool writer = threadIdx.x == 0 && lead_cta<MODE>();
+  const uint32_t TT = cta_threads<T>();
   const ModConst* __restrict__ my = mods + j0;
   uint32_t p, kh, kl;
   const long long t_begin = prof_replay ? clock64() : 0;   // phase accounting: certification + replay
   // Certify the result: all surviving residues of v are 0, so v = 0 if the surviving
   // moduli (each > 2^(L-1)) multiply to more than |v|; recovery is exact if they exceed
   // 2|u| (symmetric digits).  Otherwise report that more moduli are needed.
-  if (threadIdx.x == BOUND_THREAD) rs.cert = bound_certified(remaining, L, lu, lv) ? 0u : 1u;
+  if (threadIdx.x == bound_thread) rs.cert = bound_certified(remaining, L, lu, lv) ? 0u : 1u;
   if constexpr (MODE == SYNC_GRID) __threadfence();
   __syncthreads();
   if (rs.cert) {
@@ -839,9 +869,10 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
     __syncthreads();
     return;
   }
+  if constexpr (MODE == SYNC_CLUSTER) cluster_sync_all();   // publishes the (p, b) history
   if constexpr (MODE == SYNC_GRID) {
-    // CTA 0's thread 0 wrote the (p, b) history during the loop, whose exchanges order
-    // nothing but the keys: one fenced exchange publishes it to every CTA.
+    // CTA 0's bookkeeping thread wrote the (p, b) history during the loop, whose exchanges
+    // order nothing but the keys: one fenced exchange publishes it to every CTA.
     uint32_t h = 0xFFFFFFFFu, l = 0xFFFFFFFFu;
     if (!reduce_min<T, MODE, true>(h, l, rs, parity, gs, epoch)) {
       if (writer) *status = ST_TIMEOUT;
@@ -863,12 +894,12 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
     __shared__ uint32_t nsurv;
     if (threadIdx.x == 0) nsurv = 0u;
     __syncthreads();
-    for (uint32_t j = threadIdx.x; j < nloc; j += T)
+    for (uint32_t j = threadIdx.x; j < nloc; j += TT)
       if (st[j] != T_RETIRED) ibuf[atomicAdd(&nsurv, 1u)] = j;
     __syncthreads();
     ns = nsurv;
     int2* const hb = reinterpret_cast<int2*>(hbuf);
-    for (uint32_t base = 0; base < ns; base += T) {
+    for (uint32_t base = 0; base < ns; base += TT) {
       const bool have = base + threadIdx.x < ns;
       const uint32_t j = have ? ibuf[base + threadIdx.x] : 0u;
       const ModConst c = my[j];
@@ -877,7 +908,7 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
       for (uint32_t c0 = 0; c0 < iters; c0 += REPLAY_CHUNK) {
         const uint32_t n = iters - c0 < REPLAY_CHUNK ? iters - c0 : REPLAY_CHUNK;
         __syncthreads();                               // the previous chunk is consumed
-        for (uint32_t e = threadIdx.x; e < n; e += T) hb[e] = hist[c0 + e];
+        for (uint32_t e = threadIdx.x; e < n; e += TT) hb[e] = hist[c0 + e];
         __syncthreads();
         if (!have) continue;
         if (narrow) {
@@ -918,7 +949,7 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
       }
     }
     __syncthreads();                                   // hbuf, ibuf and the replayed values
-    for (uint32_t j = threadIdx.x; j < nloc; j += T)
+    for (uint32_t j = threadIdx.x; j < nloc; j += TT)
       if (st[j] == T_RETIRED) st[j] = U_RETIRED;
   }
   if (prof_replay) {                   // non-null in every thread of the CTA or in none
@@ -935,7 +966,7 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
   // in ibuf (in no particular order: each thread keeps the lowest index among its own)
   kh = 0xFFFFFFFFu;
   kl = 0u;
-  for (uint32_t i = threadIdx.x; i < ns; i += T) {
+  for (uint32_t i = threadIdx.x; i < ns; i += TT) {
     const uint32_t j = ibuf[i], u = st[j];
     if (u != 0u && j0 + j < kh) { kh = j0 + j; kl = (uint32_t)to_signed(u, my[j].q); }
   }
@@ -950,7 +981,7 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
   do {
     kh = 0xFFFFFFFFu;
     kl = 0u;
-    for (uint32_t i = threadIdx.x; i < ns; i += T) {
+    for (uint32_t i = threadIdx.x; i < ns; i += TT) {
       const uint32_t j = ibuf[i];
       uint32_t u = st[j];
       if (u == U_RETIRED) continue;
