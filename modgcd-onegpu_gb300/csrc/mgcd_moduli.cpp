@@ -89,7 +89,7 @@ void mod_constants(const uint32_t* q, size_t n, ModConstHost* out)
     for (int k = 0; k < 5; ++k) x *= 2u - m * x;
     const uint64_t r1 = (uint64_t{1} << 32) % m;
     out[i].q = m;
-    out[i].qinv = 0u - x;
+    out[i].qinv = x;
     out[i].r2 = (uint32_t)((r1 * r1) % m);
     out[i].r1 = (uint32_t)r1;
   }

@@ -448,17 +448,13 @@ __device__ __forceinline__ void stage_issue(const uint32_t* x, int lo, int hi, S
 }
 
 // One tile of Horner steps z' = REDC(z * (2^64 mod q) + limb), most significant limb last
-// in `chunk`.  narrow (moduli below 2^30): z stays lazily in [0, 2q) in 32-bit arithmetic
-// (z * r2 + limb < 2q^2 + 2^32 < q 2^32, so REDC without the final subtraction is below 2q).
+// in `chunk`.  narrow (moduli below 2^30): z stays lazily in [0, 2q)
+// (z * r2 + limb < 2q^2 + 2^32 < q 2^32, as redc_lazy asks).
 __device__ __forceinline__ uint32_t horner_tile(uint32_t z, const uint32_t* chunk, int len, const ModConst& c,
                                                 bool narrow)
 {
   if (narrow) {
-    for (int i = len - 1; i >= 0; --i) {
-      const uint64_t t = (uint64_t)z * c.r2 + chunk[i];
-      const uint32_t lo = (uint32_t)t, hi = (uint32_t)(t >> 32);
-      z = hi + __umulhi(lo * c.qinv, c.q) + (lo != 0u);
-    }
+    for (int i = len - 1; i >= 0; --i) z = redc_lazy((uint64_t)z * c.r2 + chunk[i], c.q, c.qinv);
   } else {
     for (int i = len - 1; i >= 0; --i) z = redc((uint64_t)z * c.r2 + chunk[i], c.q, c.qinv);
   }
@@ -882,8 +878,8 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
 
   // ---- replay: u mod q of the surviving moduli from (u0, v0) and the (p, b) history.
   // Invariant (U, V) = s * (u_i, v_i) mod q; each step (U, V, s) <- (V p, U - b V, s p) / R.
-  // Moduli below 2^30 keep U, V, s lazily in [0, 2q) (bn V + U < 2q^2 + 2q < q 2^32, so the
-  // REDC without its final subtraction stays below 2q).  The surviving moduli are first
+  // Moduli below 2^30 keep U, V, s lazily in [0, 2q) (bn V + U < 4q^2 + 2q < q 2^32, as
+  // redc_lazy asks).  The surviving moduli are first
   // listed in ibuf (shared, nloc words), so that thread t replays survivors t, t + T, ...
   // with every lane busy; the history is read in chunks of REPLAY_CHUNK entries that the
   // whole CTA stages into shared memory (hbuf), so every step reads a broadcast from shared
@@ -918,10 +914,8 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
             const int2 h = hb[e];
             const uint32_t pm = (uint32_t)h.x;
             const uint32_t bn = q - (uint32_t)h.y;
-            const uint64_t T2 = (uint64_t)bn * V + U;
             const uint32_t U2 = mont_mul_lazy(V, pm, q, qi);
-            const uint32_t lo = (uint32_t)T2, hi = (uint32_t)(T2 >> 32);
-            V = hi + __umulhi(lo * qi, q) + (lo != 0u);
+            V = redc_lazy((uint64_t)bn * V + U, q, qi);
             sc = mont_mul_lazy(sc, pm, q, qi);
             U = U2;
           }
