@@ -5,18 +5,19 @@
 // Each step takes the quotient Q = rint(f0 * rcp(f1)) from fma_rn(f0, rcp(f1), 1.5 * 2^23) and
 // the remainder fma_rn(-Q, f1, f0); it makes progress (|remainder| < |f1|) and is exact iff Q
 // is within 1 of f0 / f1 (at most 1 at multiples: Q exact) and the remainder is representable:
-//   first part, operands rounded to float: f1 of every 24-bit significand, f0 any float with
-//            f1 < f0 < 2^13 f1 (moduli below 2^30 stop at 2^18, 32-bit moduli at 2^22: ratios
-//            below 2^12 and 2^10).  Scaling both by a power of two changes nothing (one
-//            reciprocal of a normal number, products and sums well inside the range), so f1
-//            in [2^23, 2^24) covers every exponent;
-//   last part, exact operands: 2 <= f1 < f0 < 2^23 with Q below 2^22, and f0 < f1 (the step
-//            after the integer step may start there): Q of 0 or 1.
+//   first part, quotients from integer remainders rounded to float: f1 of every 24-bit
+//            significand, f0 any float with f1 < f0 < 2^13 f1.  Scaling both by a power of two
+//            changes nothing (one reciprocal of a normal number, products and sums well
+//            inside the range), so f1 in [2^23, 2^24) covers every exponent.  (Larger
+//            quotients have an error of up to 2^-22 of themselves besides: the remainder is
+//            then within 2^-20 of the dividend, which is progress all the same.)
+//   second part, exact operands: 2 <= f1 < f0 < 2^23 with Q below 2^22, and f0 < f1 (the first
+//            step of the part may start there): Q of 0 or 1.
 // On [k f1, (k+1) f1 - 1] the allowed quotients are k at f0 = k f1 and {k, k + 1} above it.
 // For a fixed f1 the estimate is non-decreasing in f0 (every operation is monotone and
 // rcp(f1) is fixed), so it is allowed on the whole interval iff it is at the two ends (the
 // lowest and the highest float in it): checking both ends of every interval, for every f1,
-// covers every pair.  First part: ~1.4e11 end points; last part: ~2.7e8.  The steps run on
+// covers every pair.  First part: ~1.4e11 end points; second part: ~2.7e8.  The steps run on
 // signed remainders; the estimate is odd in each operand (a reciprocal and
 // round-to-nearest-even products), so the positive operands checked here cover the negative
 // ones too.
@@ -66,7 +67,7 @@ __global__ void __launch_bounds__(256) certify_kernel(CertOut* out)
 {
   const uint32_t stride = gridDim.x * blockDim.x;
   unsigned long long n = 0;
-  // last part: 2 <= r1 < r0 < 2^23
+  // second part: 2 <= r1 < r0 < 2^23
   constexpr uint32_t C_TOP = (1u << 23) - 1u;
   for (uint32_t r1 = 2u + blockIdx.x * blockDim.x + threadIdx.x; r1 <= C_TOP; r1 += stride) {
     for (uint32_t k = 1; k <= C_TOP / r1; ++k) {

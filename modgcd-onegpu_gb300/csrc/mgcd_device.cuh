@@ -75,9 +75,10 @@ __device__ __forceinline__ float rcp_approx(float y)
   return r;
 }
 
-// Exact inverse by integer-only extended Euclid; the fallback that runs only if the fast
-// routine's self-check ever fails.  Cofactors as magnitudes (at most q), signs alternating.
-// Inline: a call here made the kernels keep their state in callee-saved registers.
+// Exact inverse by integer-only extended Euclid; the fallback for the operands whose quotients
+// the fast routine cannot hold (its self-check fails).  Cofactors as magnitudes (at most q),
+// signs alternating.  Inline: a call here made the kernels keep their state in callee-saved
+// registers.
 __device__ __forceinline__ uint32_t inv_mod_slow(uint32_t x, uint32_t q)
 {
   uint32_t r0 = q, r1 = x, s0 = 0u, s1 = 1u;
@@ -93,103 +94,91 @@ __device__ __forceinline__ uint32_t inv_mod_slow(uint32_t x, uint32_t q)
 }
 
 // Quotient estimate of the inverse's Euclid steps (also run by the certification kernel):
-// Q = rint(f0 / f1), |Q| < 2^22, read from the mantissa of f0 * rcp(f1) + 1.5 * 2^23; returns
-// the float whose low mantissa bits hold Q.
+// Q = rint(f0 / f1), |Q| < 2^22, read from the mantissa of f0 * rcp(f1) + 1.5 * 2^23 as two's
+// complement; inv_quot returns the float whose low mantissa bits hold Q.
 constexpr float INV_MAGIC = 12582912.0f;     // 1.5 * 2^23
+constexpr uint32_t INV_MAGIC_BITS = 0x4B400000u;
 __device__ __forceinline__ float inv_quot(float f0, float f1)
 {
   return __fmaf_rn(f0, rcp_approx(f1), INV_MAGIC);
 }
 
-// One Euclid step (f0, s0) -= Q (f1, s1) where `on`; the caller alternates the roles.
-__device__ __forceinline__ void inv_step(float& f0, float f1, float& s0, float s1, bool on)
+// A step on integer remainders (with their floats, rounded) and one on float remainders
+// (exact), the cofactors modulo 2^32; only where `on`.  The caller alternates the roles.
+__device__ __forceinline__ void inv_step_int(uint32_t& r0, uint32_t r1, float& f0, float f1, uint32_t& s0, uint32_t s1,
+                                             bool on)
 {
-  const float nq = INV_MAGIC - inv_quot(f0, f1);
+  const uint32_t Q = __float_as_uint(inv_quot(f0, f1)) - INV_MAGIC_BITS;
   if (on) {
-    f0 = __fmaf_rn(nq, f1, f0);
-    s0 = __fmaf_rn(nq, s1, s0);
+    r0 -= Q * r1;
+    s0 -= Q * s1;
+    f0 = __int2float_rn((int32_t)r0);
   }
 }
 
-// Euclid steps on (f0, f1) with cofactors (s0, s1) while both remainders are above `lim` in
-// magnitude (a lane that is done keeps its values through the rest of a trip: predicated
-// steps, two to a branch).
-__device__ __forceinline__ void inv_steps(float& f0, float& f1, float& s0, float& s1, float lim)
+__device__ __forceinline__ void inv_step(float& f0, float f1, uint32_t& s0, uint32_t s1, bool on)
 {
-  bool on = fabsf(f0) > lim && fabsf(f1) > lim;
-#pragma unroll 1
-  while (on) {
-    inv_step(f0, f1, s0, s1, on);
-    on = fabsf(f0) > lim;
-    inv_step(f1, f0, s1, s0, on);
-    on = on && fabsf(f1) > lim;
+  const float qm = inv_quot(f0, f1);
+  if (on) {
+    f0 = __fmaf_rn(INV_MAGIC - qm, f1, f0);
+    s0 -= (__float_as_uint(qm) - INV_MAGIC_BITS) * s1;
   }
 }
 
 // s with s x == +-1 (mod q), as a signed value modulo 2^32, for 0 < x < q, q an odd prime:
 // extended Euclid on (q, x) with nearest-integer quotients (remainders of either sign; about
-// 13 steps for 32-bit operands, 10.7 for 27, 8.7 for 22), every step in floats.
-//   1. On the operands rounded to float (f = r + e).  A remainder is a multiple of its
-//      divisor's ulp and below it in magnitude, so each step is exact: it is the Euclid of
-//      the rounded operands, and its steps are a unimodular map of the true ones.  The
-//      cofactors s stay below q / lim in magnitude, so a true remainder is within
-//      2^-24 q (2 q / lim) of its float: it stops once the smaller one is below lim.
-//   2. The two remainders r = S x - A q exactly, modulo 2^32, A = rint((S x - f) / q) (S x =
-//      r + A q: the estimate is off by |e| / q plus rounding, far below 1/2), and one step on
-//      them in integers, since the larger one may be far above lim: Q from the float of the
-//      larger, so |r2| <= |r1| / 2 + |e| + 2^-22 q.
-//   3. The rest exactly: r1, r2 < 2^22 (LIM22: lim = 2^22, q < 2^32; 2^18, q < 2^30), so
-//      remainders and cofactors are exact in float.  Only r2's cofactor B is carried; r1's is
-//      A = (1 - B r2) / r1, exact to the nearest integer below 2^20 and put right by one
-//      integer step above.
-// Moduli below 2^22 are exact in float from the start and need only 3.
-// What bounds it: instruction issue (87 % of the issue slots in a full SM).  Against the
-// version with integer remainders above 2^22 and integer cofactors, in a loop of dependent
-// inverses: 483 -> 303 issue slots per warp and 2,033 -> 1,458 cycles latency at 32 bits,
-// 314 -> 258 and 1,395 -> 1,198 at 27, 241 -> 172 and 1,101 -> 844 at 22.
-template <bool LIM22>
+// 13 steps for 32-bit operands, 10.7 for 27, 8.7 for 22), s_k x == r_k (mod q) throughout.
+//   1. Until both remainders are below 2^23: integer remainders (the first two are unsigned,
+//      every later one fits a signed word), quotients from their floats.  Operands rounded to
+//      float and a reciprocal good to 1 ulp leave the quotient within 1/2 + 2^-22 Q of the
+//      ratio, so the larger remainder shrinks in every step.
+//   2. Below 2^23 remainders are exact in float: the quotient, and the remainder by one FMA.
+// Quotients of 2^22 or more (a remainder that small against the other: about one inverse in
+// 10^6 at 32 bits) are not held; the caller's check then fails.  Steps are predicated, two to
+// a branch (UNROLL pairs in part 2): a lane that is done keeps its values.
+// What bounds it: instruction issue (87 % of the issue slots in a full SM).  In a loop of
+// dependent inverses, issue slots per warp inverse and latency in cycles: 271 and 1,136 at
+// 32 bits, 218 and 890 at 27, 169 and 698 at 22; a version whose first part ran on the
+// rounded operands alone (all float, the remainders rebuilt from the cofactors) took 287 and
+// 1,407, 245 and 1,151, 163 and 804.
+template <int UNROLL>
 __device__ __forceinline__ uint32_t inv_euclid(uint32_t x, uint32_t q)
 {
-  const float fq = __uint2float_rn(q), fx = __uint2float_rn(x);
-  float g0 = fq, g1 = fx, b0 = 0.0f, b1 = 1.0f;
-  if (!LIM22 && q < (1u << 22)) {
-    inv_steps(g0, g1, b0, b1, 1.0f);
-    const bool z = fabsf(g0) == 1.0f;
-    return (uint32_t)__float2int_rn((z ? g0 : g1) * (z ? b0 : b1));
+  constexpr float TOP = 8388608.0f;               // 2^23
+  uint32_t r0 = q, r1 = x, s0 = 0u, s1 = 1u;
+  float f0 = __uint2float_rn(q), f1 = __uint2float_rn(x);
+  bool on = f0 >= TOP;
+#pragma unroll 1
+  while (on) {
+    inv_step_int(r0, r1, f0, f1, s0, s1, true);
+    on = fabsf(f1) >= TOP;
+    inv_step_int(r1, r0, f1, f0, s1, s0, on);
+    on = on && fabsf(f0) >= TOP;
   }
-  constexpr float lim = LIM22 ? 4194304.0f : 262144.0f;
-  inv_steps(g0, g1, b0, b1, lim);
-  const bool sw = fabsf(g0) < fabsf(g1);
-  const float fb = sw ? g1 : g0, fs = sw ? g0 : g1, sb = sw ? b1 : b0, ss = sw ? b0 : b1;
-  const float iq = rcp_approx(fq);
-  const uint32_t S0 = (uint32_t)__float2int_rn(sb), S1 = (uint32_t)__float2int_rn(ss);
-  const uint32_t A0 = (uint32_t)__float2int_rn(__fmaf_rn(sb, fx, -fb) * iq);
-  const uint32_t A1 = (uint32_t)__float2int_rn(__fmaf_rn(ss, fx, -fs) * iq);
-  const uint32_t r1 = S1 * x - A1 * q;
-  g0 = __int2float_rn((int32_t)r1);
-  const uint32_t Q = (uint32_t)__float2int_rn(fb * rcp_approx(g0));
-  const uint32_t r2 = S0 * x - A0 * q - Q * r1;
-  const uint32_t S2 = S0 - Q * S1;
-  g1 = __int2float_rn((int32_t)r2);
-  b0 = 0.0f;
-  b1 = 1.0f;
-  inv_steps(g0, g1, b0, b1, 1.0f);
-  const bool z = fabsf(g0) == 1.0f;
-  const float b = (z ? g0 : g1) * (z ? b0 : b1);
-  const float i1 = rcp_approx(__int2float_rn((int32_t)r1));
-  const uint32_t B = (uint32_t)__float2int_rn(b);
-  uint32_t A = (uint32_t)__float2int_rn(__fmaf_rn(-b, __int2float_rn((int32_t)r2), 1.0f) * i1);
-  if (LIM22) A -= (uint32_t)__float2int_rn(__int2float_rn((int32_t)(A * r1 + B * r2 - 1u)) * i1);
-  return A * S1 + B * S2;
+  on = fabsf(f0) > 1.0f && fabsf(f1) > 1.0f;
+#pragma unroll 1
+  while (on) {
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      inv_step(f0, f1, s0, s1, on);
+      on = on && fabsf(f0) > 1.0f;
+      inv_step(f1, f0, s1, s0, on);
+      on = on && fabsf(f1) > 1.0f;
+    }
+  }
+  const bool z = fabsf(f0) == 1.0f;
+  const uint32_t s = z ? s0 : s1;
+  return (z ? f0 : f1) < 0.0f ? 0u - s : s;       // s x == -1
 }
 
 // x^{-1} mod q for 0 < x < q, q an odd prime < 2^32 (inv_euclid).  |s| < q, so s is either
 // the 32-bit value read as unsigned or that minus 2^32 (possible only for q > 2^31); the
-// candidate whose product with x is 1 is taken, and if neither is (never observed), the
-// integer-only routine recomputes it, so no float error can reach a result.
+// candidate whose product with x is 1 is taken, and if neither is, the integer-only routine
+// recomputes it, so no float error can reach a result.
+template <int UNROLL = 1>
 __device__ __forceinline__ uint32_t inv_mod(uint32_t x, uint32_t q, uint32_t qinv)
 {
-  const uint32_t s = inv_euclid<true>(x, q);
+  const uint32_t s = inv_euclid<UNROLL>(x, q);
   // inv * x == 1 (mod q)  <=>  redc(inv * x) == redc(1)
   const uint32_t one = redc(1ull, q, qinv);
   if (q < 0x80000000u) {
@@ -206,12 +195,11 @@ __device__ __forceinline__ uint32_t inv_mod(uint32_t x, uint32_t q, uint32_t qin
   return inv_mod_slow(x, q);
 }
 
-// x^{-1} mod q for 0 < x < q < 2^30 (the moduli of widths up to 30 bits): the rounded
-// operands' errors are smaller, so the first part of inv_euclid goes down to 2^18.  The
-// result is checked as inv_mod's is, with the same integer-only fallback.
+// The same for q < 2^31, where s has one reading.
+template <int UNROLL = 1>
 __device__ __forceinline__ uint32_t inv_mod_narrow(uint32_t x, uint32_t q, uint32_t qinv)
 {
-  const uint32_t s = inv_euclid<false>(x, q);
+  const uint32_t s = inv_euclid<UNROLL>(x, q);
   const uint32_t one = redc(1ull, q, qinv);
   const uint32_t inv = (int32_t)s < 0 ? s + q : s;
   if (redc((uint64_t)inv * x, q, qinv) == one) return inv;
@@ -272,18 +260,17 @@ __device__ __forceinline__ void warp_min_key(uint32_t& hi, uint32_t& lo)
 //   t' = p / (t - b)  (mod q)   since t' = u'/v' = v / ((u - b v)/p)
 // with t = INF -> 0 (v was 0: u' = 0, v' = u/p), t == b -> INF (v' = 0), degenerate and
 // retired states fixed; the pivot's own modulus retires.
-// narrow: q < 2^30 (the shorter inverse, inv_mod_narrow).
+// narrow: q < 2^30.  A pivot p < 2^32 enters the product as it is (p inv < q 2^32).
 __device__ __forceinline__ uint32_t t_update(uint32_t t, uint32_t q, uint32_t qinv, uint32_t p, int32_t b,
                                              bool narrow)
 {
   if (t >= T_MARK) return (t == T_INF) ? 0u : t;
   if (q == p) return T_RETIRED;
-  const uint32_t pm = (p > q) ? p - q : p;
   const uint32_t d = mod_sub(t, from_signed(b, q), q);
   if (d == 0u) return T_INF;
-  // redc(d) = d/R, inv = R/d, mont_mul(pm, R/d) = pm/d
+  // redc(d) = d/R, inv = R/d, mont_mul(p, R/d) = p/d
   const uint32_t x = redc((uint64_t)d, q, qinv);
-  return mont_mul(pm, narrow ? inv_mod_narrow(x, q, qinv) : inv_mod(x, q, qinv), q, qinv);
+  return mont_mul(p, narrow ? inv_mod_narrow<2>(x, q, qinv) : inv_mod<2>(x, q, qinv), q, qinv);
 }
 
 // The same update for K pairs that share the modulus q (slot s uses pivot (p[s], b[s]);
