@@ -477,7 +477,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
     bk.csize = cs;
     bk.smem = cluster_batch_smem_bytes(cs, bk.nq_max, 1);
     int nc = 0;
-    if (bk.smem > room || cluster_batch_max_clusters(bk.threads, 1, cs, bk.smem, &nc) != cudaSuccess || nc < 1)
+    if (bk.smem > room || cluster_batch_max_clusters(bk.threads, 1, c->L <= 30, cs, bk.smem, &nc) != cudaSuccess || nc < 1)
       return MGCD_ERR_GRID;
     bk.grid = (int)std::min<size_t>(v.size(), (size_t)nc);
     scratch += (size_t)bk.grid * 4 * bk.nq_max;
@@ -536,7 +536,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       bk.csize = cs;
       bk.smem = cluster_batch_smem_bytes(cs, bk.nq_max, bk.k);
       int nc = 0;
-      if (bk.smem > room || cluster_batch_max_clusters(bk.threads, bk.k, cs, bk.smem, &nc) != cudaSuccess || nc < 1)
+      if (bk.smem > room || cluster_batch_max_clusters(bk.threads, bk.k, c->L <= 30, cs, bk.smem, &nc) != cudaSuccess || nc < 1)
         return MGCD_ERR_GRID;
       bk.grid = (int)std::min<size_t>((v.size() + bk.k - 1) / bk.k, (size_t)nc);
       scratch += (size_t)bk.grid * 4 * bk.k * bk.nq_max;

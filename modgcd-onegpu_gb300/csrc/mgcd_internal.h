@@ -24,6 +24,9 @@ struct PairDesc {
                      // count; <= nq: no growth)
 };
 
+// Largest moduli count of a pair that runs on one CTA (size classes 0-2).
+constexpr uint32_t CTA_MAX_NQ = 16384;
+
 // Device-side mixed-radix conversion (mgcd_radix_dev.cu): pairs with up to RADIX_MAX
 // digits are converted on the GPU; glen = RADIX_HOST marks a pair left to the host
 // (more digits, or a failed pair).
@@ -162,7 +165,7 @@ cudaError_t launch_cluster(const GridArgs& a, int threads, int ctas, size_t smem
 // clusters of `csize` CTAs each pull pairs from the queue, k pairs per cluster in lockstep
 // (k = 1: any CTA size; k = 2, 4: 256 or 512 threads).  a.scratch_words = 4 * k * nq_max.
 size_t cluster_batch_smem_bytes(int csize, uint32_t nq_max, int k);
-cudaError_t cluster_batch_max_clusters(int threads, int k, int csize, size_t smem, int* clusters);
+cudaError_t cluster_batch_max_clusters(int threads, int k, bool narrow, int csize, size_t smem, int* clusters);
 cudaError_t launch_cluster_batch(const BatchArgs& a, int threads, int k, int csize, int clusters, size_t smem,
                                  cudaStream_t s, bool after = false);
 

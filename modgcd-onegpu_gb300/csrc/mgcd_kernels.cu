@@ -257,7 +257,7 @@ __device__ __forceinline__ uint32_t grow_step_for(uint32_t cap, uint32_t permill
 // slots take newly published entries while the others run, and a CTA whose slots stay
 // empty for a.idle_ns leaves.
 template <int T, int K, bool NARROW = false, bool RING = false>
-__global__ void __launch_bounds__(T) batchk_kernel(const BatchArgs a)
+__global__ void __launch_bounds__(T, K < 8 ? 1024 / T : 1) batchk_kernel(const BatchArgs a)
 {
   constexpr int NW = T / 32;
   static_assert(NW >= K, "one warp per slot reduces the slot's pivot");
@@ -494,6 +494,8 @@ __global__ void __launch_bounds__(T) batchk_kernel(const BatchArgs a)
   // ---- position layout
   __shared__ uint32_t bucket[1u << K];
   __shared__ uint32_t live_pos;
+  __shared__ uint32_t cmask[CTA_MAX_NQ / 128];         // a byte per 32 positions: the slots live in
+                                                       // any of them at the last re-layout
   for (uint32_t pos = threadIdx.x; pos < NQS; pos += T) pmod[pos] = (uint16_t)pos;
   auto state_at = [&](int s, uint32_t pos, uint32_t m) -> uint32_t {
     const uint32_t* ts = tS + (size_t)s * NQS;
@@ -507,6 +509,7 @@ __global__ void __launch_bounds__(T) batchk_kernel(const BatchArgs a)
     // active slot, and dead states stay dead (a slot becomes active again only as a fresh one)
     const uint32_t lim = fresh ? NQS : npos;
     if (threadIdx.x < (1u << K)) bucket[threadIdx.x] = 0u;
+    if (threadIdx.x < CTA_MAX_NQ / 128) cmask[threadIdx.x] = 0u;
     __syncthreads();
     const uint32_t below = (1u << lane) - 1u;
     for (uint32_t base = 0; base < lim; base += T) {
@@ -542,7 +545,13 @@ __global__ void __launch_bounds__(T) batchk_kernel(const BatchArgs a)
       const uint32_t grp = __match_any_sync(0xFFFFFFFFu, set);
       const int lead = __ffs((int)grp) - 1;
       uint32_t r0 = 0u;
-      if (in && lane == lead) r0 = atomicAdd(&bucket[set], (uint32_t)__popc(grp));
+      if (in && lane == lead) {
+        const uint32_t n = (uint32_t)__popc(grp);
+        r0 = atomicAdd(&bucket[set], n);
+        const uint32_t ca = r0 >> 5, cb = (r0 + n - 1u) >> 5;   // the new positions' one or two chunks
+        atomicOr(&cmask[ca >> 2], set << (8u * (ca & 3u)));
+        if (cb != ca) atomicOr(&cmask[cb >> 2], set << (8u * (cb & 3u)));
+      }
       r0 = __shfl_sync(0xFFFFFFFFu, r0, lead);
       if (in) aux[pos] = (uint16_t)(r0 + __popc(grp & below));
     }
@@ -698,21 +707,21 @@ __global__ void __launch_bounds__(T) batchk_kernel(const BatchArgs a)
     constexpr bool PREFETCH = K <= MGCD_PREFETCH_MAX_K;
     ModConst cn{};
     if constexpr (PREFETCH) cn = a.mods[pmod[threadIdx.x < npos ? threadIdx.x : 0u]];
-    for (uint32_t j = threadIdx.x; j < npos; j += T) {
+    for (uint32_t j = threadIdx.x; (j & ~31u) < npos; j += T) {   // whole warps
+      const bool in = j < npos;
       ModConst c;
       if constexpr (PREFETCH) {
         c = cn;
         if (j + T < npos) cn = a.mods[pmod[j + T]];
       } else {
-        c = a.mods[pmod[j]];
+        c = a.mods[pmod[in ? j : 0u]];
       }
-      uint32_t m = 0, tv[K];
+      const uint32_t m = (cmask[j >> 7] >> ((j >> 2) & 24u)) & active;   // byte j / 32
+      if (!m) continue;
+      uint32_t tv[K];
 #pragma unroll
-      for (int s = 0; s < K; ++s) {                   // (states beyond a pair's moduli are retired)
-        const bool on = (active >> s) & 1u;
-        m |= (uint32_t)on << s;
-        tv[s] = on ? tS[(size_t)s * NQS + j] : T_RETIRED;
-      }
+      for (int s = 0; s < K; ++s)                     // (states beyond a pair's moduli are retired)
+        if ((m >> s) & 1u) tv[s] = in ? tS[(size_t)s * NQS + j] : T_RETIRED;
       if (a.phases) {                                 // liveness accounting (thread-rounds)
         uint32_t fin = 0;
 #pragma unroll
@@ -720,17 +729,10 @@ __global__ void __launch_bounds__(T) batchk_kernel(const BatchArgs a)
         lv_any += fin != 0u;
         lv_fin += fin;
       }
-      if (!m) continue;
-      if constexpr (NARROW) t_update_k_narrow<K>(tv, c, p, b, m);
-      else t_update_k<K>(tv, c, p, b, m);
-#pragma unroll
-      for (int s = 0; s < K; ++s) {
-        if (!((m >> s) & 1u)) continue;
-        tS[(size_t)s * NQS + j] = tv[s];
-        uint32_t h, l;
-        t_key(tv[s], c.q, h, l);
-        if (key_less(h, l, kh[s], kl[s])) { kh[s] = h; kl[s] = l; }
-      }
+      t_update_k<K, NARROW>(tv, m, c, p, b, [&](int s, uint32_t t) {
+        if (in) tS[(size_t)s * NQS + j] = t;
+        t_key_min(t, c.q, kh[s], kl[s]);
+      });
     }
     if (a.phases) {
       const uint32_t wa = __reduce_add_sync(0xFFFFFFFFu, lv_any), wf = __reduce_add_sync(0xFFFFFFFFu, lv_fin);
@@ -841,8 +843,9 @@ __device__ __forceinline__ bool cluster_min_keys(uint32_t (&kh)[K], uint32_t (&k
   return cs.dead == 0u;
 }
 
-template <int T, int K>
-__global__ void __launch_bounds__(T) cluster_batchk_kernel(const BatchArgs a)
+// NARROW: moduli below 2^30, as in batchk_kernel.
+template <int T, int K, bool NARROW>
+__global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
 {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ SlotSmem<K> ss;
@@ -1000,25 +1003,17 @@ __global__ void __launch_bounds__(T) cluster_batchk_kernel(const BatchArgs a)
       if ((active >> s) & 1u) nmax = max(nmax, ck.nloc[s]);
       kh[s] = kl[s] = 0xFFFFFFFFu;
     }
-    for (uint32_t j = threadIdx.x; j < nmax; j += T) {
-      uint32_t m = 0, tv[K];
+    for (uint32_t j = threadIdx.x; (j & ~31u) < nmax; j += T) {   // whole warps
+      const bool in = j < nmax;
+      uint32_t tv[K];
 #pragma unroll
-      for (int s = 0; s < K; ++s) {
-        const bool on = ((active >> s) & 1u) && j < ck.nloc[s];
-        m |= (uint32_t)on << s;
-        tv[s] = on ? tS[(size_t)s * per + j] : T_RETIRED;
-      }
-      if (!m) continue;
-      const ModConst c = a.mods[j0 + j];
-      t_update_k<K>(tv, c, p, b, m);
-#pragma unroll
-      for (int s = 0; s < K; ++s) {
-        if (!((m >> s) & 1u)) continue;
-        tS[(size_t)s * per + j] = tv[s];
-        uint32_t h, l;
-        t_key(tv[s], c.q, h, l);
-        if (key_less(h, l, kh[s], kl[s])) { kh[s] = h; kl[s] = l; }
-      }
+      for (int s = 0; s < K; ++s)
+        tv[s] = ((active >> s) & 1u) && j < ck.nloc[s] ? tS[(size_t)s * per + j] : T_RETIRED;
+      const ModConst c = a.mods[in ? j0 + j : 0u];
+      t_update_k<K, NARROW>(tv, active, c, p, b, [&](int s, uint32_t t) {
+        if (j < ck.nloc[s]) tS[(size_t)s * per + j] = t;
+        t_key_min(t, c.q, kh[s], kl[s]);
+      });
     }
     if (!cluster_min_keys<T, K>(kh, kl, ss, ck, cs, kepoch)) {
       if (r == 0 && threadIdx.x < K && ((valid >> threadIdx.x) & 1u)) {
@@ -1351,26 +1346,33 @@ static cudaError_t prepare_cluster_fn(const void* fn, int csize, size_t smem)
   return e;
 }
 
-static const void* cluster_batch_fn_k(int threads, int k)
+template <bool NARROW>
+static const void* cluster_batchk_fn_for(int threads, int k)
 {
-  if (k == 1) return reinterpret_cast<const void*>(&cluster_batch_kernel);
   if (k == 2) {
     switch (threads) {
-      case 256: return reinterpret_cast<const void*>(&cluster_batchk_kernel<256, 2>);
-      case 512: return reinterpret_cast<const void*>(&cluster_batchk_kernel<512, 2>);
-      case 1024: return reinterpret_cast<const void*>(&cluster_batchk_kernel<1024, 2>);
+      case 256: return reinterpret_cast<const void*>(&cluster_batchk_kernel<256, 2, NARROW>);
+      case 512: return reinterpret_cast<const void*>(&cluster_batchk_kernel<512, 2, NARROW>);
+      case 1024: return reinterpret_cast<const void*>(&cluster_batchk_kernel<1024, 2, NARROW>);
       default: return nullptr;
     }
   }
   if (k == 4) {
     switch (threads) {
-      case 256: return reinterpret_cast<const void*>(&cluster_batchk_kernel<256, 4>);
-      case 512: return reinterpret_cast<const void*>(&cluster_batchk_kernel<512, 4>);
-      case 1024: return reinterpret_cast<const void*>(&cluster_batchk_kernel<1024, 4>);
+      case 256: return reinterpret_cast<const void*>(&cluster_batchk_kernel<256, 4, NARROW>);
+      case 512: return reinterpret_cast<const void*>(&cluster_batchk_kernel<512, 4, NARROW>);
+      case 1024: return reinterpret_cast<const void*>(&cluster_batchk_kernel<1024, 4, NARROW>);
       default: return nullptr;
     }
   }
   return nullptr;
+}
+
+// narrow: the context's moduli are below 2^30 (width <= 30)
+static const void* cluster_batch_fn_for(int threads, int k, bool narrow)
+{
+  if (k == 1) return reinterpret_cast<const void*>(&cluster_batch_kernel);
+  return narrow ? cluster_batchk_fn_for<true>(threads, k) : cluster_batchk_fn_for<false>(threads, k);
 }
 
 size_t cluster_batch_smem_bytes(int csize, uint32_t nq_max, int k)
@@ -1379,9 +1381,9 @@ size_t cluster_batch_smem_bytes(int csize, uint32_t nq_max, int k)
   return sizeof(uint32_t) * ((size_t)(k > 1 ? k + 1 : 2) * per + STAGE_SMEM_WORDS);
 }
 
-cudaError_t cluster_batch_max_clusters(int threads, int k, int csize, size_t smem, int* clusters)
+cudaError_t cluster_batch_max_clusters(int threads, int k, bool narrow, int csize, size_t smem, int* clusters)
 {
-  const void* fn = cluster_batch_fn_k(threads, k);
+  const void* fn = cluster_batch_fn_for(threads, k, narrow);
   cudaError_t e = prepare_cluster_fn(fn, csize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
@@ -1403,7 +1405,7 @@ cudaError_t launch_cluster(const GridArgs& a, int threads, int ctas, size_t smem
 cudaError_t launch_cluster_batch(const BatchArgs& a, int threads, int k, int csize, int clusters, size_t smem,
                                  cudaStream_t s, bool after)
 {
-  const void* fn = cluster_batch_fn_k(threads, k);
+  const void* fn = cluster_batch_fn_for(threads, k, a.L <= 30);
   cudaError_t e = prepare_cluster_fn(fn, csize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[2];

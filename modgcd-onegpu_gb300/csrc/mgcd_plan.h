@@ -51,7 +51,6 @@ struct Bucket {
 // or a serving lane asks for one); larger pairs K per thread-block cluster.
 constexpr int NSTREAMS = MGCD_NUM_SIZE_CLASSES;
 constexpr int CLUSTER_CLASS = 3;
-constexpr uint32_t CTA_MAX_NQ = 16384;
 constexpr size_t INVTAB_N = 16384;        // moduli covered by the pairwise inverse table
 
 inline int size_class(uint32_t nq) { return nq <= 1024 ? 0 : nq <= 4096 ? 1 : nq <= CTA_MAX_NQ ? 2 : CLUSTER_CLASS; }
