@@ -486,7 +486,10 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
     P.grid_scratch_off = scratch;
     return MGCD_OK;
   }
-  const uint32_t plain_cta_max = 256;   // single pairs: one CTA, else a cluster or a grid
+  // Single pairs: one CTA, whose exchange is one barrier, while its moduli leave the SM's issue
+  // slots free (512 moduli: 326 us on a CTA, 355 on a cluster; 768: 655 and 594); above that a
+  // cluster or a grid.
+  const uint32_t plain_cta_max = 512;
   std::vector<uint32_t> byb[NSTREAMS];
   for (uint32_t k : subset) {
     const uint32_t nq = descs[k].nq;
@@ -514,7 +517,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       for (size_t i = 0; i < v.size(); ++i) v[i] = key[i].second;
     }
     Bucket bk;
-    bk.threads = plain ? single_threads(plain_cta_max) : c->cfg[b].threads;
+    bk.threads = plain ? single_threads(descs[v[0]].nq) : c->cfg[b].threads;
     bk.k = plain ? 1 : c->cfg[b].k;
     bk.csize = 0;
     bk.cls = b;
@@ -666,11 +669,11 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     g.iters = P.d_iters.as<uint32_t>() + k;
     g.status = P.d_status.as<int32_t>() + k;
     const bool ref_shape = c->single_policy == MGCD_SINGLE_REFERENCE_SHAPE;
-    if (!ref_shape && d.nq <= (uint32_t)MAX_CLUSTER * 512) {
-      // thread-block cluster: as many CTAs (<= 16) as keep one modulus per thread, up to 512
-      // threads per CTA (with 1024-thread CTAs the cluster's two-level exchange measured
-      // slower than the grid's leader exchange: 16.8 vs 16.5 ms at 9,728 moduli, 20.8 vs
-      // 19.0 ms at 11,264; at 8,192 moduli the 512-thread cluster wins, 13.0 vs 14.0 ms)
+    if (!ref_shape && d.nq <= (uint32_t)MAX_CLUSTER * 1024) {
+      // thread-block cluster while one modulus per thread fits 16 CTAs: its exchange takes a
+      // third of the grid's, which outweighs the fuller CTAs (32-bit moduli, cluster / grid:
+      // 9,472 moduli 12.4 / 17.2 ms, 13,312 20.7 / 24.9, 15,872 27.0 / 29.7; with two moduli
+      // per thread, 18,432, 45.3 / 34.6)
       const int ctas = (int)std::min<uint32_t>(MAX_CLUSTER, (d.nq + 255) / 256);
       const uint32_t per = (d.nq + ctas - 1) / ctas;
       g.per_cta = per;
