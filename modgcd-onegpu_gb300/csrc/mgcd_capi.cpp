@@ -244,6 +244,7 @@ int mgcd_create(int device, int L, mgcd_context** out)
     cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
   if (rc == MGCD_OK && c->main.create() != cudaSuccess) rc = MGCD_ERR_CUDA;
+  c->main.spread = true;
   cudaStream_t s = c->main.stream;
   if (rc == MGCD_OK && c->mods.grow(mc.size() * sizeof(ModConstHost), c->pool, s) != cudaSuccess) rc = MGCD_ERR_CUDA;
   if (rc == MGCD_OK &&
@@ -448,6 +449,39 @@ int mgcd::plan_batch(mgcd_context* c, Plan& P, size_t np, const uint32_t* limbs,
 // warp more for the pair's bookkeeping (run_pair), while they fit.
 static int single_threads(uint32_t per) { return (int)std::min<uint32_t>(1024, (per + 31) / 32 * 32 + 32); }
 
+// Launch shape of a class's n pairs in a batch too small to fill the GPU: CTAs per cluster and
+// pairs per cluster within `budget` SMs, or {0, 0} to keep the class's K pairs per CTA.  The
+// pairs' loops then bound the batch, so the shape is the one with the shortest iterations,
+// by what they measured: a chunk of 32 moduli takes its SMSP 230 cycles for the shared inverse
+// and 60 per slot, at least a chain of ~1,500 cycles, and the exchange 900 and 150 per slot;
+// clusters that do not fit at once run one after another.
+struct SmallShape { int cs, k; };
+static SmallShape small_batch_shape(const mgcd_context* c, size_t n, uint32_t nq_max, int budget, bool clusters_only)
+{
+  SmallShape best{0, 0};
+  double best_cost = 1e30;
+  for (int cs = 2; cs <= MAX_CLUSTER; cs *= 2) {
+    const uint32_t per = (nq_max + cs - 1) / cs;
+    if (cs > 2 && per < 128) break;
+    for (int k = 1; k <= 4; k *= 2) {
+      const size_t need = (n + k - 1) / k;
+      const int threads = k == 1 ? single_threads(per) : per <= 256 ? 256 : per <= 512 ? 512 : 1024;
+      const size_t smem = cluster_batch_smem_bytes(cs, nq_max, k);
+      int nc = 0;
+      if (smem > c->smem_optin - 24576 ||
+          cluster_batch_max_clusters(threads, k, c->L <= 30, cs, smem, &nc) != cudaSuccess || nc < 1)
+        continue;
+      nc = std::min(nc, budget / cs);
+      if (nc < 1 || (!clusters_only && (size_t)nc < need)) continue;
+      const double waves = (double)((need + nc - 1) / nc);
+      const double update = std::max(1500.0, std::ceil(((per + 31) / 32) / 4.0) * (230.0 + 60.0 * k));
+      const double cost = waves * (update + 900.0 + 150.0 * k);
+      if (cost < best_cost) { best_cost = cost; best = {cs, k}; }
+    }
+  }
+  return best;
+}
+
 // Groups the pairs `subset` (indices into descs) into size-class buckets (batches) or
 // single-pair launches (plain); appends the processing order to P.order and returns the
 // scratch words needed.  `latency`: the few pairs rerun after a scaled batch -- one
@@ -499,9 +533,31 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       byb[size_class(nq)].push_back(k);
     }
   }
+  // A batch of few pairs (at most one per two SMs) leaves most SMs idle with K pairs per CTA,
+  // and its time is its longest pair's: each class, largest first, spreads its pairs over
+  // clusters with its full count while SMs are left for the smaller classes.  61 mixed
+  // pairs 24.3 -> 9.1 ms, 24 of 160-300 kbit 189.8 -> 134.4 ms.  Not in a server's waves, which share
+  // the GPU with the continuous lanes, nor where the table asks for clusters of its own.
+  bool spread = !plain && P.spread && subset.size() <= (size_t)c->sms / 2;
+  for (int b = 0; b < CLUSTER_CLASS; ++b) spread = spread && c->cfg[b].csize == 0;
+  int sms_left = c->sms;
   for (int b = NSTREAMS - 1; b >= 0; --b) {  // largest class first: its pairs are the longest
     auto& v = byb[b];
     if (v.empty()) continue;
+    SmallShape few{0, 0};
+    if (spread) {
+      // the count a grown set may reach, where sets grow: what K pairs per CTA would certify
+      // in the end is certified here too
+      const bool grows = b < CLUSTER_CLASS && c->grow_start > 0.0f;
+      auto count = [&](uint32_t k) { return grows ? std::max(P.ref_nq[k], grow_cap(P.ref_nq[k])) : P.ref_nq[k]; };
+      uint32_t most = 0;
+      for (uint32_t k : v) most = std::max(most, count(k));
+      int budget = sms_left;                 // less one CTA per K pairs of each smaller class
+      for (int x = 0; x < b; ++x) budget -= (int)((byb[x].size() + c->cfg[x].k - 1) / c->cfg[x].k);
+      few = small_batch_shape(c, v.size(), most, budget, b == CLUSTER_CLASS);
+      if (few.cs)
+        for (uint32_t k : v) descs[k].nq = count(k);
+    }
     // longest pairs first: by moduli count, then operand length, both descending (ties by
     // index); the keys are gathered once, which halves the sort's time against a comparator
     // that loads two descriptors per comparison
@@ -526,7 +582,19 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
     bk.nq_max = descs[v[0]].nq;
     bk.scratch_off = scratch;
     const int small_cs = (b > 0 && b < CLUSTER_CLASS) ? P.small_cluster_ctas : 0;
-    if (!plain && (b == CLUSTER_CLASS || c->cfg[b].csize > 0 || small_cs > 0)) {
+    if (few.cs) {
+      bk.k = few.k;
+      bk.csize = few.cs;
+      const uint32_t per = (bk.nq_max + few.cs - 1) / few.cs;
+      bk.threads = few.k == 1 ? single_threads(per) : per <= 256 ? 256 : per <= 512 ? 512 : 1024;
+      bk.smem = cluster_batch_smem_bytes(few.cs, bk.nq_max, few.k);
+      int nc = 0;
+      if (cluster_batch_max_clusters(bk.threads, bk.k, c->L <= 30, bk.csize, bk.smem, &nc) != cudaSuccess || nc < 1)
+        return MGCD_ERR_GRID;
+      bk.grid = (int)std::min<size_t>((v.size() + bk.k - 1) / bk.k, (size_t)nc);
+      scratch += (size_t)bk.grid * 4 * bk.k * bk.nq_max;
+      sms_left -= bk.grid * bk.csize;
+    } else if (!plain && (b == CLUSTER_CLASS || c->cfg[b].csize > 0 || small_cs > 0)) {
       // k pairs per cluster; more CTAs per cluster when a CTA's share of the moduli would
       // not fit its shared memory (24 KB kept for the kernel's static shared memory, which
       // holds the cluster keys and the recovery panel)

@@ -83,6 +83,7 @@ struct Plan {
   uint64_t direct_base = 0;
   bool plain = false;                  // single-pair latency policy
   bool graphable = true;               // may be recorded into a CUDA graph (context setting)
+  bool spread = false;                 // small batches spread their pairs over clusters (schedule)
   int cluster_ctas = 0;                // CTAs per cluster of size class 3 (0: the context's setting)
   int small_cluster_ctas = 0;          // CTAs per cluster for pairs of size classes 1-2 (0: the
                                        // context's setting); serving waves favour latency
