@@ -839,6 +839,140 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
   __syncthreads();
 }
 
+// Recovery (MGCD4) for a pair on one CTA whose moduli are all in the inverse table, in panels
+// of up to 32 digits: the lowest remaining survivors are one warp's lanes, which take digits by
+// the reference's rule among themselves (the lowest nonzero lane is the lowest nonzero modulus
+// overall) without a barrier; then every other survivor applies the panel's digits, each one
+// load from the digit's row of the table and one product.  A panel without digits falls back
+// to one round of the rule over all survivors, which also detects the end.  Digits, their
+// order and the end conditions are those of the per-digit loop below, whose rounds (a
+// barrier, a table row not seen before) took 2,000-3,000 cycles a digit; a panel takes
+// ~200.
+//   ord    the survivors' indices in table order (ns of them), st their values
+//   work   shared, 1,024 words: the panel's pairwise inverses
+template <int T>
+__device__ void recover_cta(const ModConst* __restrict__ mods, const PairDesc& d, uint32_t j0, uint32_t ns, uint32_t* st,
+                            const uint32_t* ord, uint32_t* work, RedSmem& rs, uint32_t& parity, int remaining,
+                            mgcd_pair* digits, uint32_t* count, int32_t* status, InvTab inv)
+{
+  __shared__ uint32_t pidx[32];        // panel lanes: places in ord, ascending
+  __shared__ uint32_t drow[32];        // the panel's digits: table index, value
+  __shared__ int32_t dval[32];
+  __shared__ uint32_t pn, pscan;       // panel size, then the digits it produced; places below are retired
+  const uint32_t TT = cta_threads<T>(), lane = threadIdx.x & 31u;
+  mgcd_pair* const out = digits + d.out_off;
+  uint32_t ndig = 0, scan = 0;
+  for (;;) {
+    // ---- the panel: the first <= 32 remaining survivors
+    if (threadIdx.x < 32u) {
+      uint32_t n = 0;
+      for (uint32_t base = scan; n < 32u && base < ns; base += 32u) {
+        const uint32_t i = base + lane;
+        const bool rem = i < ns && st[ord[i]] != U_RETIRED;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, rem);
+        const uint32_t pos = n + __popc(m & ((1u << lane) - 1u));
+        if (rem && pos < 32u) pidx[pos] = i;
+        n += __popc(m);
+      }
+      if (lane == 0) pn = n < 32u ? n : 32u;
+    }
+    __syncthreads();
+    const uint32_t np = pn;
+    if (np == 0u) break;               // no modulus left (not reached while remaining > 0)
+    const uint32_t next = pidx[np - 1u] + 1u;             // the first survivor past the panel
+    for (uint32_t e = threadIdx.x; e < 32u * np; e += TT) {
+      const uint32_t a = e >> 5, b = e & 31u;             // R / q_a mod q_b
+      if (b < np && a != b) work[e] = __ldg(inv.tab + (size_t)(j0 + ord[pidx[a]]) * inv.n + (j0 + ord[pidx[b]]));
+    }
+    __syncthreads();
+    if (threadIdx.x < 32u) {
+      const bool in = lane < np;
+      const uint32_t place = pidx[in ? lane : 0u], j = ord[place];
+      const ModConst c = mods[j0 + j];
+      uint32_t u = in ? st[j] : 0u;
+      bool live = in;
+      uint32_t nd = 0;
+      int rem = remaining;
+      while (nd < 32u && rem > 0) {
+        const uint32_t nz = __ballot_sync(0xFFFFFFFFu, live && u != 0u);
+        if (!nz) break;
+        const uint32_t src = __ffs((int)nz) - 1u;
+        const int32_t g = __shfl_sync(0xFFFFFFFFu, to_signed(u, c.q), (int)src);
+        if (lane == src) {
+          drow[nd] = j0 + j;
+          dval[nd] = g;
+          out[ndig + nd] = mgcd_pair{c.q, g};
+          live = false;
+        }
+        if (live) u = mont_mul(mod_sub(u, from_signed(g, c.q), c.q), work[32u * src + lane], c.q, c.qinv);
+        ++nd;
+        --rem;
+      }
+      if (in) st[j] = live ? u : U_RETIRED;
+      const uint32_t left = __ballot_sync(0xFFFFFFFFu, live);
+      if (left != 0u && lane == __ffs((int)left) - 1u) pscan = place;
+      if (lane == 0) {
+        pn = nd;
+        if (left == 0u) pscan = next;
+      }
+    }
+    __syncthreads();
+    const uint32_t nd = pn;
+    scan = pscan;
+    if (nd == 0u) {
+      // ---- one round of the rule: the lowest nonzero survivor past the panel, or the end
+      uint32_t kh = 0xFFFFFFFFu, kl = 0u;
+      for (uint32_t i = next + threadIdx.x; i < ns; i += TT) {
+        const uint32_t j = ord[i], u = st[j];
+        if (u != U_RETIRED && u != 0u) { kh = j0 + j; kl = (uint32_t)to_signed(u, mods[j0 + j].q); break; }
+      }
+      block_min_key<T>(kh, kl, rs, parity);
+      if (kh == 0xFFFFFFFFu) {                            // no nonzero value left: done
+        if (ndig == 0u) {                                 // u = 0: one zero digit
+          if (threadIdx.x == 0) out[0] = mgcd_pair{mods[0].q, 0};
+          ndig = 1u;
+        }
+        break;
+      }
+      const uint32_t p = mods[kh].q;
+      const int32_t g = (int32_t)kl;
+      for (uint32_t i = scan + threadIdx.x; i < ns; i += TT) {
+        const uint32_t j = ord[i], u = st[j];
+        if (u == U_RETIRED) continue;
+        if (j0 + j == kh) { st[j] = U_RETIRED; continue; }
+        const ModConst c = mods[j0 + j];
+        st[j] = mont_mul(mod_sub(u, from_signed(g, c.q), c.q), __ldg(inv.tab + (size_t)kh * inv.n + (j0 + j)), c.q,
+                         c.qinv);
+      }
+      if (threadIdx.x == 0) out[ndig] = mgcd_pair{p, g};
+      ++ndig;
+      remaining -= 1;
+    } else {
+      // ---- the panel's digits on every survivor past it
+      for (uint32_t i = next + threadIdx.x; i < ns; i += TT) {
+        const uint32_t j = ord[i];
+        uint32_t u = st[j];
+        if (u == U_RETIRED) continue;
+        const ModConst c = mods[j0 + j];
+        const uint32_t* const col = inv.tab + (j0 + j);
+#pragma unroll 4
+        for (uint32_t k = 0; k < nd; ++k)
+          u = mont_mul(mod_sub(u, from_signed(dval[k], c.q), c.q), __ldg(col + (size_t)drow[k] * inv.n), c.q, c.qinv);
+        st[j] = u;
+      }
+      ndig += nd;
+      remaining -= (int)nd;
+    }
+    __syncthreads();
+    if (remaining <= 0) break;
+  }
+  if (threadIdx.x == 0) {
+    *status = remaining <= 0 ? ST_RECOVERY : ST_OK;
+    *count = ndig;
+  }
+  __syncthreads();
+}
+
 // After the reduction loop of one pair: certification, replay and recovery (MGCD4).
 // st holds the final t states of this CTA's moduli; `remaining` the surviving count;
 // lu, lv (meaningful in bound_thread) the size bounds of the final u and v.
@@ -879,21 +1013,33 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
   // ---- replay: u mod q of the surviving moduli from (u0, v0) and the (p, b) history.
   // Invariant (U, V) = s * (u_i, v_i) mod q; each step (U, V, s) <- (V p, U - b V, s p) / R.
   // Moduli below 2^30 keep U, V, s lazily in [0, 2q) (bn V + U < 4q^2 + 2q < q 2^32, as
-  // redc_lazy asks).  The surviving moduli are first
-  // listed in ibuf (shared, nloc words), so that thread t replays survivors t, t + T, ...
-  // with every lane busy; the history is read in chunks of REPLAY_CHUNK entries that the
-  // whole CTA stages into shared memory (hbuf), so every step reads a broadcast from shared
-  // memory instead of waiting on a global load.
+  // redc_lazy asks).  The surviving moduli are first listed in ibuf (shared, nloc words), in
+  // table order, so that thread t replays survivors t, t + T, ... with every lane busy; the
+  // history is read in chunks of REPLAY_CHUNK entries that the whole CTA stages into shared
+  // memory (hbuf), so every step reads a broadcast from shared memory instead of waiting on a
+  // global load.
   const bool narrow = L <= 30;
   uint32_t ns;                                         // survivors, listed in ibuf
   {
-    __shared__ uint32_t nsurv;
-    if (threadIdx.x == 0) nsurv = 0u;
+    // warp w lists a contiguous range of the moduli, after the counts of the warps before it
+    __shared__ uint32_t wcount[32];
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, nw = TT / 32u;
+    const uint32_t len = (nloc + 32u * nw - 1u) / (32u * nw) * 32u, lo = w * len, hi = min(nloc, lo + len);
+    uint32_t n = 0;
+    for (uint32_t base = lo; base < hi; base += 32u)
+      n += __popc(__ballot_sync(0xFFFFFFFFu, base + lane < hi && st[base + lane] != T_RETIRED));
+    if (lane == 0) wcount[w] = n;
     __syncthreads();
-    for (uint32_t j = threadIdx.x; j < nloc; j += TT)
-      if (st[j] != T_RETIRED) ibuf[atomicAdd(&nsurv, 1u)] = j;
+    const uint32_t cnt = lane < nw ? wcount[lane] : 0u;
+    ns = __reduce_add_sync(0xFFFFFFFFu, cnt);
+    n = __reduce_add_sync(0xFFFFFFFFu, lane < w ? cnt : 0u);
+    for (uint32_t base = lo; base < hi; base += 32u) {
+      const bool in = base + lane < hi && st[base + lane] != T_RETIRED;
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
+      if (in) ibuf[n + __popc(m & ((1u << lane) - 1u))] = base + lane;
+      n += __popc(m);
+    }
     __syncthreads();
-    ns = nsurv;
     int2* const hb = reinterpret_cast<int2*>(hbuf);
     for (uint32_t base = 0; base < ns; base += TT) {
       const bool have = base + threadIdx.x < ns;
@@ -923,8 +1069,7 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
 #pragma unroll 4
           for (uint32_t e = 0; e < n; ++e) {
             const int2 h = hb[e];
-            const uint32_t pp = (uint32_t)h.x;
-            const uint32_t pm = pp > q ? pp - q : pp;
+            const uint32_t pm = (uint32_t)h.x;                      // below 2^32: as it is
             const uint32_t bn = from_signed(-h.y, q);               // -b mod q
             const uint32_t U2 = mont_mul(V, pm, q, qi);
             const uint32_t V2 = redc((uint64_t)bn * V + U, q, qi);
@@ -956,8 +1101,13 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
     return;
   }
 
-  // ---- MGCD4: recovery (GmpCudaDevice-getGcdKernel.cu:404-443), over the survivors listed
-  // in ibuf (in no particular order: each thread keeps the lowest index among its own)
+  if (j0 + nloc <= inv.n) {           // every modulus has its row in the inverse table
+    recover_cta<T>(mods, d, j0, ns, st, ibuf, hbuf, rs, parity, remaining, digits, count, status, inv);
+    return;
+  }
+
+  // ---- MGCD4: recovery (GmpCudaDevice-getGcdKernel.cu:404-443), one digit per round over the
+  // survivors listed in ibuf
   kh = 0xFFFFFFFFu;
   kl = 0u;
   for (uint32_t i = threadIdx.x; i < ns; i += TT) {
