@@ -536,8 +536,8 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
   // A batch of few pairs (at most one per two SMs) leaves most SMs idle with K pairs per CTA,
   // and its time is its longest pair's: each class, largest first, spreads its pairs over
   // clusters with its full count while SMs are left for the smaller classes.  61 mixed
-  // pairs 24.3 -> 9.1 ms, 24 of 160-300 kbit 189.8 -> 134.4 ms.  Not in a server's waves, which share
-  // the GPU with the continuous lanes, nor where the table asks for clusters of its own.
+  // pairs 24.2 -> 7.9 ms, 24 of 160-300 kbit 190.6 -> 140.0 ms.  Not in a server's waves, which
+  // share the GPU with the continuous lanes, nor where the table asks for clusters of its own.
   bool spread = !plain && P.spread && subset.size() <= (size_t)c->sms / 2;
   for (int b = 0; b < CLUSTER_CLASS; ++b) spread = spread && c->cfg[b].csize == 0;
   int sms_left = c->sms;
@@ -631,6 +631,15 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
             descs[k].nq_cap = std::max(ref, grow_cap(ref));
           }
         }
+      }
+      // Class 0 at the table's 256 x 2: its pairs live on a few warps, so what counts is how
+      // many CTAs an SM holds to fill each other's barriers and serial steps.  From 16 pairs
+      // per SM on, 128 threads (5,000 pairs of 1-8 kbit 5.93 -> 5.46 ms, 2,400 of 0.5-4 kbit even;
+      // 1,000: 1.27 -> 1.36), and from 32 on four pairs per CTA while the sets are small (16,384
+      // pairs of 0.5-4 kbit 8.92 -> 8.40, of 1-8 kbit 13.7 -> 14.5).
+      if (!plain && b == 0 && bk.threads == 256 && bk.k == 2 && v.size() >= 16 * (size_t)c->sms) {
+        bk.threads = 128;
+        if (v.size() >= 32 * (size_t)c->sms && bk.nq_max <= 1024) bk.k = 4;
       }
       // fewer pairs per CTA when k of the bucket's largest pairs would not fit shared memory
       // (16 KB kept for the kernel's static shared memory)

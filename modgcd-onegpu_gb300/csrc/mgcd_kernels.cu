@@ -1234,6 +1234,7 @@ static const void* batchk_fn_for(int threads, int k)
 {
   if (k == 2) {
     switch (threads) {
+      case 128: return reinterpret_cast<const void*>(&batchk_kernel<128, 2, NARROW>);
       case 256: return reinterpret_cast<const void*>(&batchk_kernel<256, 2, NARROW>);
       case 512: return reinterpret_cast<const void*>(&batchk_kernel<512, 2, NARROW>);
       case 1024: return reinterpret_cast<const void*>(&batchk_kernel<1024, 2, NARROW>);
@@ -1242,6 +1243,7 @@ static const void* batchk_fn_for(int threads, int k)
   }
   if (k == 4) {
     switch (threads) {
+      case 128: return reinterpret_cast<const void*>(&batchk_kernel<128, 4, NARROW>);
       case 256: return reinterpret_cast<const void*>(&batchk_kernel<256, 4, NARROW>);
       case 512: return reinterpret_cast<const void*>(&batchk_kernel<512, 4, NARROW>);
       case 1024: return reinterpret_cast<const void*>(&batchk_kernel<1024, 4, NARROW>);   // 64 registers, 32 warps/SM

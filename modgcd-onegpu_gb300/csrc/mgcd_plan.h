@@ -130,7 +130,7 @@ struct mgcd_context {
   // Per size class of the batched path: CTA size, pairs per CTA in lockstep, fraction of
   // the reference moduli count, CTAs per cluster (cluster class only).
   struct ClassCfg { int threads, k; float nq_scale; int csize; };
-  ClassCfg cfg[mgcd::NSTREAMS] = {{256, 4, 1.0f, 0}, {512, 4, 1.0f, 0}, {1024, 2, 1.0f, 0}, {1024, 1, 1.0f, 8}};
+  ClassCfg cfg[mgcd::NSTREAMS] = {{256, 2, 1.0f, 0}, {512, 2, 1.0f, 0}, {1024, 4, 1.0f, 0}, {1024, 1, 1.0f, 8}};
   bool use_graph = false;
   int single_policy = MGCD_SINGLE_AUTO;  // launch shape of pairs that span several CTAs
   unsigned long long wait_timeout_ns = 2000000000ull;   // bound of every cross-CTA wait
