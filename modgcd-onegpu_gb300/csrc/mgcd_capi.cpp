@@ -641,6 +641,10 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
         bk.threads = 128;
         if (v.size() >= 32 * (size_t)c->sms && bk.nq_max <= 1024) bk.k = 4;
       }
+      // The same for class 1 at the table's 512 x 2, whose shared memory lets three CTAs on an
+      // SM: 256 threads from 8 pairs per SM on (12-40 kbit pairs, 27 bits: 3,000 of them 51.2
+      // -> 47.6 ms, 1,600 28.6 -> 28.1, 800 16.5 -> 19.5).
+      if (!plain && b == 1 && bk.threads == 512 && bk.k == 2 && v.size() >= 8 * (size_t)c->sms) bk.threads = 256;
       // fewer pairs per CTA when k of the bucket's largest pairs would not fit shared memory
       // (16 KB kept for the kernel's static shared memory)
       while (bk.k > 1 && batch_smem_bytes(bk.threads, bk.k, bk.nq_max) > c->smem_optin - 16384) bk.k /= 2;
@@ -649,7 +653,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       if (batch_max_blocks_per_sm(bk.threads, bk.k, c->L <= 30, bk.smem, &bps) != cudaSuccess || bps < 1)
         return MGCD_ERR_GRID;
       bk.grid = (int)std::min<size_t>((v.size() + bk.k - 1) / bk.k, (size_t)c->sms * bps);
-      scratch += (size_t)bk.grid * 4 * bk.k * bk.nq_max;
+      scratch += (size_t)bk.grid * batch_scratch_words(bk.k, bk.nq_max);
     }
     P.order.insert(P.order.end(), v.begin(), v.end());
     buckets.push_back(bk);
@@ -715,7 +719,7 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     a.L = c->L;
     a.queue = queue_base + b;
     a.scratch = P.d_scratch.as<uint32_t>() + bk.scratch_off;
-    a.scratch_words = 4 * (size_t)bk.k * bk.nq_max;
+    a.scratch_words = bk.csize ? 4 * (size_t)bk.k * bk.nq_max : batch_scratch_words(bk.k, bk.nq_max);
     a.nq_max = bk.nq_max;
     a.digits = P.d_digits.as<mgcd_pair>();
     a.count = P.d_count.as<uint32_t>();

@@ -145,9 +145,10 @@ struct GridArgs {
 
 // Launch helpers (mgcd_kernels.cu).
 // k = pairs per CTA run in lockstep (1: batch_kernel; 2, 4: batchk_kernel).  Scratch per
-// CTA: 4 * k * nq_max words.  Moduli below 2^30 (a.L <= 30; `narrow` for the occupancy
+// CTA: batch_scratch_words(k, nq_max).  Moduli below 2^30 (a.L <= 30; `narrow` for the occupancy
 // query) select the kernels with lazily reduced Montgomery products.
 size_t batch_smem_bytes(int threads, int k, uint32_t nq_max);
+size_t batch_scratch_words(int k, uint32_t nq_max);
 cudaError_t batch_max_blocks_per_sm(int threads, int k, bool narrow, size_t smem, int* blocks);
 // after: a programmatic dependent launch -- the kernel may start once every CTA of the
 // stream's previous kernel has started (the batch kernels trigger at their start).

@@ -277,11 +277,13 @@ __global__ void __launch_bounds__(T, K < 8 ? 1024 / T : 1) batchk_kernel(const B
   stage_init(stage());
   const uint32_t NQS = a.nq_max;
   uint32_t* const tS = smem + STAGE_SMEM_WORDS;       // K x NQS states
-  uint32_t* const acc2 = tS + (size_t)K * NQS;        // residues of v during set-up; the
-                                                      // re-layout's and un-permute's buffer
-  uint16_t* const pmod = reinterpret_cast<uint16_t*>(acc2 + NQS);   // modulus at each position
-  uint16_t* const aux = pmod + NQS;                   // re-layout: live set, then new position
+  uint16_t* const pmod = reinterpret_cast<uint16_t*>(tS + (size_t)K * NQS);   // modulus at each position
   uint32_t* const scr = a.scratch + (size_t)blockIdx.x * a.scratch_words;   // per slot u0, v0, hist
+  // Not touched by the update loop, so in global scratch (they stay in L2): shared memory
+  // holds what each iteration reads, and more CTAs fit an SM.
+  uint32_t* const acc2 = scr + (size_t)4 * K * NQS;   // residues of v during set-up; the
+                                                      // re-layout's and un-permute's buffer
+  uint16_t* const aux = reinterpret_cast<uint16_t*>(acc2 + NQS);   // re-layout: live set, then new position
   const int L = a.L;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t rparity = 0, repoch = 0;
@@ -1225,8 +1227,15 @@ cudaError_t launch_build_invtab(const ModConst* mods, uint32_t n, uint32_t* tab,
 
 size_t batch_smem_bytes(int /*threads*/, int k, uint32_t nq_max)
 {
-  // K-slot kernels: K state arrays, the set-up / re-layout buffer and two 16-bit position arrays
-  return sizeof(uint32_t) * ((size_t)(k > 1 ? k + 2 : 2) * nq_max + STAGE_SMEM_WORDS);
+  // K-slot kernels: K state arrays and the 16-bit position array; one pair: states and set-up
+  return k > 1 ? sizeof(uint32_t) * ((size_t)k * nq_max + STAGE_SMEM_WORDS) + sizeof(uint16_t) * nq_max
+               : sizeof(uint32_t) * (2 * (size_t)nq_max + STAGE_SMEM_WORDS);
+}
+
+size_t batch_scratch_words(int k, uint32_t nq_max)
+{
+  // per slot u0, v0, history; K-slot kernels: the set-up / re-layout buffer and positions
+  return (4 * (size_t)k + (k > 1 ? 2 : 0)) * nq_max;
 }
 
 template <bool NARROW>

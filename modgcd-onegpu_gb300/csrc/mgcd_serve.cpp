@@ -254,7 +254,7 @@ int lane_init(mgcd_server* S, StreamLane& L, int l, int priority)
     if (moduli_needed(c->L, mid) <= (int)L.nq_cap) lo = mid; else hi = mid - 1;
   }
   L.limb_cap = 2 * (uint32_t)((lo + 31) / 32);
-  L.scratch_words = 4 * (size_t)L.k * L.nq_cap;
+  L.scratch_words = batch_scratch_words(L.k, L.nq_cap);
   L.entry.assign(STREAM_RING, nullptr);
   L.slot_used.assign(STREAM_MAX_CTAS[l], 0);
   const unsigned flags = cudaHostAllocMapped | cudaHostAllocPortable;
