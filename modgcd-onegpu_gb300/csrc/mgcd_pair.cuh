@@ -447,24 +447,45 @@ __device__ __forceinline__ void stage_issue(const uint32_t* x, int lo, int hi, S
                :: "r"(smem_u32(s.buf + b * STAGE_WORDS)), "l"(ga), "r"(bytes), "r"(m) : "memory");
 }
 
-// One tile of Horner steps z' = REDC(z * (2^64 mod q) + limb), most significant limb last
-// in `chunk`.  narrow (moduli below 2^30): z stays lazily in [0, 2q)
-// (z * r2 + limb < 2q^2 + 2^32 < q 2^32, as redc_lazy asks).
+// One tile of Horner steps, most significant limb last in `chunk`: z = y / R for the value y
+// of the limbs so far (R = 2^32), so a limb is z' = REDC(z R^2 + l) and n limbs at once
+// REDC(z R^(n+1) + l_(n-1) R^(n-1) + ... + l_1 R + l_0), the powers mod q.
+//   narrow (moduli below 2^29: widths 22 and 27)  four limbs a step; z stays lazily below
+//            4.6 q, which the reduction keeps: (4.6 q^2 + 3 q R + R) / R + q < 4.6 q;
+//   else     two limbs a step (32-bit moduli: R mod q = R - q, so the sum stays below 2^64 and
+//            its reduction below 2 q).
+// What bounds it is the multiplier pipe (a product and its reduction per limb) and, with few
+// warps, the chain through z: four limbs take four products and one reduction, one link of
+// the chain.  Cycles per limb, 12 warps on an SM: 45 -> 23, and two limbs at 32 bits 59 -> 44.
 __device__ __forceinline__ uint32_t horner_tile(uint32_t z, const uint32_t* chunk, int len, const ModConst& c,
                                                 bool narrow)
 {
+  int i = len - 1;
+  const uint32_t c3 = mont_mul(c.r2, c.r2, c.q, c.qinv);                       // R^3
   if (narrow) {
-    for (int i = len - 1; i >= 0; --i) z = redc_lazy((uint64_t)z * c.r2 + chunk[i], c.q, c.qinv);
+    const uint32_t c5 = mont_mul(c3, c3, c.q, c.qinv);                         // R^5
+    for (; (i & 3) != 3; --i) z = redc_lazy((uint64_t)z * c.r2 + chunk[i], c.q, c.qinv);
+#pragma unroll 2
+    for (; i >= 0; i -= 4) {
+      const uint64_t s = (uint64_t)chunk[i] * c3 + ((uint64_t)chunk[i - 1] * c.r2 +
+                                                    ((uint64_t)chunk[i - 2] * c.r1 + chunk[i - 3]));
+      z = redc_lazy((uint64_t)z * c5 + s, c.q, c.qinv);
+    }
   } else {
-    for (int i = len - 1; i >= 0; --i) z = redc((uint64_t)z * c.r2 + chunk[i], c.q, c.qinv);
+    if ((i & 1) == 0) z = redc((uint64_t)z * c.r2 + chunk[i--], c.q, c.qinv);
+#pragma unroll 2
+    for (; i >= 0; i -= 2) {
+      z = redc((uint64_t)z * c3 + ((uint64_t)chunk[i] * c.r1 + chunk[i - 1]), c.q, c.qinv);
+      if (z >= c.q) z -= c.q;
+    }
   }
   return z;
 }
 
 // x mod q_j for the nloc moduli mods[0..nloc), into acc[] (shared).  Limbs are staged
 // most-significant tile first; Horner in Montgomery form keeps z = y * 2^-32 where y is the
-// residue of the limbs consumed so far: z' = REDC(z * (2^64 mod q) + limb).  narrow: the
-// moduli are below 2^30 (z lazy until the final conversion, which is canonical).  Returns
+// residue of the limbs consumed so far (horner_tile).  narrow: the moduli are below 2^29 (z
+// lazy until the final conversion, which is canonical: 4.6 q r2 < q 2^32).  Returns
 // false if a staging wait ran out (after waiting, bounded, for the copy still in flight).
 template <int T>
 __device__ bool residues(const uint32_t* __restrict__ x, uint32_t n, const ModConst* __restrict__ mods,
