@@ -99,7 +99,7 @@ void Plan::destroy(cudaMemPool_t)
   if (stream) cudaStreamSynchronize(stream);
   drop_graph();
   for (DevBuf* b : {&d_limbs, &d_pairs, &d_order, &d_digits, &d_count, &d_iters, &d_status, &d_queue, &d_scratch,
-                    &d_gsync, &d_retry, &d_glimbs, &d_glen, &d_nqf, &d_upd, &d_span})
+                    &d_retry, &d_glimbs, &d_glen, &d_nqf, &d_upd, &d_span})
     b->release(stream);
   if (stream) cudaStreamSynchronize(stream);
   for (HostBuf* b : {&h_count, &h_iters, &h_status, &h_digits, &h_glimbs, &h_glen, &h_nqf, &h_upd}) b->release();
@@ -114,7 +114,7 @@ size_t Plan::device_bytes() const
 {
   size_t s = 0;
   for (const DevBuf* b : {&d_limbs, &d_pairs, &d_order, &d_digits, &d_count, &d_iters, &d_status, &d_queue,
-                          &d_scratch, &d_gsync, &d_retry, &d_glimbs, &d_glen, &d_nqf, &d_upd, &d_span})
+                          &d_scratch, &d_retry, &d_glimbs, &d_glen, &d_nqf, &d_upd, &d_span})
     s += b->bytes;
   return s;
 }
@@ -197,6 +197,38 @@ size_t mgcd_gen_moduli(int L, uint32_t* out, size_t count) { return gen_moduli(L
 
 int mgcd_moduli_needed(int L, size_t bits) { return moduli_needed(L, bits); }
 
+// Where the lines of the cooperative grid's exchange live: a line's home is on one of the
+// GPU's two dies, and an exchange whose leader (CTA 0) polls lines of its own die takes 2,600
+// cycles at 152 CTAs, of the other die 3,150.  The home changes every few pages, so the same
+// exchange is timed at GSYNC_PLACES places (~1 ms in all) and the fastest kept; any place is
+// correct.
+static int calibrate_exchange(mgcd_context* c, cudaStream_t s)
+{
+  if (c->d_xchg.grow(GSYNC_PLACES * GSYNC_STRIDE, c->pool, s) != cudaSuccess) return MGCD_ERR_CUDA;
+  char* const base = c->d_xchg.as<char>();
+  c->gsync = reinterpret_cast<GridSync*>(base);
+  DevBuf t;
+  if (t.grow(GSYNC_PLACES * sizeof(unsigned long long), c->pool, s) != cudaSuccess) return MGCD_ERR_CUDA;
+  unsigned long long h[GSYNC_PLACES];
+  bool ok = cudaMemsetAsync(t.p, 0xFF, sizeof h, s) == cudaSuccess;
+  for (size_t i = 0; ok && i < GSYNC_PLACES; ++i) {
+    GridSync* g = reinterpret_cast<GridSync*>(base + i * GSYNC_STRIDE);
+    ok = launch_gridsync_init(g, c->wait_timeout_ns, 0xFFFFFFFFu, s) == cudaSuccess;
+    // a GPU shared with other work may refuse the co-resident grid: then the first place stays
+    if (ok && launch_exchange_probe(g, c->sms, 40, t.as<unsigned long long>() + i, s) != cudaSuccess) {
+      cudaGetLastError();
+      break;
+    }
+  }
+  ok = ok && cudaMemcpyAsync(h, t.p, sizeof h, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+       cudaStreamSynchronize(s) == cudaSuccess;
+  t.release(s);
+  if (!ok) return MGCD_ERR_CUDA;
+  const size_t best = (size_t)(std::min_element(h, h + GSYNC_PLACES) - h);
+  c->gsync = reinterpret_cast<GridSync*>(base + best * GSYNC_STRIDE);
+  return MGCD_OK;
+}
+
 int mgcd_create(int device, int L, mgcd_context** out)
 {
   if (!out || (L != 22 && L != 27 && L != 32)) return MGCD_ERR_INVALID_ARG;
@@ -259,6 +291,7 @@ int mgcd_create(int device, int L, mgcd_context** out)
                             cudaSuccess ||
                         cudaStreamSynchronize(s) != cudaSuccess))
     rc = MGCD_ERR_CUDA;
+  if (rc == MGCD_OK) rc = calibrate_exchange(c, s);
   if (rc != MGCD_OK) {
     mgcd_destroy(c);
     return rc;
@@ -277,6 +310,7 @@ int mgcd_destroy(mgcd_context* c)
     cudaStreamSynchronize(s);
     c->mods.release(s);
     c->d_invtab.release(s);
+    c->d_xchg.release(s);
   }
   c->main.destroy(c->pool);
   if (c->pool) cudaMemPoolDestroy(c->pool);
@@ -432,7 +466,6 @@ int mgcd::plan_batch(mgcd_context* c, Plan& P, size_t np, const uint32_t* limbs,
   CK(P.d_upd.grow(std::max<size_t>(ng, 1) * sizeof(unsigned long long), c->pool, s));
   CK(P.d_queue.grow(2 * NSTREAMS * sizeof(uint32_t), c->pool, s));
   CK(P.d_scratch.grow(std::max<size_t>(scratch, 1) * sizeof(uint32_t), c->pool, s));
-  CK(P.d_gsync.grow(sizeof(GridSync), c->pool, s));
   CK(P.d_glimbs.grow(std::max<size_t>(P.nglimbs, 1) * sizeof(uint32_t), c->pool, s));
   CK(P.d_glen.grow(std::max<size_t>(ng, 1) * sizeof(uint32_t), c->pool, s));
   P.h2d_bytes = ng ? limb_end * sizeof(uint32_t) + ng * sizeof(PairDesc) + P.order.size() * sizeof(uint32_t) : 0;
@@ -778,7 +811,7 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
       }
       nclu = (int)((d.nq + per * CS - 1) / (per * CS));
       g.per_cta = per;
-      g.sync = P.d_gsync.as<GridSync>();
+      g.sync = c->gsync;
       CK(launch_gridsync_init(g.sync, c->wait_timeout_ns, c->withhold_cta, P.stream));
       ++P.launches;
       const int thr = single_threads(per);
@@ -804,7 +837,7 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     }
     if (grid > (uint32_t)MAX_GRID_CTAS) return MGCD_ERR_GRID;   // one exchange slot per CTA
     g.per_cta = per;
-    g.sync = P.d_gsync.as<GridSync>();
+    g.sync = c->gsync;
     CK(launch_gridsync_init(g.sync, c->wait_timeout_ns, c->withhold_cta, P.stream));
     ++P.launches;
     cudaError_t e = launch_grid(g, threads, (int)grid, grid_smem_bytes(per), P.stream);

@@ -259,18 +259,31 @@ __device__ __forceinline__ void warp_min_key(uint32_t& hi, uint32_t& lo)
 // One reduction-loop update of a modulus state t for pivot (p, b):
 //   t' = p / (t - b)  (mod q)   since t' = u'/v' = v / ((u - b v)/p)
 // with t = INF -> 0 (v was 0: u' = 0, v' = u/p), t == b -> INF (v' = 0), degenerate and
-// retired states fixed; the pivot's own modulus retires.
-// narrow: q < 2^30.  A pivot p < 2^32 enters the product as it is (p inv < q 2^32).
-__device__ __forceinline__ uint32_t t_update(uint32_t t, uint32_t q, uint32_t qinv, uint32_t p, int32_t b,
-                                             bool narrow)
+// retired states fixed; the pivot's own modulus retires.  The single pairs' update: its
+// latency is on the chain of iterations, so p R is formed beside the inverse and the product
+// with it beside the inverse's check (inv_mod's, with the same fallback); for q > 2^31 the
+// second candidate is 2^32 - q = R mod q less, its product p R less.
+// narrow: q < 2^31.  A pivot p < 2^32 enters the product as it is (p R^2 < q 2^32).
+__device__ __forceinline__ uint32_t t_update(uint32_t t, const ModConst& c, uint32_t p, int32_t b, bool narrow)
 {
+  const uint32_t q = c.q, qinv = c.qinv;
   if (t >= T_MARK) return (t == T_INF) ? 0u : t;
   if (q == p) return T_RETIRED;
   const uint32_t d = mod_sub(t, from_signed(b, q), q);
   if (d == 0u) return T_INF;
-  // redc(d) = d/R, inv = R/d, mont_mul(p, R/d) = p/d
-  const uint32_t x = redc((uint64_t)d, q, qinv);
-  return mont_mul(p, narrow ? inv_mod_narrow<2>(x, q, qinv) : inv_mod<2>(x, q, qinv), q, qinv);
+  const uint32_t pR = mont_mul(p, c.r2, q, qinv), one = redc(1ull, q, qinv);
+  const uint32_t s = inv_euclid<2>(d, q);
+  if (narrow) {
+    const uint32_t inv = (int32_t)s < 0 ? s + q : s;
+    const uint32_t r = mont_mul(pR, inv, q, qinv);
+    if (redc((uint64_t)inv * d, q, qinv) == one) return r;
+  } else {
+    const uint32_t inv = s >= q ? s - q : s;
+    const uint32_t r = mont_mul(pR, inv, q, qinv), k = redc((uint64_t)inv * d, q, qinv);
+    if (k == one) return r;
+    if (mod_sub(k, d, q) == one) return mod_sub(r, pR, q);
+  }
+  return mont_mul(pR, inv_mod_slow(d, q), q, qinv);
 }
 
 // Moduli below 2^30 (widths up to 30 bits): products kept lazily in [0, 2q) where no

@@ -183,9 +183,9 @@ constexpr int PH_WORDS_T0 = 11;         // words kept by thread 0
 // Iterations between two re-layouts of a K-slot CTA's positions (besides those after a pair
 // finishes, is loaded or grows).  Each iteration retires one position per slot, so a layout
 // stays close to sorted; one re-layout moves (K + 1) x nq_max words twice.  Measured on the
-// mixed batch with moduli growth (27 bits): every 8 iterations 80.4 ms, 16 76.3, 32 74.6.
+// mixed batch (27 bits): every 32 iterations 49.9 ms, 64 49.5, 128 49.9.
 #ifndef MGCD_RELAYOUT_EVERY
-#define MGCD_RELAYOUT_EVERY 32
+#define MGCD_RELAYOUT_EVERY 64
 #endif
 constexpr uint32_t RELAYOUT_EVERY = MGCD_RELAYOUT_EVERY;
 
@@ -1179,7 +1179,7 @@ __global__ void __launch_bounds__(256) int_peak_kernel(uint32_t* out, int iters)
 __global__ void __launch_bounds__(256) gridsync_init_kernel(GridSync* gs, unsigned long long timeout_ns,
                                                              uint32_t withhold)
 {
-  for (uint32_t i = threadIdx.x; i < 2u * MAX_GRID_CTAS; i += blockDim.x) (&gs->keys[0][0])[i] = 0ull;
+  for (uint32_t i = threadIdx.x; i < 2u * MAX_GRID_CTAS; i += blockDim.x) gs->keys[i] = 0ull;
   if (threadIdx.x < 32u) (&gs->bcast[0][0])[threadIdx.x] = 0ull;
   if (threadIdx.x == 0) {
     gs->slot[0] = gs->slot[1] = gs->slot[2] = ~0ull;
@@ -1194,6 +1194,27 @@ cudaError_t launch_gridsync_init(GridSync* gs, unsigned long long timeout_ns, ui
 {
   gridsync_init_kernel<<<1, 256, 0, s>>>(gs, timeout_ns, withhold);
   return cudaGetLastError();
+}
+
+// Times `n` exchanges of the cooperative grid's protocol through *gs (cycles of CTA 0).
+__global__ void __launch_bounds__(1024) exchange_probe_kernel(GridSync* gs, uint32_t n, unsigned long long* cycles)
+{
+  __shared__ RedSmem rs;
+  uint32_t parity = 0, epoch = 0;
+  long long t0 = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    if (i == 8u) t0 = clock64();                       // past the CTAs' staggered start
+    uint32_t hi = (threadIdx.x + i) & 1023u, lo = blockIdx.x + 1u;
+    if (!reduce_min<0, SYNC_GRID>(hi, lo, rs, parity, gs, epoch)) return;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *cycles = (unsigned long long)(clock64() - t0);
+}
+
+cudaError_t launch_exchange_probe(GridSync* gs, int ctas, uint32_t n, unsigned long long* cycles, cudaStream_t s)
+{
+  void* args[] = {&gs, &n, &cycles};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&exchange_probe_kernel), dim3(ctas), dim3(288), args,
+                                     0, s);
 }
 
 cudaError_t launch_int_peak(uint32_t* out, int blocks, int iters, cudaStream_t s)

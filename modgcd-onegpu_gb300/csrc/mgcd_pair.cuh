@@ -317,10 +317,13 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
     // Leader exchange (GridSync): tagged slots, relaxed stores and loads, bounded polls.
     // PUB adds release fences before the stores and acquire fences after the polls, for
     // exchanges that also publish data written before them.  What bounds it: two hops through
-    // L2, each a store (~300 cycles) and the poll that sees it (295 cycles a round trip).
+    // L2, each a store that has to reach the line's home (~300 cycles, ~550 more from the
+    // other die: the slots are kept near the leader, calibrate_exchange) and the poll that
+    // sees it (295 cycles a round trip); a thread per slot polls faster than a warp with
+    // several slots a lane (2,600 and 2,820 cycles an exchange of 152 CTAs).
     const uint32_t b = epoch & 1u;
     const unsigned long long tag = key_tag(epoch);
-    unsigned long long* const keys = gs->keys[b];
+    unsigned long long* const keys = gs->keys + b * ((gridDim.x + 15u) & ~15u);
     unsigned long long k = pack_key(hi, lo);
     uint32_t bad = 0;
     PollClock clk;
@@ -643,13 +646,13 @@ __device__ void run_pair(const uint32_t* __restrict__ limbs, const PairDesc& d, 
     kl = 0xFFFFFFFFu;
     if (one) {
       if (have) {
-        t1 = t_update(t1, c1.q, c1.qinv, p, b, L <= 30);
+        t1 = t_update(t1, c1, p, b, L <= 30);
         t_key(t1, c1.q, kh, kl);
       }
     } else {
       for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
         const ModConst c = my[j];
-        const uint32_t t = t_update(st[j], c.q, c.qinv, p, b, L <= 30);
+        const uint32_t t = t_update(st[j], c, p, b, L <= 30);
         st[j] = t;
         uint32_t h, l;
         t_key(t, c.q, h, l);
@@ -675,6 +678,45 @@ __device__ void run_pair(const uint32_t* __restrict__ limbs, const PairDesc& d, 
   if (writer) *iters_out = iters;
   finish_pair<T, MODE>(mods, d, L, j0, nloc, st, rs, parity, epoch, gs, u0g, v0g, hist, iters, remaining, lu, lv, book,
                        digits, count, status, inv, stg.buf, acc2);
+}
+
+// One warp's digits of a recovery panel by the reference's rule: the lowest lane with a nonzero
+// value gives (its modulus, its symmetric value g) and every other live lane's u becomes
+// (u - g) / p, at most `most` digits.  Lane l < np holds a panel member; pinv[32 a + b] = R /
+// q_a mod q_b.  Returns the digits produced; a lane that gave one has live = false, its value
+// in g and its place in `rank`.  While the lanes come in order (no lane is zero at its turn,
+// nearly always) the next digit's lane and inverses are known beforehand, and a digit is one
+// chain of a shuffle and a product, ~110 cycles; finding the lane by a vote took 420.
+__device__ __forceinline__ uint32_t panel_digits(uint32_t& u, bool& live, const ModConst& c, const uint32_t* pinv,
+                                                 uint32_t np, uint32_t most, int32_t& g, uint32_t& rank)
+{
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t nd = 0;
+  live = lane < np;
+  for (; nd < np && nd < most; ++nd) {
+    const int32_t x = __shfl_sync(0xFFFFFFFFu, to_signed(u, c.q), (int)nd);
+    const uint32_t inv = pinv[32u * nd + lane];
+    if (x == 0) break;
+    if (lane == nd) {
+      g = x;
+      rank = nd;
+      live = false;
+    }
+    if (live) u = mont_mul(mod_sub(u, from_signed(x, c.q), c.q), inv, c.q, c.qinv);
+  }
+  for (; nd < most; ++nd) {
+    const uint32_t nz = __ballot_sync(0xFFFFFFFFu, live && u != 0u);
+    if (!nz) break;
+    const uint32_t src = __ffs((int)nz) - 1u;
+    const int32_t x = __shfl_sync(0xFFFFFFFFu, to_signed(u, c.q), (int)src);
+    if (lane == src) {
+      g = x;
+      rank = nd;
+      live = false;
+    }
+    if (live) u = mont_mul(mod_sub(u, from_signed(x, c.q), c.q), pinv[32u * src + lane], c.q, c.qinv);
+  }
+  return nd;
 }
 
 // Recovery (MGCD4, GmpCudaDevice-getGcdKernel.cu:404-443) for a pair spread over several
@@ -755,26 +797,16 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
         const bool in = lane < np;
         const uint32_t j = in ? pidx[lane] : 0u;
         const ModConst c = my[in ? j : pidx[0]];
-        uint32_t u = in ? st[j] : 0u;
-        uint32_t live = __ballot_sync(0xFFFFFFFFu, in);
-        uint32_t nd = 0;
-        int rem = remaining;
-        while (nd < 32u && rem > 0) {
-          const uint32_t nz = __ballot_sync(0xFFFFFFFFu, ((live >> lane) & 1u) && u != 0u);
-          if (!nz) break;
-          const uint32_t src = __ffs((int)nz) - 1u;
-          const int32_t g = __shfl_sync(0xFFFFFFFFu, to_signed(u, c.q), (int)src);
-          const uint32_t p = __shfl_sync(0xFFFFFFFFu, c.q, (int)src);
-          if (lane == 0) out[ndig + nd] = mgcd_pair{p, g};
-          live &= ~(1u << src);
-          if ((live >> lane) & 1u) u = mont_mul(mod_sub(u, from_signed(g, c.q), c.q), pinv[src][lane], c.q, c.qinv);
-          ++nd;
-          --rem;
-        }
-        if (in) st[j] = ((live >> lane) & 1u) ? u : U_RETIRED;
+        uint32_t u = in ? st[j] : 0u, rank = 0u;
+        int32_t g = 0;
+        bool live;
+        const uint32_t nd = panel_digits(u, live, c, &pinv[0][0], np, (uint32_t)min(remaining, 32), g, rank);
+        if (in && !live) out[ndig + rank] = mgcd_pair{c.q, g};
+        if (in) st[j] = live ? u : U_RETIRED;
+        __threadfence();               // the digits before the count
+        __syncwarp();
         if (lane == 0) {
           pn = nd;
-          __threadfence();             // the digits before the count
           *count = ndig + nd;          // published by the exchange below
           __threadfence();
         }
@@ -867,8 +899,7 @@ __device__ void recover_panels(const ModConst* __restrict__ mods, const PairDesc
 // load from the digit's row of the table and one product.  A panel without digits falls back
 // to one round of the rule over all survivors, which also detects the end.  Digits, their
 // order and the end conditions are those of the per-digit loop below, whose rounds (a
-// barrier, a table row not seen before) took 2,000-3,000 cycles a digit; a panel takes
-// ~200.
+// barrier, a table row not seen before) took 2,000-3,000 cycles a digit.
 //   ord    the survivors' indices in table order (ns of them), st their values
 //   work   shared, 1,024 words: the panel's pairwise inverses
 template <int T>
@@ -910,24 +941,14 @@ __device__ void recover_cta(const ModConst* __restrict__ mods, const PairDesc& d
       const bool in = lane < np;
       const uint32_t place = pidx[in ? lane : 0u], j = ord[place];
       const ModConst c = mods[j0 + j];
-      uint32_t u = in ? st[j] : 0u;
-      bool live = in;
-      uint32_t nd = 0;
-      int rem = remaining;
-      while (nd < 32u && rem > 0) {
-        const uint32_t nz = __ballot_sync(0xFFFFFFFFu, live && u != 0u);
-        if (!nz) break;
-        const uint32_t src = __ffs((int)nz) - 1u;
-        const int32_t g = __shfl_sync(0xFFFFFFFFu, to_signed(u, c.q), (int)src);
-        if (lane == src) {
-          drow[nd] = j0 + j;
-          dval[nd] = g;
-          out[ndig + nd] = mgcd_pair{c.q, g};
-          live = false;
-        }
-        if (live) u = mont_mul(mod_sub(u, from_signed(g, c.q), c.q), work[32u * src + lane], c.q, c.qinv);
-        ++nd;
-        --rem;
+      uint32_t u = in ? st[j] : 0u, rank = 0u;
+      int32_t g = 0;
+      bool live;
+      const uint32_t nd = panel_digits(u, live, c, work, np, (uint32_t)min(remaining, 32), g, rank);
+      if (in && !live) {
+        drow[rank] = j0 + j;
+        dval[rank] = g;
+        out[ndig + rank] = mgcd_pair{c.q, g};
       }
       if (in) st[j] = live ? u : U_RETIRED;
       const uint32_t left = __ballot_sync(0xFFFFFFFFu, live);
@@ -935,6 +956,13 @@ __device__ void recover_cta(const ModConst* __restrict__ mods, const PairDesc& d
       if (lane == 0) {
         pn = nd;
         if (left == 0u) pscan = next;
+      }
+    } else {
+      // the other warps meanwhile bring the panel's rows of the table into L2
+      for (uint32_t i = next + threadIdx.x - 32u; i < ns; i += TT - 32u) {
+        const uint32_t* const col = inv.tab + (j0 + ord[i]);
+        for (uint32_t k = 0; k < np; ++k)
+          asm volatile("prefetch.global.L2 [%0];" :: "l"(col + (size_t)(j0 + ord[pidx[k]]) * inv.n));
       }
     }
     __syncthreads();

@@ -51,6 +51,7 @@ struct Bucket {
 // or a serving lane asks for one); larger pairs K per thread-block cluster.
 constexpr int NSTREAMS = MGCD_NUM_SIZE_CLASSES;
 constexpr int CLUSTER_CLASS = 3;
+constexpr size_t GSYNC_PLACES = 16, GSYNC_STRIDE = 36864;   // bytes between the places
 constexpr size_t INVTAB_N = 16384;        // moduli covered by the pairwise inverse table
 
 inline int size_class(uint32_t nq) { return nq <= 1024 ? 0 : nq <= 4096 ? 1 : nq <= CTA_MAX_NQ ? 2 : CLUSTER_CLASS; }
@@ -89,7 +90,7 @@ struct Plan {
                                        // context's setting); serving waves favour latency
   int cluster_k = 0;                   // pairs per cluster of size class 3 (0: the context's setting)
 
-  DevBuf d_limbs, d_pairs, d_order, d_digits, d_count, d_iters, d_status, d_queue, d_scratch, d_gsync, d_retry;
+  DevBuf d_limbs, d_pairs, d_order, d_digits, d_count, d_iters, d_status, d_queue, d_scratch, d_retry;
   DevBuf d_nqf, d_upd;                 // per pair (K-slot kernels): final moduli count, loop updates
   DevBuf d_span;                       // per bucket kernel: earliest CTA start, ~(latest CTA end), ns
   DevBuf d_glimbs, d_glen;             // binary gcds converted on the device
@@ -124,6 +125,8 @@ struct mgcd_context {
   mgcd::DevBuf mods;
   mgcd::DevBuf d_invtab;               // pairwise inverse table (InvTab)
   uint32_t invtab_n = 0;
+  mgcd::DevBuf d_xchg;                 // GSYNC_PLACES places for the grid exchange's lines
+  mgcd::GridSync* gsync = nullptr;     // the fastest of them (calibrate_exchange)
   mgcd::Plan main;                     // the plan of the context's own calls
   bool serving = false;                // a request server runs on this context
 
