@@ -98,11 +98,9 @@ void Plan::destroy(cudaMemPool_t)
 {
   if (stream) cudaStreamSynchronize(stream);
   drop_graph();
-  for (DevBuf* b : {&d_limbs, &d_pairs, &d_order, &d_digits, &d_count, &d_iters, &d_status, &d_queue, &d_scratch,
-                    &d_retry, &d_glimbs, &d_glen, &d_nqf, &d_upd, &d_span})
-    b->release(stream);
+  for (DevBuf* b : {&d_in, &d_res, &d_scratch, &d_retry}) b->release(stream);
   if (stream) cudaStreamSynchronize(stream);
-  for (HostBuf* b : {&h_count, &h_iters, &h_status, &h_digits, &h_glimbs, &h_glen, &h_nqf, &h_upd}) b->release();
+  for (HostBuf* b : {&h_res, &h_digits}) b->release();
   if (t_run0) cudaEventDestroy(t_run0);
   if (t_run1) cudaEventDestroy(t_run1);
   if (stream) cudaStreamDestroy(stream);
@@ -113,10 +111,29 @@ void Plan::destroy(cudaMemPool_t)
 size_t Plan::device_bytes() const
 {
   size_t s = 0;
-  for (const DevBuf* b : {&d_limbs, &d_pairs, &d_order, &d_digits, &d_count, &d_iters, &d_status, &d_queue,
-                          &d_scratch, &d_retry, &d_glimbs, &d_glen, &d_nqf, &d_upd, &d_span})
-    s += b->bytes;
+  for (const DevBuf* b : {&d_in, &d_res, &d_scratch, &d_retry}) s += b->bytes;
   return s;
+}
+
+// Offsets of the parts of d_in (limb_words operand limbs) and d_res for ng pairs.
+void Plan::layout(size_t ng, uint64_t limb_words)
+{
+  auto up = [](size_t x) { return (x + 15) / 16 * 16; };
+  // + 4 limbs: the kernels stage operand tiles by bulk copies widened to 16-byte bounds
+  in.pairs = up((limb_words + 4) * sizeof(uint32_t));
+  in.order = up(in.pairs + ng * sizeof(PairDesc));
+  in.end = in.order + 2 * ng * sizeof(uint32_t);
+  res.span = 0;
+  res.status = 2 * NSTREAMS * sizeof(unsigned long long);
+  res.upd = up(res.status + ng * sizeof(int32_t));
+  res.nqf = res.upd + ng * sizeof(unsigned long long);
+  res.queue = res.nqf + ng * sizeof(uint32_t);
+  res.count = res.queue + 2 * NSTREAMS * sizeof(uint32_t);
+  res.iters = res.count + ng * sizeof(uint32_t);
+  res.glen = res.iters + ng * sizeof(uint32_t);
+  res.glimbs = up(res.glen + ng * sizeof(uint32_t));
+  res.digits = up(res.glimbs + nglimbs * sizeof(uint32_t));
+  res.end = res.digits + ndig * sizeof(mgcd_pair);
 }
 
 int to_status(int32_t st)
@@ -358,6 +375,7 @@ int mgcd::plan_batch(mgcd_context* c, Plan& P, size_t np, const uint32_t* limbs,
   P.np = np;
   P.plain = plain;
   P.ran = false;
+  P.fetched = false;
   P.status.assign(np, -1);
   P.slot.assign(np, -1);
   P.trivial.assign(np, {});
@@ -452,28 +470,25 @@ int mgcd::plan_batch(mgcd_context* c, Plan& P, size_t np, const uint32_t* limbs,
 
   // Device buffers and upload.
   cudaStream_t s = P.stream;
-  // + 4 limbs: the kernels stage operand tiles by bulk copies widened to 16-byte bounds
-  CK(P.d_limbs.grow((std::max<uint64_t>(limb_end, 1) + 4) * sizeof(uint32_t), c->pool, s));
-  if (reinterpret_cast<uintptr_t>(P.d_limbs.p) % 16 != 0) return MGCD_ERR_CUDA;   // pool blocks are 256-aligned
-  CK(P.d_pairs.grow(std::max<size_t>(ng, 1) * sizeof(PairDesc), c->pool, s));
-  CK(P.d_order.grow(std::max<size_t>(P.order.size(), 1) * sizeof(uint32_t), c->pool, s));
-  CK(P.d_digits.grow(std::max<size_t>(P.ndig, 1) * sizeof(mgcd_pair), c->pool, s));
-  CK(P.d_count.grow(std::max<size_t>(ng, 1) * sizeof(uint32_t), c->pool, s));
-  CK(P.d_iters.grow(std::max<size_t>(ng, 1) * sizeof(uint32_t), c->pool, s));
-  CK(P.d_status.grow(std::max<size_t>(ng, 1) * sizeof(int32_t), c->pool, s));
-  CK(P.d_nqf.grow(std::max<size_t>(ng, 1) * sizeof(uint32_t), c->pool, s));
-  CK(P.d_span.grow(2 * NSTREAMS * sizeof(unsigned long long), c->pool, s));
-  CK(P.d_upd.grow(std::max<size_t>(ng, 1) * sizeof(unsigned long long), c->pool, s));
-  CK(P.d_queue.grow(2 * NSTREAMS * sizeof(uint32_t), c->pool, s));
+  P.layout(ng, limb_end);
+  CK(P.d_in.grow(P.in.end, c->pool, s));
+  if (reinterpret_cast<uintptr_t>(P.d_in.p) % 16 != 0) return MGCD_ERR_CUDA;   // pool blocks are 256-aligned
+  CK(P.d_res.grow(P.res.end, c->pool, s));
   CK(P.d_scratch.grow(std::max<size_t>(scratch, 1) * sizeof(uint32_t), c->pool, s));
-  CK(P.d_glimbs.grow(std::max<size_t>(P.nglimbs, 1) * sizeof(uint32_t), c->pool, s));
-  CK(P.d_glen.grow(std::max<size_t>(ng, 1) * sizeof(uint32_t), c->pool, s));
-  P.h2d_bytes = ng ? limb_end * sizeof(uint32_t) + ng * sizeof(PairDesc) + P.order.size() * sizeof(uint32_t) : 0;
-  if (ng) {
-    CK(cudaMemcpyAsync(P.d_limbs.p, limbs, limb_end * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(P.d_pairs.p, P.descs.data(), ng * sizeof(PairDesc), cudaMemcpyHostToDevice, s));
-    if (!P.order.empty())
-      CK(cudaMemcpyAsync(P.d_order.p, P.order.data(), P.order.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+  const size_t lb = limb_end * sizeof(uint32_t), pb = ng * sizeof(PairDesc), ob = P.order.size() * sizeof(uint32_t);
+  P.h2d_bytes = ng ? lb + pb + ob : 0;
+  // Up to 64 KB go as one copy out of the plan's own host memory, which the runtime has read
+  // when the call returns; more is copied from where it lies.
+  if (ng && P.in.order + ob <= 65536) {
+    P.in_host.resize(P.in.order + ob);
+    std::memcpy(P.in_host.data(), limbs, lb);
+    std::memcpy(P.in_host.data() + P.in.pairs, P.descs.data(), pb);
+    if (ob) std::memcpy(P.in_host.data() + P.in.order, P.order.data(), ob);
+    CK(cudaMemcpyAsync(P.d_in.p, P.in_host.data(), P.in.order + ob, cudaMemcpyHostToDevice, s));
+  } else if (ng) {
+    CK(cudaMemcpyAsync(P.d_in.p, limbs, lb, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(P.din<void>(P.in.pairs), P.descs.data(), pb, cudaMemcpyHostToDevice, s));
+    if (ob) CK(cudaMemcpyAsync(P.din<void>(P.in.order), P.order.data(), ob, cudaMemcpyHostToDevice, s));
   }
   return MGCD_OK;
 }
@@ -700,12 +715,11 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
 
 // Launches the buckets (one stream each, joined back into P.stream) and then the
 // single-pair launches.  `pairs` is the descriptor array on the device, `queue_base` the
-// first of the bucket work counters (zeroed here).
+// first of the bucket work counters (zeroed by the caller).
 static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& buckets,
                       const std::vector<uint32_t>& grid_pairs, const std::vector<PairDesc>& descs, PairDesc* pairs,
                       uint32_t* queue_base, bool time_buckets, bool traced = true)
 {
-  CK(cudaMemsetAsync(queue_base, 0, NSTREAMS * sizeof(uint32_t), P.stream));
   unsigned long long* trace = nullptr;
   unsigned long long* phases = nullptr;
   if (c->trace && traced) {
@@ -729,13 +743,12 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
   // programmatic dependent of the one before (it starts once all CTAs of that one have
   // started, cta_begin): the kernels run side by side, the larger classes' persistent CTAs
   // placed first.  The span of each (earliest CTA start, latest CTA end) is its time.
-  if (time_buckets) CK(cudaMemsetAsync(P.d_span.p, 0xFF, 2 * NSTREAMS * sizeof(unsigned long long), P.stream));
   for (size_t b = 0; b < buckets.size(); ++b) {
     const Bucket& bk = buckets[b];
     BatchArgs a{};
     a.trace = trace;
     a.phases = phases;
-    a.span = time_buckets ? P.d_span.as<unsigned long long>() + 2 * b : nullptr;
+    a.span = time_buckets ? P.dres<unsigned long long>(P.res.span) + 2 * b : nullptr;
     if (trace) {
       const int n = bk.grid * (bk.csize ? bk.csize : 1);
       trace += 4 * (size_t)n;
@@ -744,9 +757,9 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     }
     a.stage_fail = c->stage_fail_cta;
     a.inv = InvTab{c->d_invtab.as<uint32_t>(), c->invtab_n};
-    a.limbs = P.d_limbs.as<uint32_t>();
+    a.limbs = P.din<uint32_t>(0);
     a.pairs = pairs;
-    a.order = P.d_order.as<uint32_t>() + bk.first;
+    a.order = P.din<uint32_t>(P.in.order) + bk.first;
     a.npairs = bk.n;
     a.mods = c->mods.as<ModConst>();
     a.L = c->L;
@@ -754,13 +767,13 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     a.scratch = P.d_scratch.as<uint32_t>() + bk.scratch_off;
     a.scratch_words = bk.csize ? 4 * (size_t)bk.k * bk.nq_max : batch_scratch_words(bk.k, bk.nq_max);
     a.nq_max = bk.nq_max;
-    a.digits = P.d_digits.as<mgcd_pair>();
-    a.count = P.d_count.as<uint32_t>();
-    a.iters = P.d_iters.as<uint32_t>();
-    a.status = P.d_status.as<int32_t>();
+    a.digits = P.dres<mgcd_pair>(P.res.digits);
+    a.count = P.dres<uint32_t>(P.res.count);
+    a.iters = P.dres<uint32_t>(P.res.iters);
+    a.status = P.dres<int32_t>(P.res.status);
     a.grow_permille = c->grow_permille;
-    a.nq_final = P.d_nqf.as<uint32_t>();
-    a.updates = P.d_upd.as<unsigned long long>();
+    a.nq_final = P.dres<uint32_t>(P.res.nqf);
+    a.updates = P.dres<unsigned long long>(P.res.upd);
     if (bk.csize)
       CK(launch_cluster_batch(a, bk.threads, bk.k, bk.csize, bk.grid, bk.smem, P.stream, b > 0));
     else
@@ -773,15 +786,15 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     GridArgs g;
     g.stage_fail = c->stage_fail_cta;
     g.inv = InvTab{c->d_invtab.as<uint32_t>(), c->invtab_n};
-    g.limbs = P.d_limbs.as<uint32_t>();
+    g.limbs = P.din<uint32_t>(0);
     g.pair = d;
     g.mods = c->mods.as<ModConst>();
     g.L = c->L;
     g.scratch = P.d_scratch.as<uint32_t>() + P.grid_scratch_off;
-    g.digits = P.d_digits.as<mgcd_pair>();
-    g.count = P.d_count.as<uint32_t>() + k;
-    g.iters = P.d_iters.as<uint32_t>() + k;
-    g.status = P.d_status.as<int32_t>() + k;
+    g.digits = P.dres<mgcd_pair>(P.res.digits);
+    g.count = P.dres<uint32_t>(P.res.count) + k;
+    g.iters = P.dres<uint32_t>(P.res.iters) + k;
+    g.status = P.dres<int32_t>(P.res.status) + k;
     const bool ref_shape = c->single_policy == MGCD_SINGLE_REFERENCE_SHAPE;
     if (!ref_shape && d.nq <= (uint32_t)MAX_CLUSTER * 1024) {
       // thread-block cluster while one modulus per thread fits 16 CTAs: its exchange takes a
@@ -853,9 +866,17 @@ static int launch_convert(mgcd_context* c, Plan& P)
 {
   const uint32_t ng = (uint32_t)P.descs.size();
   const int grid = (int)std::min<uint32_t>(ng, (uint32_t)c->sms * 2);
-  CK(launch_radix(P.d_pairs.as<PairDesc>(), ng, P.d_digits.as<mgcd_pair>(), P.d_count.as<uint32_t>(),
-                  P.d_status.as<int32_t>(), P.d_glimbs.as<uint32_t>(), P.d_glen.as<uint32_t>(), grid, P.stream));
+  CK(launch_radix(P.din<PairDesc>(P.in.pairs), ng, P.dres<mgcd_pair>(P.res.digits), P.dres<uint32_t>(P.res.count),
+                  P.dres<int32_t>(P.res.status), P.dres<uint32_t>(P.res.glimbs), P.dres<uint32_t>(P.res.glen), grid, P.stream));
   ++P.launches;
+  return MGCD_OK;
+}
+
+// Fills the results' parts that the kernels add to or the host tells unwritten ones by.
+static int reset_results(Plan& P)
+{
+  CK(cudaMemsetAsync(P.d_res.p, 0xFF, P.res.upd, P.stream));
+  CK(cudaMemsetAsync(P.dres<void>(P.res.upd), 0, P.res.count - P.res.upd, P.stream));
   return MGCD_OK;
 }
 
@@ -874,16 +895,12 @@ int mgcd::run_plan(mgcd_context* c, Plan& P)
   for (size_t k = 0; k < ng; ++k) P.eff_nq[k] = P.descs[k].nq;
   if (c->use_graph && P.graphable && !P.plain) {
     if (!P.graph) {
-      // Record the run once (status reset, queue reset, the chained bucket kernels, the
+      // Record the run once (the results' reset, the chained bucket kernels, the
       // conversion); each later run is a single graph launch.
       CK(cudaStreamBeginCapture(P.stream, cudaStreamCaptureModeThreadLocal));
-      int rc = MGCD_OK;
-      if (cudaMemsetAsync(P.d_status.p, 0xFF, ng * sizeof(int32_t), P.stream) != cudaSuccess ||
-          cudaMemsetAsync(P.d_nqf.p, 0, ng * sizeof(uint32_t), P.stream) != cudaSuccess ||
-          cudaMemsetAsync(P.d_upd.p, 0, ng * sizeof(unsigned long long), P.stream) != cudaSuccess)
-        rc = MGCD_ERR_CUDA;
+      int rc = reset_results(P);
       if (rc == MGCD_OK)
-        rc = launch_set(c, P, P.buckets, P.grid_pairs, P.descs, P.d_pairs.as<PairDesc>(), P.d_queue.as<uint32_t>(),
+        rc = launch_set(c, P, P.buckets, P.grid_pairs, P.descs, P.din<PairDesc>(P.in.pairs), P.dres<uint32_t>(P.res.queue),
                         true);
       if (rc == MGCD_OK) rc = launch_convert(c, P);
       cudaGraph_t g = nullptr;
@@ -903,10 +920,9 @@ int mgcd::run_plan(mgcd_context* c, Plan& P)
     P.bucket_timed = true;
   } else {
     CK(cudaEventRecord(P.t_run0, P.stream));
-    CK(cudaMemsetAsync(P.d_status.p, 0xFF, ng * sizeof(int32_t), P.stream));
-    CK(cudaMemsetAsync(P.d_nqf.p, 0, ng * sizeof(uint32_t), P.stream));
-    CK(cudaMemsetAsync(P.d_upd.p, 0, ng * sizeof(unsigned long long), P.stream));
-    int rc = launch_set(c, P, P.buckets, P.grid_pairs, P.descs, P.d_pairs.as<PairDesc>(), P.d_queue.as<uint32_t>(),
+    int rc = reset_results(P);
+    if (rc == MGCD_OK)
+      rc = launch_set(c, P, P.buckets, P.grid_pairs, P.descs, P.din<PairDesc>(P.in.pairs), P.dres<uint32_t>(P.res.queue),
                         true);
     if (rc == MGCD_OK) rc = launch_convert(c, P);
     if (rc != MGCD_OK) return rc;
@@ -919,22 +935,28 @@ int mgcd::run_plan(mgcd_context* c, Plan& P)
 }
 
 // Waits for the run; pairs that ran with fewer moduli than the reference count and could
-// not be certified are rerun once with the reference count (same digit slots).
-int mgcd::sync_plan(mgcd_context* c, Plan& P)
+// not be certified are rerun once with the reference count (same digit slots).  With
+// `fetch_next` the caller goes on to fetch, which waits itself: a run in which no pair can be
+// rerun is not waited for here as well.
+int mgcd::sync_plan(mgcd_context* c, Plan& P, bool fetch_next)
 {
   if (!c || !P.ran) return MGCD_ERR_INVALID_ARG;
   CK(cudaSetDevice(c->device));
-  CK(cudaStreamSynchronize(P.stream));
-  if (P.synced) return MGCD_OK;
-  P.synced = true;
   const size_t ng = P.descs.size();
   bool scaled = false;
-  for (size_t k = 0; k < ng && !scaled; ++k) scaled = P.descs[k].nq < P.ref_nq[k];
-  if (!scaled) return MGCD_OK;
-  CK(P.h_status.grow(ng * sizeof(int32_t)));
-  CK(cudaMemcpyAsync(P.h_status.p, P.d_status.p, ng * sizeof(int32_t), cudaMemcpyDeviceToHost, P.stream));
+  if (!P.synced)
+    for (size_t k = 0; k < ng && !scaled; ++k) scaled = P.descs[k].nq < P.ref_nq[k];
+  if (!scaled) {
+    if (!fetch_next) CK(cudaStreamSynchronize(P.stream));
+    P.synced = true;
+    return MGCD_OK;
+  }
+  CK(P.h_res.grow(P.fetch_bytes()));
+  CK(cudaMemcpyAsync(P.hres<void>(P.res.status), P.dres<void>(P.res.status), ng * sizeof(int32_t),
+                     cudaMemcpyDeviceToHost, P.stream));
   CK(cudaStreamSynchronize(P.stream));
-  const int32_t* st = P.h_status.as<int32_t>();
+  P.synced = true;
+  const int32_t* st = P.hres<int32_t>(P.res.status);
   std::vector<uint32_t> redo;
   for (uint32_t k = 0; k < ng; ++k)
     if (st[k] != ST_OK && st[k] != ST_TIMEOUT && P.descs[k].nq < P.ref_nq[k]) redo.push_back(k);
@@ -955,24 +977,16 @@ int mgcd::sync_plan(mgcd_context* c, Plan& P)
   // device buffers: retry descriptors after the main ones, retry order after the main order
   cudaStream_t s = P.stream;
   CK(P.d_retry.grow(ng * sizeof(PairDesc), c->pool, s));
-  if (P.order.size() * sizeof(uint32_t) > P.d_order.bytes) {
-    // keep the main order: grow by copying
-    DevBuf nb;
-    CK(nb.grow(P.order.size() * sizeof(uint32_t), c->pool, s));
-    CK(cudaMemcpyAsync(nb.p, P.d_order.p, main_order * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-    P.drop_graph();
-    P.d_order.release(s);
-    P.d_order = nb;
-  }
   if (scratch > P.d_scratch.bytes / sizeof(uint32_t)) {
     P.drop_graph();
     P.d_scratch.release(s);
     CK(P.d_scratch.grow(scratch * sizeof(uint32_t), c->pool, s));
   }
   CK(cudaMemcpyAsync(P.d_retry.p, rd.data(), ng * sizeof(PairDesc), cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(P.d_order.as<uint32_t>() + main_order, P.order.data() + main_order,
+  CK(cudaMemsetAsync(P.dres<uint32_t>(P.res.queue) + NSTREAMS, 0, NSTREAMS * sizeof(uint32_t), s));
+  CK(cudaMemcpyAsync(P.din<uint32_t>(P.in.order) + main_order, P.order.data() + main_order,
                      (P.order.size() - main_order) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  rc = launch_set(c, P, bks, gp, rd, P.d_retry.as<PairDesc>(), P.d_queue.as<uint32_t>() + NSTREAMS, false,
+  rc = launch_set(c, P, bks, gp, rd, P.d_retry.as<PairDesc>(), P.dres<uint32_t>(P.res.queue) + NSTREAMS, false,
                   false);                   // the trace keeps the main run
   P.order.resize(main_order);               // the plan itself is unchanged for later runs
   P.grid_scratch_off = keep_grid_off;
@@ -990,35 +1004,20 @@ int mgcd::fetch(mgcd_context* c, Plan& P, uint32_t* direct_g)
   const size_t ng = P.descs.size();
   CK(cudaSetDevice(c->device));
   if (ng == 0) return MGCD_OK;
-  CK(P.h_count.grow(ng * sizeof(uint32_t)));
-  CK(P.h_iters.grow(ng * sizeof(uint32_t)));
-  CK(P.h_status.grow(ng * sizeof(int32_t)));
-  CK(P.h_glen.grow(ng * sizeof(uint32_t)));
   P.in_place = P.direct && direct_g != nullptr;
-  if (!P.in_place) CK(P.h_glimbs.grow(std::max<size_t>(P.nglimbs, 1) * sizeof(uint32_t)));
-  CK(P.h_nqf.grow(ng * sizeof(uint32_t)));
-  CK(P.h_upd.grow(ng * sizeof(unsigned long long)));
-  if (P.plain) CK(P.h_digits.grow(std::max<size_t>(P.ndig, 1) * sizeof(mgcd_pair)));
+  CK(P.h_res.grow(P.fetch_bytes()));
   cudaStream_t s = P.stream;
   // Results as binary limbs (converted on the device); digits only where the caller wants
   // them (single pairs) or the host converts (very long gcds).
-  CK(cudaMemcpyAsync(P.h_count.p, P.d_count.p, ng * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(P.h_iters.p, P.d_iters.p, ng * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(P.h_status.p, P.d_status.p, ng * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(P.h_glen.p, P.d_glen.p, ng * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(P.in_place ? (void*)(direct_g + P.direct_base) : P.h_glimbs.p, P.d_glimbs.p,
-                     P.nglimbs * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(P.h_nqf.p, P.d_nqf.p, ng * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(P.h_upd.p, P.d_upd.p, ng * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-  uint64_t d2h = ng * (5 * sizeof(uint32_t) + sizeof(unsigned long long)) + P.nglimbs * sizeof(uint32_t);
-  if (P.plain) {
-    CK(cudaMemcpyAsync(P.h_digits.p, P.d_digits.p, P.ndig * sizeof(mgcd_pair), cudaMemcpyDeviceToHost, s));
-    d2h += P.ndig * sizeof(mgcd_pair);
-  }
+  CK(cudaMemcpyAsync(P.h_res.p, P.d_res.p, P.in_place ? P.res.glimbs : P.fetch_bytes(), cudaMemcpyDeviceToHost, s));
+  if (P.in_place)
+    CK(cudaMemcpyAsync(direct_g + P.direct_base, P.dres<void>(P.res.glimbs), P.nglimbs * sizeof(uint32_t),
+                       cudaMemcpyDeviceToHost, s));
+  uint64_t d2h = P.in_place ? P.res.glimbs + P.nglimbs * sizeof(uint32_t) : P.fetch_bytes();
   CK(cudaStreamSynchronize(s));
   if (!P.plain) {
-    const uint32_t* gl = P.h_glen.as<uint32_t>();
-    const int32_t* st0 = P.h_status.as<int32_t>();
+    const uint32_t* gl = P.hres<uint32_t>(P.res.glen);
+    const int32_t* st0 = P.hres<int32_t>(P.res.status);
     bool any = false;
     for (size_t k = 0; k < ng && !any; ++k) any = gl[k] == RADIX_HOST && st0[k] == ST_OK;
     if (any) CK(P.h_digits.grow(std::max<size_t>(P.ndig, 1) * sizeof(mgcd_pair)));
@@ -1026,23 +1025,24 @@ int mgcd::fetch(mgcd_context* c, Plan& P, uint32_t* direct_g)
     for (size_t k = 0; k < ng; ++k) {
       if (gl[k] != RADIX_HOST || st0[k] != ST_OK) continue;
       const PairDesc& d = P.descs[k];
-      const size_t n = P.h_count.as<uint32_t>()[k];
-      CK(cudaMemcpyAsync(P.h_digits.as<mgcd_pair>() + d.out_off, P.d_digits.as<mgcd_pair>() + d.out_off,
+      const size_t n = P.hres<uint32_t>(P.res.count)[k];
+      CK(cudaMemcpyAsync(P.h_digits.as<mgcd_pair>() + d.out_off, P.dres<mgcd_pair>(P.res.digits) + d.out_off,
                          n * sizeof(mgcd_pair), cudaMemcpyDeviceToHost, s));
       d2h += n * sizeof(mgcd_pair);
       any = true;
     }
     if (any) CK(cudaStreamSynchronize(s));
   }
+  P.fetched = true;
   P.d2h_bytes = d2h;
   // work by the cost model
-  const uint32_t* it = P.h_iters.as<uint32_t>();
-  const uint32_t* cnt = P.h_count.as<uint32_t>();
-  const int32_t* st = P.h_status.as<int32_t>();
+  const uint32_t* it = P.hres<uint32_t>(P.res.iters);
+  const uint32_t* cnt = P.hres<uint32_t>(P.res.count);
+  const int32_t* st = P.hres<int32_t>(P.res.status);
   double R = 0, E = 0, M = 0, B = 0, AB = 0;
   std::vector<double> pw(4 * ng, 0.0);    // per pair: R, E, M, B
-  const uint32_t* nqf = P.h_nqf.as<uint32_t>();
-  const unsigned long long* upd = P.h_upd.as<unsigned long long>();
+  const uint32_t* nqf = P.hres<uint32_t>(P.res.nqf);
+  const unsigned long long* upd = P.hres<unsigned long long>(P.res.upd);
   for (size_t k = 0; k < ng; ++k) {
     const PairDesc& d = P.descs[k];
     double* w = &pw[4 * k];
@@ -1076,11 +1076,11 @@ int mgcd::convert_all(mgcd_context* c, Plan& P, uint32_t* g, const uint64_t* g_o
 {
   (void)c;
   const size_t np = P.np;
-  const mgcd_pair* dig = P.h_digits.as<mgcd_pair>();
-  const uint32_t* cnt = P.h_count.as<uint32_t>();
-  const int32_t* st = P.h_status.as<int32_t>();
-  const uint32_t* gl = P.h_glen.as<uint32_t>();
-  const uint32_t* gv = P.h_glimbs.as<uint32_t>();
+  const mgcd_pair* dig = P.plain ? P.hres<mgcd_pair>(P.res.digits) : P.h_digits.as<mgcd_pair>();
+  const uint32_t* cnt = P.hres<uint32_t>(P.res.count);
+  const int32_t* st = P.hres<int32_t>(P.res.status);
+  const uint32_t* gl = P.hres<uint32_t>(P.res.glen);
+  const uint32_t* gv = P.hres<uint32_t>(P.res.glimbs);
   std::atomic<size_t> next{0};
   auto work = [&]() {
     for (;;) {
@@ -1349,7 +1349,7 @@ static int bucket_span_ms(const mgcd_context* c, int i, float* ms)
 {
   unsigned long long sp[2] = {0, 0};
   CK(cudaSetDevice(c->device));
-  CK(cudaMemcpy(sp, c->main.d_span.as<unsigned long long>() + 2 * i, sizeof sp, cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(sp, c->main.dres<unsigned long long>(c->main.res.span) + 2 * i, sizeof sp, cudaMemcpyDeviceToHost));
   const unsigned long long t0 = sp[0], t1 = ~sp[1];
   *ms = (sp[0] != ~0ull && sp[1] != ~0ull && t1 >= t0) ? (float)((double)(t1 - t0) * 1e-6) : 0.f;
   return MGCD_OK;
@@ -1545,17 +1545,17 @@ int mgcd_batch_pair_digits(mgcd_context* c, size_t i, mgcd_pair* out, size_t cap
   Plan& P = c->main;
   if (!P.synced || i >= P.np) return MGCD_ERR_INVALID_ARG;
   const int k = P.slot[i];
-  if (k < 0 || P.h_count.p == nullptr) return MGCD_ERR_INVALID_ARG;
-  const size_t cnt = P.h_count.as<uint32_t>()[k];
+  if (k < 0 || !P.fetched) return MGCD_ERR_INVALID_ARG;
+  const size_t cnt = P.hres<uint32_t>(P.res.count)[k];
   *n = cnt;
   if (nq_final) {
-    const uint32_t f = P.h_nqf.p ? P.h_nqf.as<uint32_t>()[k] : 0u;
+    const uint32_t f = P.hres<uint32_t>(P.res.nqf)[k];
     *nq_final = (f != 0u && P.eff_nq[k] == P.descs[k].nq) ? f : P.eff_nq[k];
   }
   if (cnt > cap) return MGCD_ERR_CAPACITY;
   CK(cudaSetDevice(c->device));
   if (cnt)
-    CK(cudaMemcpy(out, P.d_digits.as<mgcd_pair>() + P.descs[k].out_off, cnt * sizeof(mgcd_pair),
+    CK(cudaMemcpy(out, P.dres<mgcd_pair>(P.res.digits) + P.descs[k].out_off, cnt * sizeof(mgcd_pair),
                   cudaMemcpyDeviceToHost));
   return MGCD_OK;
 }
@@ -1566,7 +1566,7 @@ int mgcd_batch_download(mgcd_context* c, uint32_t* g, const uint64_t* g_off, con
   if (!c) return MGCD_ERR_INVALID_ARG;
   Plan& P = c->main;
   if (!P.ran || (P.np && (!g || !g_off || !g_cap || !g_len || !status))) return MGCD_ERR_INVALID_ARG;
-  int rc = sync_plan(c, P);
+  int rc = sync_plan(c, P, true);
   if (rc != MGCD_OK) return rc;
   rc = fetch(c, P);
   if (rc != MGCD_OK) return rc;
@@ -1586,7 +1586,7 @@ int mgcd_gcd_batch(mgcd_context* c, size_t np, const uint32_t* limbs, const uint
   if (rc != MGCD_OK) return rc;
   rc = run_plan(c, P);
   if (rc != MGCD_OK) return rc;
-  rc = sync_plan(c, P);
+  rc = sync_plan(c, P, true);
   if (rc != MGCD_OK) return rc;
   rc = fetch(c, P, g);
   if (rc != MGCD_OK) return rc;
@@ -1611,7 +1611,7 @@ static int single(mgcd_context* c, const uint32_t* u, size_t uSz, const uint32_t
   if (rc != MGCD_OK) return rc;
   rc = run_plan(c, P);
   if (rc != MGCD_OK) return rc;
-  rc = sync_plan(c, P);
+  rc = sync_plan(c, P, true);
   if (rc != MGCD_OK) return rc;
   return fetch(c, P);
 }
@@ -1626,11 +1626,11 @@ int mgcd_gcd_digits(mgcd_context* c, const uint32_t* u, size_t uSz, const uint32
   if (rc != MGCD_OK) return rc;
   const Plan& P = c->main;
   if (P.slot[0] < 0) return P.status[0];
-  const int32_t st = P.h_status.as<int32_t>()[0];
+  const int32_t st = P.hres<int32_t>(P.res.status)[0];
   if (st != ST_OK) return to_status(st);
-  const uint32_t n = P.h_count.as<uint32_t>()[0];
+  const uint32_t n = P.hres<uint32_t>(P.res.count)[0];
   if (n > cap) return MGCD_ERR_CAPACITY;
-  std::memcpy(digits, P.h_digits.as<mgcd_pair>() + P.descs[0].out_off, n * sizeof(mgcd_pair));
+  std::memcpy(digits, P.hres<mgcd_pair>(P.res.digits) + P.descs[0].out_off, n * sizeof(mgcd_pair));
   *count = n;
   return MGCD_OK;
 }

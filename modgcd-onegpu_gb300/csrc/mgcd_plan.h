@@ -78,7 +78,7 @@ struct Plan {
   std::vector<uint32_t> ref_nq, eff_nq; // per GPU pair: reference count, count of the final run
   size_t ndig = 0, scratch_words = 0, grid_scratch_off = 0;
   size_t nglimbs = 0;                  // result limbs reserved (sum of g_cap)
-  // results planned in the caller's layout (mgcd_gcd_batch, slots contiguous): d_glimbs[x]
+  // results planned in the caller's layout (mgcd_gcd_batch, slots contiguous): the device's limb x
   // is the caller's g[direct_base + x], copied there in one piece; in_place: fetch did so
   bool direct = false, in_place = false;
   uint64_t direct_base = 0;
@@ -90,14 +90,30 @@ struct Plan {
                                        // context's setting); serving waves favour latency
   int cluster_k = 0;                   // pairs per cluster of size class 3 (0: the context's setting)
 
-  DevBuf d_limbs, d_pairs, d_order, d_digits, d_count, d_iters, d_status, d_queue, d_scratch, d_retry;
-  DevBuf d_nqf, d_upd;                 // per pair (K-slot kernels): final moduli count, loop updates
-  DevBuf d_span;                       // per bucket kernel: earliest CTA start, ~(latest CTA end), ns
-  DevBuf d_glimbs, d_glen;             // binary gcds converted on the device
+  // One block for what goes up and one for what comes back, so that a small call costs one
+  // copy each way and two fills: a copy or a fill takes about 2 us of the stream and as much of
+  // the host, and the separate buffers had 3 copies up, 8 back and 5 fills (a 512-bit pair
+  // 125 us with them, 106 with the blocks).
+  DevBuf d_in;                         // operand limbs, then `in`'s parts
+  DevBuf d_res;                        // `res`'s parts
+  struct In { size_t pairs = 0, order = 0, end = 0; } in;      // byte offsets; order has room for a rerun's
+  struct Res {                         // byte offsets
+    size_t span = 0, status = 0;       // filled with ones: span (per bucket kernel: earliest CTA
+                                       // start, ~(latest CTA end), ns), status per pair
+    size_t upd = 0, nqf = 0, queue = 0;   // zeroed: per pair (K-slot kernels) loop updates and final
+                                       // moduli count; the buckets' work counters, a rerun's after them
+    size_t count = 0, iters = 0, glen = 0;   // per pair
+    size_t glimbs = 0;                 // binary gcds converted on the device
+    size_t digits = 0, end = 0;
+  } res;
+  std::vector<unsigned char> in_host;  // a small plan's d_in, put together for one copy
+  DevBuf d_scratch, d_retry;
   DevBuf d_trace;                      // per-CTA occupancy trace of the bucket kernels (4 words each)
   DevBuf d_phases;                     // per-CTA phase accounting of the K-slot kernels (8 words each)
   std::vector<int> trace_cls;          // size class of each traced CTA (launch order)
-  HostBuf h_count, h_iters, h_status, h_digits, h_glimbs, h_glen, h_nqf, h_upd;
+  HostBuf h_res;                       // d_res's start, up to what fetch copies
+  HostBuf h_digits;                    // digits the host converts (batches)
+  bool fetched = false;                // h_res holds a run of this plan
   int launches = 0, retried = 0;
   bool ran = false, synced = false, bucket_timed = false;
   double work[4] = {0, 0, 0, 0};       // residue steps, loop updates, recovery updates, operand bytes
@@ -113,6 +129,11 @@ struct Plan {
   void destroy(cudaMemPool_t pool);
   void drop_graph();
   size_t device_bytes() const;
+  void layout(size_t ng, uint64_t limb_words);
+  size_t fetch_bytes() const { return plain ? res.end : res.digits; }   // d_res's part for the host
+  template <class T> T* din(size_t off) const { return reinterpret_cast<T*>(d_in.as<unsigned char>() + off); }
+  template <class T> T* dres(size_t off) const { return reinterpret_cast<T*>(d_res.as<unsigned char>() + off); }
+  template <class T> T* hres(size_t off) const { return reinterpret_cast<T*>(h_res.as<unsigned char>() + off); }
 };
 
 }  // namespace mgcd
@@ -164,7 +185,7 @@ int plan_batch(mgcd_context* c, Plan& P, size_t np, const uint32_t* limbs, const
                const uint32_t* u_len, const uint64_t* v_off, const uint32_t* v_len, bool plain,
                const uint64_t* g_off = nullptr, const uint32_t* g_cap = nullptr);
 int run_plan(mgcd_context* c, Plan& P);
-int sync_plan(mgcd_context* c, Plan& P);
+int sync_plan(mgcd_context* c, Plan& P, bool fetch_next = false);
 int fetch(mgcd_context* c, Plan& P, uint32_t* direct_g = nullptr);
 int convert_all(mgcd_context* c, Plan& P, uint32_t* g, const uint64_t* g_off, const uint32_t* g_cap,
                 uint32_t* g_len, int32_t* status, bool threaded);

@@ -207,7 +207,7 @@ int finish_wave(mgcd_server* S, Wave& w)
 {
   mgcd_context* c = S->c;
   const size_t n = w.reqs.size();
-  int rc = sync_plan(c, w.plan);
+  int rc = sync_plan(c, w.plan, true);
   if (rc == MGCD_OK) rc = fetch(c, w.plan);
   if (rc != MGCD_OK) return rc;
   w.goff.resize(n); w.gcap.resize(n); w.glen.resize(n); w.st.resize(n);
