@@ -138,15 +138,17 @@ int mgcd_set_nq_scale(mgcd_context *ctx, float scale);
    state it would have had from the start (residues of the operands, then the pivots so far
    replayed on it), so the result is the pair's gcd as before; the pivots after a growth may
    differ from a run with the larger set from the start.  A pair that still fails is rerun
-   with the reference's count.  start in [0.1, 1] with step_permille in [10, 500], or
+   with the reference's count.  A batch of at most half as many pairs as the GPU has SMs
+   runs them on clusters with the larger of the reference's count and the cap from the
+   start.  start in [0.1, 1] with step_permille in [10, 500], or
    start = 0 (off: the class fractions of mgcd_set_nq_scale apply).  Default 0.4, 50.
    No counterpart in the reference (its count is fixed per call, GmpCudaDevice-gcd.cu:49-55). */
 int mgcd_set_growth(mgcd_context *ctx, float start, unsigned step_permille);
 int mgcd_get_growth(const mgcd_context *ctx, float *start, unsigned *step_permille);
-/* Launch shape of single pairs too large for one CTA:
+/* Launch shape of single pairs too large for one CTA (above 512 moduli):
      MGCD_SINGLE_AUTO              a thread-block cluster of up to 16 CTAs (pivot exchange
                                    through distributed shared memory) while the pair's
-                                   moduli fit 16 x 512 threads, else a cooperative grid
+                                   moduli fit 16 x 1,024 threads, else a cooperative grid
                                    with at most one CTA per SM and a leader exchange of
                                    tagged per-CTA slots (default);
      MGCD_SINGLE_REFERENCE_SHAPE   the reference's launch shape: a cooperative grid of
@@ -154,7 +156,7 @@ int mgcd_get_growth(const mgcd_context *ctx, float *start, unsigned *step_permil
                                    exchange per iteration (GmpCudaDevice-gcd.cu:80-96). */
 #define MGCD_SINGLE_AUTO            0
 #define MGCD_SINGLE_REFERENCE_SHAPE 1
-/*   MGCD_SINGLE_CLUSTER_GRID      above 16 x 512 moduli: a cooperative grid of 8-CTA
+/*   MGCD_SINGLE_CLUSTER_GRID      above 16 x 1,024 moduli: a cooperative grid of 8-CTA
                                    clusters; keys meet in each cluster through DSMEM and one
                                    leader per cluster joins a global exchange of atomic
                                    minimum and arrival counter (measured 20-40 % slower than

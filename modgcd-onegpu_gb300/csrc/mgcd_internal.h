@@ -108,7 +108,7 @@ struct BatchArgs {
 
 // State of the cross-CTA reduction used by a single pair spread over a cooperative grid.
 // Cooperative grid (leader exchange), exchange e: every CTA stores its minimum, tagged with
-// bit (e / 2 + 1) & 1, into keys[e & 1][cta]; CTA 0 polls all slots until their tags
+// bit (e / 2 + 1) & 1, into its slot of half e & 1 of keys; CTA 0 polls all slots until their tags
 // match, reduces them and stores the tagged result into bcast[e & 1]; the other CTAs poll
 // that word.  A slot read in exchange e holds the value of e or of e - 2 (no CTA can be two
 // exchanges ahead of another), which the tag tells apart: no atomics and no fences.
@@ -178,9 +178,9 @@ cudaError_t launch_cluster_batch(const BatchArgs& a, int threads, int k, int csi
 cudaError_t cgrid_max_clusters(int threads, int csize, size_t smem, int* clusters);
 cudaError_t launch_cgrid(const GridArgs& a, int threads, int csize, int clusters, size_t smem, cudaStream_t s);
 
-// Resets the grid exchange state on the device (capturable in a CUDA graph).
 // Times n exchanges of `ctas` CTAs through *gs, for choosing where the exchange's lines live.
 cudaError_t launch_exchange_probe(GridSync* gs, int ctas, uint32_t n, unsigned long long* cycles, cudaStream_t s);
+// Resets the grid exchange state on the device (capturable in a CUDA graph).
 cudaError_t launch_gridsync_init(GridSync* gs, unsigned long long timeout_ns, uint32_t withhold, cudaStream_t s);
 
 size_t grid_smem_bytes(uint32_t per_cta);

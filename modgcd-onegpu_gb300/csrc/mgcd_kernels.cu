@@ -6,7 +6,7 @@
 // Stages, with the reference's labels (GmpCudaDevice-getGcdKernel.cu:342-444):
 //   MGCD2  residues of u and v for every modulus: limb tiles brought into shared memory by
 //          bulk copies (cp.async.bulk, double-buffered), Montgomery Horner per modulus
-//          (z <- REDC(z * 2^64 mod q + limb));
+//          (four limbs a step, two for 32-bit moduli);
 //   MGCD3  reduction loop: per modulus only t = u/v mod q is kept; each iteration picks
 //          the pivot (p, b) = argmin of the reference's key (|t|, q - sign) with warp
 //          redux.sync minima and one barrier (plus a DSMEM or grid exchange across CTAs),
@@ -16,8 +16,8 @@
 //          to their initial residues projectively (three Montgomery products per step, no
 //          inverse) and dividing out the accumulated scale once;
 //   MGCD4  recovery: signed mixed-radix digits, next digit from the lowest-indexed
-//          modulus with a nonzero value, exactly as the reference selects it (in panels of
-//          up to 32 digits when the pair spans several CTAs).
+//          modulus with a nonzero value, exactly as the reference selects it, in panels of
+//          up to 32 digits.
 // The (p, b) sequence and the digits are identical to the reference algorithm's.
 #include <cstdint>
 #include <cstdlib>
@@ -765,8 +765,8 @@ __global__ void __launch_bounds__(T, K < 8 ? 1024 / T : 1) batchk_kernel(const B
     }
     ph_mark(PH_UPDATE);
     // ---- the next pivots (GmpCudaDevice-getGcdKernel.cu:365-402): warp minima, one
-    // barrier, then warp s reduces slot s's minima, stores its pivot and steps its
-    // bookkeeping (the K slots in parallel)
+    // barrier, then warp s reduces slot s's minima and stores its pivot
+    // (the K slots in parallel)
 #pragma unroll
     for (int s = 0; s < K; ++s) {
       warp_min_key(kh[s], kl[s]);

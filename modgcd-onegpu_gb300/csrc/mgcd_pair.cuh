@@ -17,7 +17,7 @@ constexpr uint32_t REPLAY_CHUNK = 512;   // history entries per replay chunk (2 
 // How the CTAs that share one pair synchronise.
 enum SyncMode : int {
   SYNC_CTA = 0,      // the pair lives in one CTA
-  SYNC_CLUSTER = 1,  // the pair spans a thread-block cluster: DSMEM exchange + barrier.cluster
+  SYNC_CLUSTER = 1,  // the pair spans a thread-block cluster: tagged DSMEM exchange, bounded polls
   SYNC_GRID = 2,     // the pair spans a cooperative grid: global-memory exchange, bounded wait
   SYNC_CGRID = 3     // a cooperative grid of clusters: DSMEM inside each cluster, one
                      // leader per cluster in the global exchange
