@@ -163,13 +163,15 @@ int mgcd_get_growth(const mgcd_context *ctx, float *start, unsigned *step_permil
                                    the default on GB300). */
 #define MGCD_SINGLE_CLUSTER_GRID    2
 int mgcd_set_single_pair_policy(mgcd_context *ctx, int policy);
-/* Bound of every wait a cooperative-grid pair makes on the other CTAs (default 2,000 ms).
-   When it runs out, every CTA returns and the pair fails with MGCD_ERR_TIMEOUT; the
-   context stays usable.  (The reference's grid barrier spins without a bound,
-   GmpCuda.h:68-83.) */
+/* Bound of every wait for another CTA's key by a pair that spans several CTAs, on a cluster
+   or a cooperative grid (default 2,000 ms).  When it runs out, every CTA leaves the pair and
+   it fails with MGCD_ERR_TIMEOUT (in a batch, the pairs that share the cluster's slots; the
+   cluster goes on with the others); the context stays usable.  The allocation-free call
+   waits 2,000 ms.  (The reference's grid barrier spins without a bound, GmpCuda.h:68-83.) */
 int mgcd_set_wait_timeout_ms(mgcd_context *ctx, unsigned ms);
-/* Test hook for the bounded waits: CTA `cta` of the next cooperative-grid pairs never
-   publishes its minimum, so the other CTAs' waits run out (-1 turns the hook off). */
+/* Test hook for the bounded waits: the CTA with block index `cta` of the next grid and
+   cluster kernels never publishes its minimum, so the other CTAs' waits run out (-1 turns
+   the hook off). */
 int mgcd_test_withhold_cta(mgcd_context *ctx, int cta);
 /* Test hook for the operand-staging failure path: the CTA with block index `cta` of every
    later kernel (batched, cluster or grid) reports that its bulk copies of the operand limbs

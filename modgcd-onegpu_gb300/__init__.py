@@ -411,7 +411,7 @@ class Device:
         _check(self._lib.mgcd_set_wait_timeout_ms(self._h, int(ms)))
 
     def test_withhold_cta(self, cta):
-        """Test hook: CTA `cta` of grid-mode pairs never publishes (-1: off)."""
+        """Test hook: CTA `cta` of grid and cluster kernels never publishes (-1: off)."""
         _check(self._lib.mgcd_test_withhold_cta(self._h, int(cta)))
 
     def test_fail_staging(self, cta):

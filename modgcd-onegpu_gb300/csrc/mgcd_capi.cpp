@@ -756,6 +756,8 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
       P.trace_cls.insert(P.trace_cls.end(), n, bk.cls);
     }
     a.stage_fail = c->stage_fail_cta;
+    a.wait_ns = c->wait_timeout_ns;
+    a.withhold = c->withhold_cta;
     a.inv = InvTab{c->d_invtab.as<uint32_t>(), c->invtab_n};
     a.limbs = P.din<uint32_t>(0);
     a.pairs = pairs;
@@ -785,6 +787,8 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     const PairDesc& d = descs[k];
     GridArgs g;
     g.stage_fail = c->stage_fail_cta;
+    g.wait_ns = c->wait_timeout_ns;
+    g.withhold = c->withhold_cta;
     g.inv = InvTab{c->d_invtab.as<uint32_t>(), c->invtab_n};
     g.limbs = P.din<uint32_t>(0);
     g.pair = d;

@@ -91,6 +91,8 @@ struct BatchArgs {
   uint32_t* iters;           // reduction iterations per pair (work accounting)
   int32_t* status;
   uint32_t stage_fail;       // test hook: this CTA reports an operand-staging failure (~0: none)
+  unsigned long long wait_ns;  // clusters: bound of every wait
+  uint32_t withhold;         // clusters, test hook: this CTA's keys reach no other CTA (~0: none)
   unsigned long long* trace; // per CTA: start and end (globaltimer ns), SM id, pairs taken (null: off)
   unsigned long long* phases; // per CTA (K-slot kernel, PHASE_WORDS each): clock cycles of thread 0 in
                               // set-up, update, pivot choice and finish, reduction iterations, moduli
@@ -144,6 +146,8 @@ struct GridArgs {
   uint32_t* iters;
   int32_t* status;
   uint32_t stage_fail;       // test hook: this CTA reports an operand-staging failure (~0: none)
+  unsigned long long wait_ns;  // one cluster: bound of every wait (a grid's: GridSync)
+  uint32_t withhold;         // one cluster, test hook: this CTA's keys reach no other CTA (~0: none)
 };
 
 // Launch helpers (mgcd_kernels.cu).

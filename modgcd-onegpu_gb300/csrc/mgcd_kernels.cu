@@ -828,8 +828,10 @@ __global__ void __launch_bounds__(T, K < 8 ? 1024 / T : 1) batchk_kernel(const B
 // pair (per = ceil(nq_max / C), the same slice for all slots, so a thread's K updates share
 // one modulus and one inverse).  Pivot keys: after the warp minima and one __syncthreads, warp
 // s reduces slot s's and exchanges it with the other CTAs (cluster_min_key, the K slots in
-// parallel).  Queue pops are made by CTA 0 and broadcast through DSMEM.  Set-up and finish of one slot run the cluster single-pair code
-// on the CTA's slice while the other slots wait.
+// parallel).  Queue pops are made by CTA 0 and broadcast through DSMEM.  Set-up and finish of
+// one slot run the cluster single-pair code on the CTA's slice while the other slots wait.
+// When a wait expires the CTAs meet at their next cluster barrier (cluster_meet), the pairs in
+// the slots time out and the cluster goes on with the queue.
 
 template <int K>
 struct SlotSmem {
@@ -859,12 +861,13 @@ __device__ __forceinline__ bool cluster_min_keys(uint32_t (&kh)[K], uint32_t (&k
     warp_min_key(kh[s], kl[s]);
     if (lane == 0) ss.key[s][w] = ((unsigned long long)kh[s] << 32) | kl[s];
   }
+  const bool withhold = cs.withhold != 0u;
   __syncthreads();
   if (w < K) {
     const unsigned long long k = lane < T / 32 ? ss.key[w][lane] : ~0ull;
     uint32_t h = (uint32_t)(k >> 32), l = (uint32_t)k;
     warp_min_key(h, l);
-    cluster_min_key(h, l, ck.key[b][w], cs, key_tag(epoch));
+    cluster_min_key(h, l, ck.key[b][w], cs, key_tag(epoch), withhold);
     if (lane == 0) ck.res[b][w] = ((unsigned long long)h << 32) | l;
   }
   __syncthreads();
@@ -874,7 +877,7 @@ __device__ __forceinline__ bool cluster_min_keys(uint32_t (&kh)[K], uint32_t (&k
     kl[s] = (uint32_t)ck.res[b][s];
   }
   epoch += 1u;
-  return cs.dead == 0u;
+  return cs.failed == 0u;
 }
 
 // NARROW: moduli below 2^30, as in batchk_kernel.
@@ -900,32 +903,41 @@ __global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
   const int L = a.L;
   GridSync* const gcs = reinterpret_cast<GridSync*>(&cs);
   // exchange counts: slot keys (ck), single keys (rs in the CTA, cs across the cluster)
-  uint32_t kepoch = 0, rparity = 0, repoch = 0;
-  uint32_t valid = 0, active = 0, redux = 0;
+  uint32_t kepoch, rparity = 0, repoch;
+  uint32_t valid, active;
   int rem[K], ubits[K], vbits[K];
   uint32_t iters[K], p[K], kh[K], kl[K];
   int32_t b[K];
   cta_begin(a);
   uint32_t taken = 0;
 
-  for (uint32_t i = threadIdx.x; i < 2u * K * MAX_CLUSTER; i += T) (&ck.key[0][0][0])[i] = 0ull;
-  cluster_exchange_init(cs);
+  // The exchanges and slots at the start, and again after an expired wait.
+  auto start = [&]() {
+    kepoch = repoch = valid = active = 0u;
+    for (uint32_t i = threadIdx.x; i < 2u * K * MAX_CLUSTER; i += T) (&ck.key[0][0][0])[i] = 0ull;
+    cluster_exchange_init(cs, a.wait_ns, blockIdx.x == a.withhold);
+  };
   // Takes the next pair of the queue into slot s.  A CTA whose operands could not be staged
   // contributes the key (0, 0) (no modulus produces it), so the whole cluster answers that
-  // pair with ST_TIMEOUT and takes the next one together.
+  // pair with ST_TIMEOUT and takes the next one together.  A wait that expires while a pair is
+  // taken loses that pair (the one of ck.next) and ends in cs.lost.
+  auto lost_pair = [&]() {
+    if (r == 0 && threadIdx.x == 0 && ck.next < a.npairs) {
+      a.status[a.order[ck.next]] = ST_TIMEOUT;
+      a.count[a.order[ck.next]] = 0;
+    }
+    return false;
+  };
   auto load = [&](int s) -> bool {
     uint32_t h0, l0;
     for (;;) {
       if (r == 0 && threadIdx.x < C) {
         const uint32_t k = __shfl_sync(0xFFFFFFFFu >> (32 - C), threadIdx.x == 0 ? atomicAdd(a.queue, 1u) : 0u, 0);
-        const uint32_t ad = (uint32_t)__cvta_generic_to_shared(&ck.next);
-        uint32_t ra;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(ad), "r"(threadIdx.x));
-        asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(ra), "r"(k) : "memory");
+        st_cluster_u32(&ck.next, threadIdx.x, k);
       }
-      cluster_sync_all();
+      if (!cluster_meet(cs)) return lost_pair();
       const uint32_t k = ck.next;
-      cluster_sync_all();                             // everyone has read next before it changes
+      if (!cluster_meet(cs)) return lost_pair();      // everyone has read next before it changes
       if (k >= a.npairs) return false;
       ++taken;
       if (threadIdx.x == 0) {
@@ -960,7 +972,10 @@ __global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
         ss.lv[s] = bound_init(a.limbs + d.v_off, d.v_len);
       }
       if (!ok) h0 = l0 = 0u;
-      if (!reduce_min<T, SYNC_CLUSTER>(h0, l0, rs, rparity, gcs, repoch)) h0 = l0 = 0u;
+      if (!reduce_min<T, SYNC_CLUSTER>(h0, l0, rs, rparity, gcs, repoch)) {
+        cluster_meet(cs);
+        return lost_pair();
+      }
       if (h0 != 0u || l0 != 0u) break;
       if (r == 0 && threadIdx.x == 0) {
         a.status[ss.pi[s]] = ST_TIMEOUT;
@@ -982,32 +997,44 @@ __global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
     return true;
   };
 
-#pragma unroll 1
-  for (int s = 0; s < K; ++s)
-    if (load(s)) { valid |= 1u << s; active |= 1u << s; }
-
+  constexpr uint32_t ALL = (1u << K) - 1u, LOST = 1u << K;
+  uint32_t empty = ALL;                               // slots to fill; LOST: the exchange failed
+  start();
   for (;;) {
+    if (empty == LOST) {                              // the pairs in the slots time out, the queue goes on
+      if (r == 0 && threadIdx.x < K && ((valid >> threadIdx.x) & 1u)) {
+        a.status[ss.pi[threadIdx.x]] = ST_TIMEOUT;
+        a.count[ss.pi[threadIdx.x]] = 0;
+      }
+      __syncthreads();
+      start();
+      empty = ALL;
+    }
     const uint32_t done = valid & ~active;
 #pragma unroll 1
-    for (int s = 0; s < K; ++s) {
-      if (!((done >> s) & 1u)) continue;
-      const uint32_t pi = ss.pi[s];
-      const uint32_t it = pick(iters, s);
-      if (threadIdx.x == 0 && r == 0) a.iters[pi] = it;
-      if ((redux >> s) & 1u) {
-        if (threadIdx.x == 0 && r == 0) { a.status[pi] = ST_REDUX; a.count[pi] = 0; }
-      } else {
-        uint32_t* u0 = scr + (size_t)s * 4 * NQS;
-        finish_pair<T, SYNC_CLUSTER>(a.mods, ss.d[s], L, j0, ck.nloc[s], tS + (size_t)s * per, rs, rparity, repoch,
-                                     gcs, u0 + j0, u0 + NQS + j0, reinterpret_cast<const int2*>(u0 + 2 * (size_t)NQS),
-                                     it, pick(rem, s), ss.lu[s], ss.lv[s], 0u, a.digits, a.count + pi, a.status + pi,
-                                     a.inv, smem, acc2);
+    for (int s = 0; s < K && empty != LOST; ++s) {
+      if (!(((done | empty) >> s) & 1u)) continue;
+      if ((done >> s) & 1u) {
+        const uint32_t pi = ss.pi[s];
+        const uint32_t it = pick(iters, s);
+        if (threadIdx.x == 0 && r == 0) a.iters[pi] = it;
+        if (pick(b, s) != MOD_INFINITY) {             // the loop ran out of moduli
+          if (threadIdx.x == 0 && r == 0) { a.status[pi] = ST_REDUX; a.count[pi] = 0; }
+        } else {
+          uint32_t* u0 = scr + (size_t)s * 4 * NQS;
+          finish_pair<T, SYNC_CLUSTER>(a.mods, ss.d[s], L, j0, ck.nloc[s], tS + (size_t)s * per, rs, rparity, repoch,
+                                       gcs, u0 + j0, u0 + NQS + j0, reinterpret_cast<const int2*>(u0 + 2 * (size_t)NQS),
+                                       it, pick(rem, s), ss.lu[s], ss.lv[s], 0u, a.digits, a.count + pi, a.status + pi,
+                                       a.inv, smem, acc2);
+        }
+        valid &= ~(1u << s);
+        if (!cluster_meet(cs)) { empty = LOST; break; }   // the slot's scratch is free in every CTA
       }
-      cluster_sync_all();                             // the slot's scratch is free in every CTA
-      valid &= ~(1u << s);
-      redux &= ~(1u << s);
+      empty &= ~(1u << s);
       if (load(s)) { valid |= 1u << s; active |= 1u << s; }
+      else if (cs.lost) empty = LOST;
     }
+    if (empty == LOST) continue;
     if (!valid) break;
 
 #pragma unroll
@@ -1027,7 +1054,7 @@ __global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
       const int tbits = ubits[s] - (L - 1) + __ffs((int)ab);
       ubits[s] = vbits[s];
       vbits[s] = tbits;
-      if (rem[s] * (L - 2) <= ubits[s]) { redux |= 1u << s; active &= ~(1u << s); }
+      if (rem[s] * (L - 2) <= ubits[s]) active &= ~(1u << s);
     }
     if (!active) continue;
 
@@ -1050,11 +1077,9 @@ __global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
       });
     }
     if (!cluster_min_keys<T, K>(kh, kl, ss, ck, cs, kepoch)) {
-      if (r == 0 && threadIdx.x < K && ((valid >> threadIdx.x) & 1u)) {
-        a.status[ss.pi[threadIdx.x]] = ST_TIMEOUT;
-        a.count[ss.pi[threadIdx.x]] = 0;
-      }
-      break;
+      cluster_meet(cs);
+      empty = LOST;
+      continue;
     }
 #pragma unroll
     for (int s = 0; s < K; ++s)
@@ -1107,7 +1132,7 @@ __global__ void __launch_bounds__(1024) cluster_kernel(const GridArgs a)
   uint32_t* u0 = a.scratch + j0;
   uint32_t* v0 = a.scratch + nq + j0;
   int2* hist = reinterpret_cast<int2*>(a.scratch + 2 * (size_t)nq);
-  cluster_exchange_init(cs);
+  cluster_exchange_init(cs, a.wait_ns, blockIdx.x == a.withhold);
   uint32_t epoch = 0;
   run_pair<0, SYNC_CLUSTER>(a.limbs, a.pair, a.mods, a.L, j0, nloc, st, acc2, stg, rs, u0, v0, hist,
                             reinterpret_cast<GridSync*>(&cs), epoch, a.digits, a.count, a.iters, a.status, a.inv);
@@ -1166,14 +1191,11 @@ __global__ void __launch_bounds__(1024) cluster_batch_kernel(const BatchArgs a)
   uint32_t* scr = a.scratch + (size_t)(blockIdx.x / C) * a.scratch_words;
   cta_begin(a);
   uint32_t taken = 0, epoch = 0;
-  cluster_exchange_init(cs);
+  cluster_exchange_init(cs, a.wait_ns, blockIdx.x == a.withhold);
   for (;;) {
     if (r == 0 && threadIdx.x < C) {
       const uint32_t k = __shfl_sync(0xFFFFFFFFu >> (32 - C), threadIdx.x == 0 ? atomicAdd(a.queue, 1u) : 0u, 0);
-      const uint32_t ad = (uint32_t)__cvta_generic_to_shared(&next);
-      uint32_t ra;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(ad), "r"(threadIdx.x));
-      asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(ra), "r"(k) : "memory");
+      st_cluster_u32(&next, threadIdx.x, k);
     }
     cluster_sync_all();
     const uint32_t k = next;
@@ -1188,6 +1210,11 @@ __global__ void __launch_bounds__(1024) cluster_batch_kernel(const BatchArgs a)
                               reinterpret_cast<int2*>(scr + 2 * (size_t)d.nq), reinterpret_cast<GridSync*>(&cs), epoch,
                               a.digits, a.count + pi, a.iters + pi, a.status + pi, a.inv);
     cluster_sync_all();   // every CTA is done with `next` and with the pair's scratch
+    if (cs.dead != 0u) {  // a wait expired in some CTA (the same answer in all: the next exchange is
+      __syncthreads();    // behind another barrier): the exchange starts anew for the next pair
+      cluster_exchange_init(cs, a.wait_ns, blockIdx.x == a.withhold);
+      epoch = 0;
+    }
   }
   cluster_sync_all();     // no CTA leaves while others may still address its shared memory
   cta_end(a, taken);

@@ -35,7 +35,14 @@ struct RedSmem {
 struct ClusterSmem {
   unsigned long long key[2][MAX_CLUSTER];  // zero before use (cluster_exchange_init)
   unsigned long long bcast[2];             // the cluster-wide result, for the CTA's other warps
-  uint32_t dead;                           // a bounded wait expired: later exchanges fail at once
+  unsigned long long limit_ns;             // bound of every wait
+  unsigned long long since[4];             // per polling warp: the start of a wait that is not short
+  uint32_t meet;                           // number (from 1) of the next cluster barrier that every
+                                           // CTA of the cluster comes to
+  uint32_t dead;                           // a wait of some CTA expired: the barrier at which they meet
+  uint32_t failed;                         // an exchange of this CTA has failed
+  uint32_t lost;                           // the CTAs have met there (cluster_meet)
+  uint32_t withhold;                       // test hook: this CTA's keys reach no other CTA
 };
 
 // Cluster-grid mode: the global exchange state and, per CTA, the cluster's slots.
@@ -65,14 +72,27 @@ __device__ __forceinline__ void cluster_sync_all()
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Stores v at the same shared-memory offset as *local in CTA `rank` of this cluster.
-__device__ __forceinline__ void st_cluster_u64(unsigned long long* local, uint32_t rank, unsigned long long v)
+// The shared::cluster address of *local's offset in CTA `rank`, and stores to it.
+__device__ __forceinline__ uint32_t map_cluster(const void* local, uint32_t rank)
 {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
   uint32_t ra;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
-  asm volatile("st.shared::cluster.u64 [%0], %1;" :: "r"(ra), "l"(v) : "memory");
+  return ra;
 }
+
+__device__ __forceinline__ void st_cluster_u64(unsigned long long* local, uint32_t rank, unsigned long long v)
+{
+  asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" :: "r"(map_cluster(local, rank)), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ void st_cluster_u32(uint32_t* local, uint32_t rank, uint32_t v)
+{
+  asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" :: "r"(map_cluster(local, rank)), "r"(v) : "memory");
+}
+
+// Orders this thread's (and, after a __syncthreads, its CTA's) accesses for the cluster's CTAs.
+__device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 
 static __device__ __forceinline__ unsigned long long globaltimer_ns()
 {
@@ -173,8 +193,8 @@ __device__ __forceinline__ unsigned long long key_tag(uint32_t epoch)
   return (unsigned long long)(((epoch >> 1) + 1u) & 1u) << 63;
 }
 
-// A grid poll looks at the error flag and the clock once in POLL_CHECK polls: on every one,
-// they made the two hops of an exchange ~370 cycles longer.
+// A poll looks at the error flag and the clock once in POLL_CHECK polls: on every one, they
+// made the two hops of a grid exchange ~370 cycles longer.
 constexpr uint32_t POLL_CHECK = 256u;
 struct PollClock {
   uint32_t n = 0;
@@ -187,16 +207,38 @@ struct PollClock {
     return t - t0 > limit_ns;
   }
 };
-constexpr uint32_t CLUSTER_POLLS = 1u << 25;   // bound of a cluster poll: ~0.5 s of polls
 
-// Once per kernel, before the first exchange: every CTA's slots are zero when any CTA of the
-// cluster stores into them.
-__device__ __forceinline__ void cluster_exchange_init(ClusterSmem& cs)
+// Before the first exchange, and again after a failed one (with the exchange counts at zero):
+// every CTA's slots are zero when any CTA of the cluster stores into them.
+__device__ __forceinline__ void cluster_exchange_init(ClusterSmem& cs, unsigned long long limit_ns, bool withhold)
 {
   if (threadIdx.x < 2u * MAX_CLUSTER) (&cs.key[0][0])[threadIdx.x] = 0ull;
-  if (threadIdx.x == 0) cs.dead = 0u;
+  if (threadIdx.x == 0) {
+    cs.limit_ns = limit_ns;
+    cs.meet = 1u;
+    cs.dead = cs.failed = cs.lost = 0u;
+    cs.withhold = withhold;
+  }
   __syncthreads();
   cluster_sync_all();
+}
+
+// A cluster barrier in a kernel whose CTAs may come to different ones after an expired wait.
+// When a wait expires in some CTA, it stores the number of the next barrier into every CTA's
+// `dead` and goes straight to that barrier; the others come to the same one, by their own
+// path or because their next exchange fails, and all of them learn it there: false, and `lost`
+// is set.  (A number stored by a CTA that is already past this barrier is a later one, so all
+// CTAs answer alike; two expired waits between the same barriers store the same number.)
+__device__ __forceinline__ bool cluster_meet(ClusterSmem& cs)
+{
+  cluster_sync_all();
+  if (threadIdx.x == 0) {
+    const uint32_t n = cs.meet, dead = *reinterpret_cast<volatile uint32_t*>(&cs.dead);
+    cs.lost = dead != 0u && dead <= n;
+    cs.meet = n + 1u;
+  }
+  __syncthreads();
+  return cs.lost == 0u;
 }
 
 // Warp 0, with the CTA's minimum in every lane: lane c stores it, tagged with the exchange
@@ -205,31 +247,42 @@ __device__ __forceinline__ void cluster_exchange_init(ClusterSmem& cs)
 // exchanges ahead of another), which the tag tells apart, so there is neither a cluster
 // barrier nor a fence.  What bounds it is one DSMEM hop, ~450 cycles: with the CTA's own
 // reduction 725-783 cycles per exchange (2-16 CTAs of 256 or 512 threads) against 950-1,630
-// with stores and a cluster barrier (barrier.cluster, release and acquire).  False (sticky)
-// if a wait expired.
-__device__ __forceinline__ bool cluster_min_key(uint32_t& hi, uint32_t& lo, unsigned long long (&slots)[MAX_CLUSTER],
-                                                ClusterSmem& cs, unsigned long long tag)
+// with stores and a cluster barrier (barrier.cluster, release and acquire).  If the wait
+// expires here or in another CTA, cs.failed is set and the result is void: then every exchange
+// of the cluster fails, within one look at `dead`, until its next cluster_exchange_init.
+__device__ __forceinline__ void cluster_min_key(uint32_t& hi, uint32_t& lo, unsigned long long (&slots)[MAX_CLUSTER],
+                                                ClusterSmem& cs, unsigned long long tag, bool withhold)
 {
-  const uint32_t lane = threadIdx.x & 31u, nc = cluster_size();
-  if (lane < nc) st_cluster_u64(&slots[cluster_rank()], lane, tag | pack_key(hi, lo));
+  const uint32_t lane = threadIdx.x & 31u, nc = cluster_size(), me = cluster_rank();
+  if (lane < nc && (lane == me || !withhold)) st_cluster_u64(&slots[me], lane, tag | pack_key(hi, lo));
   const volatile unsigned long long* const mine = &slots[lane < nc ? lane : 0u];
-  bool ok = *reinterpret_cast<volatile uint32_t*>(&cs.dead) == 0u;
-  unsigned long long v = 0ull;
-  for (uint32_t n = 0; ok; ++n) {
+  unsigned long long v;
+  for (uint32_t n = 1;; ++n) {
     v = *mine;
     if (__all_sync(0xFFFFFFFFu, (v & KEY_TAG) == tag)) break;
-    if (n >= CLUSTER_POLLS) { cs.dead = 1u; ok = false; }
+    if (n % POLL_CHECK != 0u) continue;
+    volatile unsigned long long* const since = &cs.since[threadIdx.x >> 5];   // (no register on the chain)
+    const unsigned long long now = globaltimer_ns();
+    if (n == POLL_CHECK) *since = now;
+    __syncwarp();
+    const bool over = *reinterpret_cast<volatile uint32_t*>(&cs.dead) != 0u ||
+                      (long long)(now - *since) > (long long)cs.limit_ns;
+    if (!__any_sync(0xFFFFFFFFu, over)) continue;
+    if (lane < nc) st_cluster_u32(&cs.dead, lane, cs.meet);
+    cs.failed = 1u;
+    break;
   }
   unpack_key(v & ~KEY_TAG, hi, lo);
   warp_min_key(hi, lo);
-  return ok;
 }
 
 // Minimum over the CTA and, with several CTAs, over the cluster (cluster_min_key), the
 // cooperative grid (leader exchange over tagged slots) or the cluster grid (atomic minimum
 // and arrival counter per cluster leader); the grid protocols are described at GridSync.
 // Every wait is bounded; returns false if one expired (the pair then unwinds; the host sees
-// ST_TIMEOUT).  PUB: the exchange also publishes data written before it to every CTA.
+// ST_TIMEOUT).  PUB: the exchange also publishes data written before it to every CTA.  In a
+// cluster there is no other barrier between two exchanges of a pair, so that a CTA whose wait
+// expired can leave the pair at any of them (cluster_meet).
 template <int T, int MODE, bool PUB = false>
 __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& rs, uint32_t& parity,
                                            GridSync* gs, uint32_t& epoch)
@@ -241,7 +294,7 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
   if constexpr (MODE == SYNC_CLUSTER) {
     ClusterSmem& cs = *reinterpret_cast<ClusterSmem*>(gs);
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, cb = epoch & 1u;
-    if constexpr (PUB) cluster_sync_all();           // release / acquire in the cluster
+    const bool withhold = cs.withhold != 0u;         // (read off the chain)
     warp_min_key(hi, lo);
     if (lane == 0) rs.key[parity][w] = ((unsigned long long)hi << 32) | lo;
     __syncthreads();
@@ -250,7 +303,9 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
       hi = (uint32_t)(k >> 32);
       lo = (uint32_t)k;
       warp_min_key(hi, lo);
-      cluster_min_key(hi, lo, cs.key[cb], cs, key_tag(epoch));
+      if constexpr (PUB) fence_cluster();            // release / acquire in the cluster
+      cluster_min_key(hi, lo, cs.key[cb], cs, key_tag(epoch), withhold);
+      if constexpr (PUB) fence_cluster();
       if (lane == 0) cs.bcast[cb] = ((unsigned long long)hi << 32) | lo;
     }
     __syncthreads();
@@ -259,7 +314,7 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
     lo = (uint32_t)k;
     parity ^= 1u;
     epoch += 1u;
-    return cs.dead == 0u;
+    return cs.failed == 0u;
   }
   block_min_key<T>(hi, lo, rs, parity);
   if constexpr (MODE == SYNC_CGRID) {
@@ -300,10 +355,7 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
       bad = __shfl_sync(0xFFFFFFFFu, bad, 0);
       if (lane < nc) {
         st_cluster_u64(&cg.res[cb], lane, res);
-        const uint32_t ad = (uint32_t)__cvta_generic_to_shared(&cg.bad[cb]);
-        uint32_t ra;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(ad), "r"(lane));
-        asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(ra), "r"(bad) : "memory");
+        st_cluster_u32(&cg.bad[cb], lane, bad);
       }
     }
     cluster_sync_all();
@@ -1048,8 +1100,7 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
     __syncthreads();
     return;
   }
-  if constexpr (MODE == SYNC_CLUSTER) cluster_sync_all();   // publishes the (p, b) history
-  if constexpr (MODE == SYNC_GRID) {
+  if constexpr (MODE == SYNC_CLUSTER || MODE == SYNC_GRID) {
     // CTA 0's bookkeeping thread wrote the (p, b) history during the loop, whose exchanges
     // order nothing but the keys: one fenced exchange publishes it to every CTA.
     uint32_t h = 0xFFFFFFFFu, l = 0xFFFFFFFFu;
