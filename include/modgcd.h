@@ -126,7 +126,7 @@ int mgcd_batch_download(mgcd_context *ctx, uint32_t *g, const uint64_t *g_off, c
    reduction iteration): scale in [0.5, 1], 1 = the reference's count (default).  Every
    result is certified on the device (the surviving moduli must bound both operands); a pair
    that cannot be certified is rerun with the reference's count, so results do not change.
-   Single-pair calls always use the reference's count. */
+   Single-pair calls always use the reference's count.  Turns mgcd_set_spread off. */
 int mgcd_set_nq_scale(mgcd_context *ctx, float scale);
 /* Moduli grown on demand in batches (pairs of up to 16,384 moduli that run K per CTA):
    each pair starts its reduction loop with `start` times the reference's count (rounded up
@@ -138,13 +138,22 @@ int mgcd_set_nq_scale(mgcd_context *ctx, float scale);
    state it would have had from the start (residues of the operands, then the pivots so far
    replayed on it), so the result is the pair's gcd as before; the pivots after a growth may
    differ from a run with the larger set from the start.  A pair that still fails is rerun
-   with the reference's count.  A batch of at most half as many pairs as the GPU has SMs
-   runs them on clusters with the larger of the reference's count and the cap from the
-   start.  start in [0.1, 1] with step_permille in [10, 500], or
+   with the reference's count.  start in [0.1, 1] with step_permille in [10, 500], or
    start = 0 (off: the class fractions of mgcd_set_nq_scale apply).  Default 0.4, 50.
+   Turns mgcd_set_spread off.
    No counterpart in the reference (its count is fixed per call, GmpCudaDevice-gcd.cu:49-55). */
 int mgcd_set_growth(mgcd_context *ctx, float start, unsigned step_permille);
 int mgcd_get_growth(const mgcd_context *ctx, float *start, unsigned *step_permille);
+/* Batches of at most half as many pairs as the GPU has SMs (default on; not in a server):
+   each size class whose pairs fit the idle SMs runs them on thread-block clusters, in the
+   shape with the shortest iterations and with the larger of the reference's count and, where
+   sets grow, their cap from the start, in place of the class's shape, fraction and growth
+   (a loaded table's too; a table that puts one of the classes 0-2 on clusters keeps its
+   shapes).  The kernels record no phases for mgcd_batch_cta_trace.  Setting a class's shape,
+   a cluster size, a fraction or the growth turns this off, so that what is set is what runs;
+   a later call of this function decides again.  No counterpart in the reference. */
+int mgcd_set_spread(mgcd_context *ctx, int enable);
+int mgcd_get_spread(const mgcd_context *ctx, int *enabled);
 /* Launch shape of single pairs too large for one CTA (above 512 moduli):
      MGCD_SINGLE_AUTO              a thread-block cluster of up to 16 CTAs (pivot exchange
                                    through distributed shared memory) while the pair's
@@ -189,7 +198,7 @@ int mgcd_test_force_moduli(mgcd_context *ctx, unsigned nq);
    (class 3: one cluster) runs in lockstep, sharing one modular inverse per modulus and
    iteration (1, 2, 4, or 8 with threads = 512 outside class 3; a bucket whose k largest
    pairs would not fit one CTA's shared memory runs with fewer pairs per CTA); nq_scale as
-   above.  The autotuner writes these. */
+   above.  The autotuner writes these.  Turns mgcd_set_spread off, as the next two do. */
 #define MGCD_NUM_SIZE_CLASSES 4
 int mgcd_set_size_class(mgcd_context *ctx, int cls, int threads, int k, float nq_scale);
 int mgcd_get_size_class(const mgcd_context *ctx, int cls, int *threads, int *k, float *nq_scale);

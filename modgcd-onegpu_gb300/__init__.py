@@ -101,6 +101,8 @@ SIGNATURES = {
                                     _c.POINTER(_c.c_uint64), _c.POINTER(_c.c_uint64)]),
     "mgcd_serve_trace": (_c.c_int, [_P, _P, _c.c_size_t, _c.POINTER(_c.c_size_t)]),
     "mgcd_set_growth": (_c.c_int, [_P, _c.c_float, _c.c_uint]),
+    "mgcd_set_spread": (_c.c_int, [_P, _c.c_int]),
+    "mgcd_get_spread": (_c.c_int, [_P, _c.POINTER(_c.c_int)]),
     "mgcd_get_growth": (_c.c_int, [_P, _c.POINTER(_c.c_float), _c.POINTER(_c.c_uint)]),
     "mgcd_batch_pair_digits": (_c.c_int, [_P, _c.c_size_t, _P, _c.c_size_t, _c.POINTER(_c.c_size_t),
                                           _c.POINTER(_c.c_uint32)]),
@@ -346,6 +348,16 @@ class Device:
         st, pm = ctypes.c_float(), ctypes.c_uint()
         _check(self._lib.mgcd_get_growth(self._h, ctypes.byref(st), ctypes.byref(pm)))
         return st.value, pm.value
+
+    def set_spread(self, enable=True):
+        """Batches of few pairs on clusters (mgcd_set_spread; setting a shape, fraction or
+        growth turns it off)."""
+        _check(self._lib.mgcd_set_spread(self._h, int(bool(enable))))
+
+    def spread(self):
+        n = ctypes.c_int()
+        _check(self._lib.mgcd_get_spread(self._h, ctypes.byref(n)))
+        return bool(n.value)
 
     def batch_pair_digits(self, i):
         """Digits [(modulus, value), ...] of pair i of the last batch and its final moduli count."""

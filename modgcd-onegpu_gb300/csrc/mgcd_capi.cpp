@@ -585,8 +585,9 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
   // and its time is its longest pair's: each class, largest first, spreads its pairs over
   // clusters with its full count while SMs are left for the smaller classes.  61 mixed
   // pairs 24.2 -> 7.9 ms, 24 of 160-300 kbit 190.6 -> 140.0 ms.  Not in a server's waves, which
-  // share the GPU with the continuous lanes, nor where the table asks for clusters of its own.
-  bool spread = !plain && P.spread && subset.size() <= (size_t)c->sms / 2;
+  // share the GPU with the continuous lanes, nor where the caller has set shapes or counts
+  // (c->spread) or the table asks for clusters of its own.
+  bool spread = !plain && P.spread && c->spread && subset.size() <= (size_t)c->sms / 2;
   for (int b = 0; b < CLUSTER_CLASS; ++b) spread = spread && c->cfg[b].csize == 0;
   int sms_left = c->sms;
   for (int b = NSTREAMS - 1; b >= 0; --b) {  // largest class first: its pairs are the longest
@@ -1154,6 +1155,21 @@ int mgcd_set_nq_scale(mgcd_context* c, float scale)
 {
   if (!c || !(scale >= 0.5f && scale <= 1.0f)) return MGCD_ERR_INVALID_ARG;
   for (auto& b : c->cfg) b.nq_scale = scale;
+  c->spread = false;
+  return MGCD_OK;
+}
+
+int mgcd_set_spread(mgcd_context* c, int enable)
+{
+  if (!c) return MGCD_ERR_INVALID_ARG;
+  c->spread = enable != 0;
+  return MGCD_OK;
+}
+
+int mgcd_get_spread(const mgcd_context* c, int* enabled)
+{
+  if (!c || !enabled) return MGCD_ERR_INVALID_ARG;
+  *enabled = c->spread ? 1 : 0;
   return MGCD_OK;
 }
 
@@ -1167,6 +1183,7 @@ int mgcd_set_growth(mgcd_context* c, float start, unsigned step_permille)
   if (!c || !valid_growth(start, step_permille)) return MGCD_ERR_INVALID_ARG;
   c->grow_start = start;
   c->grow_permille = step_permille;
+  c->spread = false;
   return MGCD_OK;
 }
 
@@ -1194,6 +1211,7 @@ int mgcd_set_size_class(mgcd_context* c, int cls, int threads, int k, float nq_s
   c->cfg[cls].threads = threads;
   c->cfg[cls].k = k;
   c->cfg[cls].nq_scale = nq_scale;
+  c->spread = false;
   return MGCD_OK;
 }
 
@@ -1201,6 +1219,7 @@ int mgcd_set_cluster_size(mgcd_context* c, int ctas)
 {
   if (!c || ctas < 2 || ctas > MAX_CLUSTER) return MGCD_ERR_INVALID_ARG;
   c->cfg[CLUSTER_CLASS].csize = ctas;
+  c->spread = false;
   return MGCD_OK;
 }
 
@@ -1217,6 +1236,7 @@ int mgcd_set_class_cluster(mgcd_context* c, int cls, int ctas)
       (cls == CLUSTER_CLASS && ctas == 0))
     return MGCD_ERR_INVALID_ARG;
   c->cfg[cls].csize = ctas;
+  c->spread = false;
   return MGCD_OK;
 }
 

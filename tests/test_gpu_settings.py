@@ -1,0 +1,97 @@
+"""What a caller sets for batches is what runs, in batches of few pairs too: the shapes of the
+launches (occupancy trace: one record per CTA, phases for the K-slot CTAs), the moduli counts
+and reruns, with exact gcds."""
+import math
+import random
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _pairs(rng, bits):
+    out = []
+    for nb in bits:
+        g = rng.getrandbits(nb // 4) | 1
+        out.append((g * (rng.getrandbits(nb - nb // 4) | 1), g * (rng.getrandbits(nb // 2) | 1)))
+    return [p[0] for p in out], [p[1] for p in out]
+
+
+def _run(dev, us, vs):
+    """The size class's CTA counts, the K-slot CTAs among them, and the longest kernel's CTA size."""
+    dev.set_cta_trace(True)
+    assert dev.gcd_batch(us, vs) == [math.gcd(u, v) for u, v in zip(us, vs)]
+    rec = dev.batch_cta_trace()
+    dev.set_cta_trace(False)
+    ctas = [int((rec["size_class"] == c).sum()) for c in range(4)]
+    kslot = [int(((rec["size_class"] == c) & (rec["iterations"] > 0)).sum()) for c in range(4)]
+    return ctas, kslot, dev.batch_elapsed_ms()[2]
+
+
+@pytest.mark.parametrize("threads,k", [(256, 2), (512, 4), (512, 8), (1024, 2)])
+def test_class_shapes(mgcd, threads, k):
+    rng = random.Random(threads + k)
+    us, vs = _pairs(rng, [3000] * 16 + [12000] * 8 + [40000] * 3)
+    with mgcd.Device(0, 32) as dev:
+        assert dev.spread()
+        assert _run(dev, us, vs)[1] == [0, 0, 0, 0]          # on clusters
+        for c in (0, 1, 2):
+            dev.set_size_class(c, threads, k, 1.0)
+        assert not dev.spread()
+        ctas, kslot, longest = _run(dev, us, vs)
+        assert ctas == kslot == [-(-16 // k), -(-8 // k), -(-3 // k), 0] and longest == threads
+        dev.set_spread(True)
+        assert _run(dev, us, vs)[1] == [0, 0, 0, 0]
+        dev.set_spread(False)
+        assert _run(dev, us, vs)[1] == ctas
+
+
+@pytest.mark.parametrize("threads,k,ctas", [(512, 2, 8), (512, 4, 16), (1024, 1, 4), (256, 2, 2)])
+def test_cluster_class_shapes(mgcd, threads, k, ctas):
+    rng = random.Random(7 * threads + k)
+    us, vs = _pairs(rng, [200000] * 5 + [3000] * 6)
+    with mgcd.Device(0, 32) as dev:
+        dev.set_size_class(3, threads, k, 1.0)
+        dev.set_cluster_size(ctas)
+        n, kslot, longest = _run(dev, us, vs)
+        assert n[3] == ctas * -(-5 // k) and longest == threads
+        assert n[0] == kslot[0] > 0
+
+
+def test_fraction_and_growth(mgcd, oracle):
+    """A low fraction reruns the pairs it cannot hold; a pair's set grows from where it is set."""
+    rng = random.Random(3)
+    us, vs = _pairs(rng, [230000] * 3 + [20000] * 4)
+    us.append(rng.getrandbits(240000) | 1)                   # (almost surely) coprime
+    vs.append(rng.getrandbits(239000) | 1)
+    exp = [math.gcd(u, v) for u, v in zip(us, vs)]
+    with mgcd.Device(0, 32) as dev:
+        dev.set_size_class(3, 512, 2, 0.6)
+        dev.set_cluster_size(4)
+        assert dev.gcd_batch(us, vs) == exp
+        assert dev.batch_retried() > 0
+    with mgcd.Device(0, 32) as dev:
+        dev.set_growth(0.2, 20)
+        us, vs = us[3:7], vs[3:7]
+        assert dev.gcd_batch(us, vs) == exp[3:7]
+        for i, (u, v) in enumerate(zip(us, vs)):
+            a, b = max(u, v), min(u, v)
+            ref = oracle.num_moduli_needed(a.bit_length(), 32)
+            dig, n = dev.batch_pair_digits(i)
+            st, odig, _, on = oracle.modgcd_grow(a, b, 32, oracle.gen_moduli(32, 4096),
+                                                 oracle.grow_start_count(ref, 0.2), oracle.grow_cap(ref), 20)
+            if st != 0:                                      # rerun with the reference's count
+                st, odig, _, _ = oracle.modgcd(a, b, 32, oracle.gen_moduli(32, 4096), ref)
+                on = ref
+            assert st == 0 and (dig, n) == (odig, on)
+
+
+def test_loaded_table_keeps_the_switch(mgcd):
+    rng = random.Random(4)
+    us, vs = _pairs(rng, [5000] * 20)
+    with mgcd.Device(0, 27) as dev:
+        dev.load_tuning(mgcd.default_tuning_path(dev))
+        assert dev.spread() and _run(dev, us, vs)[1] == [0, 0, 0, 0]
+        dev.set_spread(False)
+        dev.load_tuning(mgcd.default_tuning_path(dev))
+        assert not dev.spread() and sum(_run(dev, us, vs)[1]) > 0
