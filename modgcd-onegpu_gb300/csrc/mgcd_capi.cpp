@@ -681,19 +681,21 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
           }
         }
       }
-      // Class 0 at the table's 256 x 2: its pairs live on a few warps, so what counts is how
+      // A shape that the caller has set is run as set; one of the defaults or of a table gives
+      // way for a long queue.  Class 0 at 256 x 2: its pairs live on a few warps, so what counts is how
       // many CTAs an SM holds to fill each other's barriers and serial steps.  From 16 pairs
       // per SM on, 128 threads (5,000 pairs of 1-8 kbit 5.93 -> 5.46 ms, 2,400 of 0.5-4 kbit even;
       // 1,000: 1.27 -> 1.36), and from 32 on four pairs per CTA while the sets are small (16,384
       // pairs of 0.5-4 kbit 8.92 -> 8.40, of 1-8 kbit 13.7 -> 14.5).
-      if (!plain && b == 0 && bk.threads == 256 && bk.k == 2 && v.size() >= 16 * (size_t)c->sms) {
+      const bool open = !plain && !c->shaped[b];
+      if (open && b == 0 && bk.threads == 256 && bk.k == 2 && v.size() >= 16 * (size_t)c->sms) {
         bk.threads = 128;
         if (v.size() >= 32 * (size_t)c->sms && bk.nq_max <= 1024) bk.k = 4;
       }
-      // The same for class 1 at the table's 512 x 2, whose shared memory lets three CTAs on an
+      // The same for class 1 at 512 x 2, whose shared memory lets three CTAs on an
       // SM: 256 threads from 8 pairs per SM on (12-40 kbit pairs, 27 bits: 3,000 of them 51.2
       // -> 47.6 ms, 1,600 28.6 -> 28.1, 800 16.5 -> 19.5).
-      if (!plain && b == 1 && bk.threads == 512 && bk.k == 2 && v.size() >= 8 * (size_t)c->sms) bk.threads = 256;
+      if (open && b == 1 && bk.threads == 512 && bk.k == 2 && v.size() >= 8 * (size_t)c->sms) bk.threads = 256;
       // fewer pairs per CTA when k of the bucket's largest pairs would not fit shared memory
       // (16 KB kept for the kernel's static shared memory)
       while (bk.k > 1 && batch_smem_bytes(bk.threads, bk.k, bk.nq_max) > c->smem_optin - 16384) bk.k /= 2;
@@ -1211,6 +1213,7 @@ int mgcd_set_size_class(mgcd_context* c, int cls, int threads, int k, float nq_s
   c->cfg[cls].threads = threads;
   c->cfg[cls].k = k;
   c->cfg[cls].nq_scale = nq_scale;
+  c->shaped[cls] = true;
   c->spread = false;
   return MGCD_OK;
 }
@@ -1285,6 +1288,7 @@ int mgcd_load_tuning(mgcd_context* c, const char* path)
   std::fclose(f);
   if (rc == MGCD_OK) {
     std::memcpy(c->cfg, cfg, sizeof(cfg));
+    for (bool& b : c->shaped) b = false;
     c->grow_start = g_start;
     c->grow_permille = g_step;
   }

@@ -157,6 +157,7 @@ struct mgcd_context {
   ClassCfg cfg[mgcd::NSTREAMS] = {{256, 2, 1.0f, 0}, {512, 2, 1.0f, 0}, {1024, 4, 1.0f, 0}, {1024, 1, 1.0f, 8}};
   bool spread = true;                  // small batches spread their pairs over clusters; off once the
                                        // caller sets a shape, fraction or growth (mgcd_set_spread)
+  bool shaped[mgcd::NSTREAMS] = {};    // classes whose shape the caller has set (mgcd_set_size_class)
   bool use_graph = false;
   int single_policy = MGCD_SINGLE_AUTO;  // launch shape of pairs that span several CTAs
   unsigned long long wait_timeout_ns = 2000000000ull;   // bound of every cross-CTA wait

@@ -95,3 +95,20 @@ def test_loaded_table_keeps_the_switch(mgcd):
         dev.set_spread(False)
         dev.load_tuning(mgcd.default_tuning_path(dev))
         assert not dev.spread() and sum(_run(dev, us, vs)[1]) > 0
+
+
+@pytest.mark.parametrize("cls,threads,n,bits", [(0, 256, 16, 400), (0, 256, 32, 300), (1, 512, 8, 9000)])
+def test_long_queues(mgcd, cls, threads, n, bits):
+    """n pairs per SM, the least at which a default shape gives way to smaller CTAs: one that
+    the caller has set, the same numbers even, does not."""
+    torch = pytest.importorskip("torch")
+    rng = random.Random(n + bits)
+    us, vs = _pairs(rng, [bits] * (n * torch.cuda.get_device_properties(0).multi_processor_count))
+    with mgcd.Device(0, 32) as dev:
+        assert dev.get_size_class(cls)[:2] == (threads, 2)
+        assert _run(dev, us, vs)[2] == threads // 2
+        dev.set_size_class(cls, threads, 2, 1.0)
+        assert _run(dev, us, vs)[2] == threads
+        dev.load_tuning(mgcd.default_tuning_path(dev))
+        assert dev.get_size_class(cls)[:2] == (threads, 2)
+        assert _run(dev, us, vs)[2] == threads // 2
