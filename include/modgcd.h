@@ -200,7 +200,8 @@ int mgcd_test_force_moduli(mgcd_context *ctx, unsigned nq);
    pairs would not fit one CTA's shared memory runs with fewer pairs per CTA); nq_scale as
    above.  The autotuner writes these.  A shape set here is run as set; one of the defaults
    or of a loaded table (512 x 2 of class 1, 256 x 2 of class 0) gives way to smaller CTAs
-   for long queues (8 or 16 pairs per SM and more).  Turns mgcd_set_spread off, as the next
+   for long queues (8 or 16 pairs per SM and more), or to four pairs per CTA (1,024 x 2 of
+   class 2, more than 2 pairs per SM).  Turns mgcd_set_spread off, as the next
    two do. */
 #define MGCD_NUM_SIZE_CLASSES 4
 int mgcd_set_size_class(mgcd_context *ctx, int cls, int threads, int k, float nq_scale);

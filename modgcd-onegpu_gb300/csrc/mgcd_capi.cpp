@@ -696,6 +696,12 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       // SM: 256 threads from 8 pairs per SM on (12-40 kbit pairs, 27 bits: 3,000 of them 51.2
       // -> 47.6 ms, 1,600 28.6 -> 28.1, 800 16.5 -> 19.5).
       if (open && b == 1 && bk.threads == 512 && bk.k == 2 && v.size() >= 8 * (size_t)c->sms) bk.threads = 256;
+      // Class 2 at 1,024 x 2: four pairs per CTA only once two fill every SM, since a CTA with
+      // four takes 1.6 times as long as one with two (40-kbit pairs, 32 bits: 304 of them 12.6 ms
+      // with two, 20.5 with four, 310 21.6 and 20.5, 620 34.0 and 30.9; 27 bits 11.7 and 19.7,
+      // 20.3 and 19.8, 31.8 and 30.0; mixed pairs of 1-64 kbit, 32 bits: 1,500 27.6 and 43.0, 4,096
+      // 70.9 and 57.9).
+      if (open && b == 2 && bk.threads == 1024 && bk.k == 2 && v.size() > 2 * (size_t)c->sms) bk.k = 4;
       // fewer pairs per CTA when k of the bucket's largest pairs would not fit shared memory
       // (16 KB kept for the kernel's static shared memory)
       while (bk.k > 1 && batch_smem_bytes(bk.threads, bk.k, bk.nq_max) > c->smem_optin - 16384) bk.k /= 2;

@@ -154,7 +154,7 @@ struct mgcd_context {
   // Per size class of the batched path: CTA size, pairs per CTA in lockstep, fraction of
   // the reference moduli count, CTAs per cluster (cluster class only).
   struct ClassCfg { int threads, k; float nq_scale; int csize; };
-  ClassCfg cfg[mgcd::NSTREAMS] = {{256, 2, 1.0f, 0}, {512, 2, 1.0f, 0}, {1024, 4, 1.0f, 0}, {1024, 1, 1.0f, 8}};
+  ClassCfg cfg[mgcd::NSTREAMS] = {{256, 2, 1.0f, 0}, {512, 2, 1.0f, 0}, {1024, 2, 1.0f, 0}, {1024, 1, 1.0f, 8}};
   bool spread = true;                  // small batches spread their pairs over clusters; off once the
                                        // caller sets a shape, fraction or growth (mgcd_set_spread)
   bool shaped[mgcd::NSTREAMS] = {};    // classes whose shape the caller has set (mgcd_set_size_class)

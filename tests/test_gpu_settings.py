@@ -112,3 +112,15 @@ def test_long_queues(mgcd, cls, threads, n, bits):
         dev.load_tuning(mgcd.default_tuning_path(dev))
         assert dev.get_size_class(cls)[:2] == (threads, 2)
         assert _run(dev, us, vs)[2] == threads // 2
+
+
+def test_class2_queues(mgcd):
+    """By default two pairs per CTA while they fit the SMs, four beyond."""
+    torch = pytest.importorskip("torch")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    us, vs = _pairs(random.Random(5), [40000] * (2 * sms + 1))
+    with mgcd.Device(0, 32) as dev:
+        assert _run(dev, us[:-1], vs[:-1])[0] == [0, 0, sms, 0]
+        assert _run(dev, us, vs)[0] == [0, 0, -(-(2 * sms + 1) // 4), 0]
+        dev.set_size_class(2, 1024, 4, 1.0)
+        assert _run(dev, us[:-1], vs[:-1])[0] == [0, 0, -(-2 * sms // 4), 0]
