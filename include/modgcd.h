@@ -175,7 +175,8 @@ int mgcd_set_single_pair_policy(mgcd_context *ctx, int policy);
 /* Bound of every wait for another CTA's key by a pair that spans several CTAs, on a cluster
    or a cooperative grid (default 2,000 ms).  When it runs out, every CTA leaves the pair and
    it fails with MGCD_ERR_TIMEOUT (in a batch, the pairs that share the cluster's slots; the
-   cluster goes on with the others); the context stays usable.  The allocation-free call
+   cluster goes on with the others); the context stays usable.  On a cluster the bound is a
+   number of polls that take about that long, at most a minute.  The allocation-free call
    waits 2,000 ms.  (The reference's grid barrier spins without a bound, GmpCuda.h:68-83.) */
 int mgcd_set_wait_timeout_ms(mgcd_context *ctx, unsigned ms);
 /* Test hook for the bounded waits: the CTA with block index `cta` of the next grid and

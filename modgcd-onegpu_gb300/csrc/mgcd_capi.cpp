@@ -765,7 +765,7 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
       P.trace_cls.insert(P.trace_cls.end(), n, bk.cls);
     }
     a.stage_fail = c->stage_fail_cta;
-    a.wait_ns = c->wait_timeout_ns;
+    a.wait_polls = cluster_wait_polls(c->wait_timeout_ns);
     a.withhold = c->withhold_cta;
     a.inv = InvTab{c->d_invtab.as<uint32_t>(), c->invtab_n};
     a.limbs = P.din<uint32_t>(0);
@@ -796,7 +796,7 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     const PairDesc& d = descs[k];
     GridArgs g;
     g.stage_fail = c->stage_fail_cta;
-    g.wait_ns = c->wait_timeout_ns;
+    g.wait_polls = cluster_wait_polls(c->wait_timeout_ns);
     g.withhold = c->withhold_cta;
     g.inv = InvTab{c->d_invtab.as<uint32_t>(), c->invtab_n};
     g.limbs = P.din<uint32_t>(0);

@@ -861,13 +861,12 @@ __device__ __forceinline__ bool cluster_min_keys(uint32_t (&kh)[K], uint32_t (&k
     warp_min_key(kh[s], kl[s]);
     if (lane == 0) ss.key[s][w] = ((unsigned long long)kh[s] << 32) | kl[s];
   }
-  const bool withhold = cs.withhold != 0u;
   __syncthreads();
   if (w < K) {
     const unsigned long long k = lane < T / 32 ? ss.key[w][lane] : ~0ull;
     uint32_t h = (uint32_t)(k >> 32), l = (uint32_t)k;
     warp_min_key(h, l);
-    cluster_min_key(h, l, ck.key[b][w], cs, key_tag(epoch), withhold);
+    cluster_min_key(h, l, ck.key[b][w], cs, key_tag(epoch));
     if (lane == 0) ck.res[b][w] = ((unsigned long long)h << 32) | l;
   }
   __syncthreads();
@@ -913,9 +912,10 @@ __global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
 
   // The exchanges and slots at the start, and again after an expired wait.
   auto start = [&]() {
-    kepoch = repoch = valid = active = 0u;
+    kepoch = valid = active = 0u;
+    repoch = blockIdx.x == a.withhold ? EPOCH_WITHHELD : 0u;
     for (uint32_t i = threadIdx.x; i < 2u * K * MAX_CLUSTER; i += T) (&ck.key[0][0][0])[i] = 0ull;
-    cluster_exchange_init(cs, a.wait_ns, blockIdx.x == a.withhold);
+    cluster_exchange_init(cs, a.wait_polls);
   };
   // Takes the next pair of the queue into slot s.  A CTA whose operands could not be staged
   // contributes the key (0, 0) (no modulus produces it), so the whole cluster answers that
@@ -1132,8 +1132,8 @@ __global__ void __launch_bounds__(1024) cluster_kernel(const GridArgs a)
   uint32_t* u0 = a.scratch + j0;
   uint32_t* v0 = a.scratch + nq + j0;
   int2* hist = reinterpret_cast<int2*>(a.scratch + 2 * (size_t)nq);
-  cluster_exchange_init(cs, a.wait_ns, blockIdx.x == a.withhold);
-  uint32_t epoch = 0;
+  cluster_exchange_init(cs, a.wait_polls);
+  uint32_t epoch = blockIdx.x == a.withhold ? EPOCH_WITHHELD : 0u;
   run_pair<0, SYNC_CLUSTER>(a.limbs, a.pair, a.mods, a.L, j0, nloc, st, acc2, stg, rs, u0, v0, hist,
                             reinterpret_cast<GridSync*>(&cs), epoch, a.digits, a.count, a.iters, a.status, a.inv);
   cluster_sync_all();   // no CTA leaves while others may still address its shared memory
@@ -1191,8 +1191,13 @@ __global__ void __launch_bounds__(1024) cluster_batch_kernel(const BatchArgs a)
   uint32_t* scr = a.scratch + (size_t)(blockIdx.x / C) * a.scratch_words;
   cta_begin(a);
   uint32_t taken = 0, epoch = 0;
-  cluster_exchange_init(cs, a.wait_ns, blockIdx.x == a.withhold);
+  bool fresh = true;
   for (;;) {
+    if (fresh) {          // the exchange starts, or starts anew after an expired wait
+      __syncthreads();
+      cluster_exchange_init(cs, a.wait_polls);
+      epoch = blockIdx.x == a.withhold ? EPOCH_WITHHELD : 0u;
+    }
     if (r == 0 && threadIdx.x < C) {
       const uint32_t k = __shfl_sync(0xFFFFFFFFu >> (32 - C), threadIdx.x == 0 ? atomicAdd(a.queue, 1u) : 0u, 0);
       st_cluster_u32(&next, threadIdx.x, k);
@@ -1210,11 +1215,7 @@ __global__ void __launch_bounds__(1024) cluster_batch_kernel(const BatchArgs a)
                               reinterpret_cast<int2*>(scr + 2 * (size_t)d.nq), reinterpret_cast<GridSync*>(&cs), epoch,
                               a.digits, a.count + pi, a.iters + pi, a.status + pi, a.inv);
     cluster_sync_all();   // every CTA is done with `next` and with the pair's scratch
-    if (cs.dead != 0u) {  // a wait expired in some CTA (the same answer in all: the next exchange is
-      __syncthreads();    // behind another barrier): the exchange starts anew for the next pair
-      cluster_exchange_init(cs, a.wait_ns, blockIdx.x == a.withhold);
-      epoch = 0;
-    }
+    fresh = cs.dead != 0u;   // the same in every CTA: the next exchange is behind another barrier
   }
   cluster_sync_all();     // no CTA leaves while others may still address its shared memory
   cta_end(a, taken);

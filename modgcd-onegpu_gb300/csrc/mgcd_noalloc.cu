@@ -46,7 +46,7 @@ constexpr uint32_t NA_PER_CTA = 256;           // moduli per CTA of a cluster: a
 static_assert(NA_MAX_NQ <= NA_PER_CTA * MAX_CLUSTER, "one cluster");
 constexpr int NA_L = 32;
 constexpr size_t NA_SCRATCH_WORDS = 4 * (size_t)NA_MAX_NQ;   // u0, v0, then (p, b) history
-constexpr unsigned long long NA_WAIT_NS = 2000000000ull;     // bound of the cluster's waits
+constexpr uint32_t NA_WAIT_POLLS = cluster_wait_polls(2000000000ull);   // bound of the cluster's waits
 constexpr int NA_MAX_DEVICES = 64;
 
 static __device__ __align__(256) uint32_t g_na_scratch[NA_SCRATCH_WORDS];
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(1024) noalloc_kernel(const NaArgs a)
     return;
   }
   constexpr uint32_t room = MODE == SYNC_CLUSTER ? NA_PER_CTA : NA_CTA_NQ;
-  if constexpr (MODE == SYNC_CLUSTER) cluster_exchange_init(cs, NA_WAIT_NS, false);
+  if constexpr (MODE == SYNC_CLUSTER) cluster_exchange_init(cs, NA_WAIT_POLLS);
   const uint32_t per = (d.nq + nc - 1) / nc, j0 = rank * per;   // per <= room
   const uint32_t nloc = j0 >= d.nq ? 0u : (d.nq - j0 < per ? d.nq - j0 : per);
   uint32_t* u0 = a.scratch + j0;

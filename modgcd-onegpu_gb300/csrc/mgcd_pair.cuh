@@ -35,14 +35,12 @@ struct RedSmem {
 struct ClusterSmem {
   unsigned long long key[2][MAX_CLUSTER];  // zero before use (cluster_exchange_init)
   unsigned long long bcast[2];             // the cluster-wide result, for the CTA's other warps
-  unsigned long long limit_ns;             // bound of every wait
-  unsigned long long since[4];             // per polling warp: the start of a wait that is not short
+  uint32_t limit;                          // bound of every wait, in polls
   uint32_t meet;                           // number (from 1) of the next cluster barrier that every
                                            // CTA of the cluster comes to
   uint32_t dead;                           // a wait of some CTA expired: the barrier at which they meet
   uint32_t failed;                         // an exchange of this CTA has failed
   uint32_t lost;                           // the CTAs have met there (cluster_meet)
-  uint32_t withhold;                       // test hook: this CTA's keys reach no other CTA
 };
 
 // Cluster-grid mode: the global exchange state and, per CTA, the cluster's slots.
@@ -193,8 +191,8 @@ __device__ __forceinline__ unsigned long long key_tag(uint32_t epoch)
   return (unsigned long long)(((epoch >> 1) + 1u) & 1u) << 63;
 }
 
-// A poll looks at the error flag and the clock once in POLL_CHECK polls: on every one, they
-// made the two hops of a grid exchange ~370 cycles longer.
+// A poll looks at the error flag and the clock or count once in POLL_CHECK polls: on every
+// one, they made the two hops of a grid exchange ~370 cycles longer.
 constexpr uint32_t POLL_CHECK = 256u;
 struct PollClock {
   uint32_t n = 0;
@@ -210,14 +208,13 @@ struct PollClock {
 
 // Before the first exchange, and again after a failed one (with the exchange counts at zero):
 // every CTA's slots are zero when any CTA of the cluster stores into them.
-__device__ __forceinline__ void cluster_exchange_init(ClusterSmem& cs, unsigned long long limit_ns, bool withhold)
+__device__ __forceinline__ void cluster_exchange_init(ClusterSmem& cs, uint32_t limit)
 {
   if (threadIdx.x < 2u * MAX_CLUSTER) (&cs.key[0][0])[threadIdx.x] = 0ull;
   if (threadIdx.x == 0) {
-    cs.limit_ns = limit_ns;
+    cs.limit = limit;
     cs.meet = 1u;
     cs.dead = cs.failed = cs.lost = 0u;
-    cs.withhold = withhold;
   }
   __syncthreads();
   cluster_sync_all();
@@ -251,22 +248,17 @@ __device__ __forceinline__ bool cluster_meet(ClusterSmem& cs)
 // expires here or in another CTA, cs.failed is set and the result is void: then every exchange
 // of the cluster fails, within one look at `dead`, until its next cluster_exchange_init.
 __device__ __forceinline__ void cluster_min_key(uint32_t& hi, uint32_t& lo, unsigned long long (&slots)[MAX_CLUSTER],
-                                                ClusterSmem& cs, unsigned long long tag, bool withhold)
+                                                ClusterSmem& cs, unsigned long long tag)
 {
-  const uint32_t lane = threadIdx.x & 31u, nc = cluster_size(), me = cluster_rank();
-  if (lane < nc && (lane == me || !withhold)) st_cluster_u64(&slots[me], lane, tag | pack_key(hi, lo));
+  const uint32_t lane = threadIdx.x & 31u, nc = cluster_size();
+  if (lane < nc) st_cluster_u64(&slots[cluster_rank()], lane, tag | pack_key(hi, lo));
   const volatile unsigned long long* const mine = &slots[lane < nc ? lane : 0u];
   unsigned long long v;
   for (uint32_t n = 1;; ++n) {
     v = *mine;
     if (__all_sync(0xFFFFFFFFu, (v & KEY_TAG) == tag)) break;
     if (n % POLL_CHECK != 0u) continue;
-    volatile unsigned long long* const since = &cs.since[threadIdx.x >> 5];   // (no register on the chain)
-    const unsigned long long now = globaltimer_ns();
-    if (n == POLL_CHECK) *since = now;
-    __syncwarp();
-    const bool over = *reinterpret_cast<volatile uint32_t*>(&cs.dead) != 0u ||
-                      (long long)(now - *since) > (long long)cs.limit_ns;
+    const bool over = *reinterpret_cast<volatile uint32_t*>(&cs.dead) != 0u || n >= cs.limit;
     if (!__any_sync(0xFFFFFFFFu, over)) continue;
     if (lane < nc) st_cluster_u32(&cs.dead, lane, cs.meet);
     cs.failed = 1u;
@@ -294,7 +286,6 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
   if constexpr (MODE == SYNC_CLUSTER) {
     ClusterSmem& cs = *reinterpret_cast<ClusterSmem*>(gs);
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, cb = epoch & 1u;
-    const bool withhold = cs.withhold != 0u;         // (read off the chain)
     warp_min_key(hi, lo);
     if (lane == 0) rs.key[parity][w] = ((unsigned long long)hi << 32) | lo;
     __syncthreads();
@@ -304,7 +295,7 @@ __device__ __forceinline__ bool reduce_min(uint32_t& hi, uint32_t& lo, RedSmem& 
       lo = (uint32_t)k;
       warp_min_key(hi, lo);
       if constexpr (PUB) fence_cluster();            // release / acquire in the cluster
-      cluster_min_key(hi, lo, cs.key[cb], cs, key_tag(epoch), withhold);
+      cluster_min_key(hi, lo, cs.key[cb], cs, key_tag(epoch));
       if constexpr (PUB) fence_cluster();
       if (lane == 0) cs.bcast[cb] = ((unsigned long long)hi << 32) | lo;
     }
