@@ -501,8 +501,9 @@ static int single_threads(uint32_t per) { return (int)std::min<uint32_t>(1024, (
 // pairs per cluster within `budget` SMs, or {0, 0} to keep the class's K pairs per CTA.  The
 // pairs' loops then bound the batch, so the shape is the one with the shortest iterations,
 // by what they measured: a chunk of 32 moduli takes its SMSP 230 cycles for the shared inverse
-// and 60 per slot, at least a chain of ~1,500 cycles, and the exchange 900 and 150 per slot;
-// clusters that do not fit at once run one after another.
+// and 60 per slot, 564 with four slots (with 470, 76 pairs of 40 kbit took 4 CTAs x 4, 18.3 ms at
+// 32 bits and 16.5 at 27, instead of 2 x 1, 10.3 and 9.7), at least a chain of ~1,500 cycles,
+// and the exchange 900 and 150 per slot; clusters that do not fit at once run one after another.
 struct SmallShape { int cs, k; };
 static SmallShape small_batch_shape(const mgcd_context* c, size_t n, uint32_t nq_max, int budget, bool clusters_only)
 {
@@ -522,7 +523,7 @@ static SmallShape small_batch_shape(const mgcd_context* c, size_t n, uint32_t nq
       nc = std::min(nc, budget / cs);
       if (nc < 1 || (!clusters_only && (size_t)nc < need)) continue;
       const double waves = (double)((need + nc - 1) / nc);
-      const double update = std::max(1500.0, std::ceil(((per + 31) / 32) / 4.0) * (230.0 + 60.0 * k));
+      const double update = std::max(1500.0, std::ceil(((per + 31) / 32) / 4.0) * (k == 4 ? 564.0 : 230.0 + 60.0 * k));
       const double cost = waves * (update + 900.0 + 150.0 * k);
       if (cost < best_cost) { best_cost = cost; best = {cs, k}; }
     }

@@ -124,3 +124,14 @@ def test_class2_queues(mgcd):
         assert _run(dev, us, vs)[0] == [0, 0, -(-(2 * sms + 1) // 4), 0]
         dev.set_size_class(2, 1024, 4, 1.0)
         assert _run(dev, us[:-1], vs[:-1])[0] == [0, 0, -(-2 * sms // 4), 0]
+
+
+@pytest.mark.parametrize("L", [27, 32])
+def test_small_batch_of_equal_pairs(mgcd, L):
+    """Half as many pairs as SMs: clusters of two CTAs, one pair each, rather than larger
+    clusters with several pairs."""
+    torch = pytest.importorskip("torch")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    us, vs = _pairs(random.Random(6), [40000] * (sms // 2))
+    with mgcd.Device(0, L) as dev:
+        assert _run(dev, us, vs)[0] == [0, 0, sms // 2 * 2, 0]
