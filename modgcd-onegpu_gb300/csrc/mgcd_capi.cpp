@@ -497,17 +497,17 @@ int mgcd::plan_batch(mgcd_context* c, Plan& P, size_t np, const uint32_t* limbs,
 // warp more for the pair's bookkeeping (run_pair), while they fit.
 static int single_threads(uint32_t per) { return (int)std::min<uint32_t>(1024, (per + 31) / 32 * 32 + 32); }
 
-// Launch shape of a class's n pairs in a batch too small to fill the GPU: CTAs per cluster and
-// pairs per cluster within `budget` SMs, or {0, 0} to keep the class's K pairs per CTA.  The
+// Launch shape of a class's n pairs in a batch too small to fill the GPU: CTAs per cluster, pairs
+// per cluster and clusters within `budget` SMs, or {} to keep the class's K pairs per CTA.  The
 // pairs' loops then bound the batch, so the shape is the one with the shortest iterations,
 // by what they measured: a chunk of 32 moduli takes its SMSP 230 cycles for the shared inverse
 // and 60 per slot, 564 with four slots (with 470, 76 pairs of 40 kbit took 4 CTAs x 4, 18.3 ms at
 // 32 bits and 16.5 at 27, instead of 2 x 1, 10.3 and 9.7), at least a chain of ~1,500 cycles,
 // and the exchange 900 and 150 per slot; clusters that do not fit at once run one after another.
-struct SmallShape { int cs, k; };
+struct SmallShape { int cs = 0, k = 0, clusters = 0; };
 static SmallShape small_batch_shape(const mgcd_context* c, size_t n, uint32_t nq_max, int budget, bool clusters_only)
 {
-  SmallShape best{0, 0};
+  SmallShape best;
   double best_cost = 1e30;
   for (int cs = 2; cs <= MAX_CLUSTER; cs *= 2) {
     const uint32_t per = (nq_max + cs - 1) / cs;
@@ -525,7 +525,7 @@ static SmallShape small_batch_shape(const mgcd_context* c, size_t n, uint32_t nq
       const double waves = (double)((need + nc - 1) / nc);
       const double update = std::max(1500.0, std::ceil(((per + 31) / 32) / 4.0) * (k == 4 ? 564.0 : 230.0 + 60.0 * k));
       const double cost = waves * (update + 900.0 + 150.0 * k);
-      if (cost < best_cost) { best_cost = cost; best = {cs, k}; }
+      if (cost < best_cost) { best_cost = cost; best = {cs, k, (int)std::min<size_t>(need, (size_t)nc)}; }
     }
   }
   return best;
@@ -594,7 +594,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
   for (int b = NSTREAMS - 1; b >= 0; --b) {  // largest class first: its pairs are the longest
     auto& v = byb[b];
     if (v.empty()) continue;
-    SmallShape few{0, 0};
+    SmallShape few;
     if (spread) {
       // the count a grown set may reach, where sets grow: what K pairs per CTA would certify
       // in the end is certified here too
@@ -638,10 +638,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       const uint32_t per = (bk.nq_max + few.cs - 1) / few.cs;
       bk.threads = few.k == 1 ? single_threads(per) : per <= 256 ? 256 : per <= 512 ? 512 : 1024;
       bk.smem = cluster_batch_smem_bytes(few.cs, bk.nq_max, few.k);
-      int nc = 0;
-      if (cluster_batch_max_clusters(bk.threads, bk.k, c->L <= 30, bk.csize, bk.smem, &nc) != cudaSuccess || nc < 1)
-        return MGCD_ERR_GRID;
-      bk.grid = (int)std::min<size_t>((v.size() + bk.k - 1) / bk.k, (size_t)nc);
+      bk.grid = few.clusters;
       scratch += (size_t)bk.grid * 4 * bk.k * bk.nq_max;
       sms_left -= bk.grid * bk.csize;
     } else if (!plain && (b == CLUSTER_CLASS || c->cfg[b].csize > 0 || small_cs > 0)) {

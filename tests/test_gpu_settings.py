@@ -135,3 +135,13 @@ def test_small_batch_of_equal_pairs(mgcd, L):
     us, vs = _pairs(random.Random(6), [40000] * (sms // 2))
     with mgcd.Device(0, L) as dev:
         assert _run(dev, us, vs)[0] == [0, 0, sms // 2 * 2, 0]
+
+
+@pytest.mark.parametrize("bits", [[200000] * 30 + [16000] * 46, [200000] * 3 + [64000] * 40 + [3000] * 30,
+                                  [64000] * 50 + [16000] * 20])
+def test_small_batch_fits_the_sms(mgcd, bits):
+    """The classes of a small batch share the SMs: no more CTAs than SMs."""
+    torch = pytest.importorskip("torch")
+    us, vs = _pairs(random.Random(7), bits)
+    with mgcd.Device(0, 27) as dev:
+        assert sum(_run(dev, us, vs)[0]) <= torch.cuda.get_device_properties(0).multi_processor_count
