@@ -214,38 +214,6 @@ size_t mgcd_gen_moduli(int L, uint32_t* out, size_t count) { return gen_moduli(L
 
 int mgcd_moduli_needed(int L, size_t bits) { return moduli_needed(L, bits); }
 
-// Where the lines of the cooperative grid's exchange live: a line's home is on one of the
-// GPU's two dies, and an exchange whose leader (CTA 0) polls lines of its own die takes 2,600
-// cycles at 152 CTAs, of the other die 3,150.  The home changes every few pages, so the same
-// exchange is timed at GSYNC_PLACES places (~1 ms in all) and the fastest kept; any place is
-// correct.
-static int calibrate_exchange(mgcd_context* c, cudaStream_t s)
-{
-  if (c->d_xchg.grow(GSYNC_PLACES * GSYNC_STRIDE, c->pool, s) != cudaSuccess) return MGCD_ERR_CUDA;
-  char* const base = c->d_xchg.as<char>();
-  c->gsync = reinterpret_cast<GridSync*>(base);
-  DevBuf t;
-  if (t.grow(GSYNC_PLACES * sizeof(unsigned long long), c->pool, s) != cudaSuccess) return MGCD_ERR_CUDA;
-  unsigned long long h[GSYNC_PLACES];
-  bool ok = cudaMemsetAsync(t.p, 0xFF, sizeof h, s) == cudaSuccess;
-  for (size_t i = 0; ok && i < GSYNC_PLACES; ++i) {
-    GridSync* g = reinterpret_cast<GridSync*>(base + i * GSYNC_STRIDE);
-    ok = launch_gridsync_init(g, c->wait_timeout_ns, 0xFFFFFFFFu, s) == cudaSuccess;
-    // a GPU shared with other work may refuse the co-resident grid: then the first place stays
-    if (ok && launch_exchange_probe(g, c->sms, 40, t.as<unsigned long long>() + i, s) != cudaSuccess) {
-      cudaGetLastError();
-      break;
-    }
-  }
-  ok = ok && cudaMemcpyAsync(h, t.p, sizeof h, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-       cudaStreamSynchronize(s) == cudaSuccess;
-  t.release(s);
-  if (!ok) return MGCD_ERR_CUDA;
-  const size_t best = (size_t)(std::min_element(h, h + GSYNC_PLACES) - h);
-  c->gsync = reinterpret_cast<GridSync*>(base + best * GSYNC_STRIDE);
-  return MGCD_OK;
-}
-
 int mgcd_create(int device, int L, mgcd_context** out)
 {
   if (!out || (L != 22 && L != 27 && L != 32)) return MGCD_ERR_INVALID_ARG;
@@ -308,7 +276,7 @@ int mgcd_create(int device, int L, mgcd_context** out)
                             cudaSuccess ||
                         cudaStreamSynchronize(s) != cudaSuccess))
     rc = MGCD_ERR_CUDA;
-  if (rc == MGCD_OK) rc = calibrate_exchange(c, s);
+  if (rc == MGCD_OK && c->d_xchg.grow(GSYNC_PLACES * GSYNC_STRIDE, c->pool, s) != cudaSuccess) rc = MGCD_ERR_CUDA;
   if (rc != MGCD_OK) {
     mgcd_destroy(c);
     return rc;
@@ -720,6 +688,12 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
   return MGCD_OK;
 }
 
+// Of the single pairs too large for one CTA: on a cooperative grid, not on a cluster.
+static bool on_grid(const mgcd_context* c, uint32_t nq)
+{
+  return c->single_policy == MGCD_SINGLE_REFERENCE_SHAPE || nq > (uint32_t)MAX_CLUSTER * 1024;
+}
+
 // Launches the buckets (one stream each, joined back into P.stream) and then the
 // single-pair launches.  `pairs` is the descriptor array on the device, `queue_base` the
 // first of the bucket work counters (zeroed by the caller).
@@ -807,7 +781,7 @@ static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& bucke
     g.iters = P.dres<uint32_t>(P.res.iters) + k;
     g.status = P.dres<int32_t>(P.res.status) + k;
     const bool ref_shape = c->single_policy == MGCD_SINGLE_REFERENCE_SHAPE;
-    if (!ref_shape && d.nq <= (uint32_t)MAX_CLUSTER * 1024) {
+    if (!on_grid(c, d.nq)) {
       // thread-block cluster while one modulus per thread fits 16 CTAs: its exchange takes a
       // third of the grid's, which outweighs the fuller CTAs (32-bit moduli, cluster / grid:
       // 9,472 moduli 12.4 / 17.2 ms, 13,312 20.7 / 24.9, 15,872 27.0 / 29.7; with two moduli
@@ -891,6 +865,39 @@ static int reset_results(Plan& P)
   return MGCD_OK;
 }
 
+// Where the lines of the cooperative grid's exchange live: a line's home is on one of the
+// GPU's two dies, and an exchange whose leader (CTA 0) polls lines of its own die takes 2,600
+// cycles at 152 CTAs, of the other die 3,150.  The home changes every few pages, so the same
+// exchange is timed at GSYNC_PLACES places twice (1.4 ms in all) and the fastest kept; any place is
+// correct.  Done at the context's first pair on a grid, which needs the SMs for itself anyway:
+// at creation the CTAs would wait for whatever else holds SMs, and time an exchange beside it.
+static int calibrate_exchange(mgcd_context* c, cudaStream_t s)
+{
+  char* const base = c->d_xchg.as<char>();
+  c->gsync = reinterpret_cast<GridSync*>(base);
+  DevBuf t;
+  constexpr size_t TRIES = 2 * GSYNC_PLACES;          // every place twice, the better time counts
+  if (t.grow(TRIES * sizeof(unsigned long long), c->pool, s) != cudaSuccess) return MGCD_ERR_CUDA;
+  unsigned long long h[TRIES];
+  bool ok = cudaMemsetAsync(t.p, 0xFF, sizeof h, s) == cudaSuccess;
+  for (size_t i = 0; ok && i < TRIES; ++i) {
+    GridSync* g = reinterpret_cast<GridSync*>(base + i % GSYNC_PLACES * GSYNC_STRIDE);
+    ok = launch_gridsync_init(g, c->wait_timeout_ns, 0xFFFFFFFFu, s) == cudaSuccess;
+    // a grid that cannot be co-resident at all: the first place stays
+    if (ok && launch_exchange_probe(g, c->sms, 24, t.as<unsigned long long>() + i, s) != cudaSuccess) {
+      cudaGetLastError();
+      break;
+    }
+  }
+  ok = ok && cudaMemcpyAsync(h, t.p, sizeof h, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+       cudaStreamSynchronize(s) == cudaSuccess;
+  t.release(s);
+  if (!ok) return MGCD_ERR_CUDA;
+  const size_t best = (size_t)(std::min_element(h, h + TRIES) - h) % GSYNC_PLACES;
+  c->gsync = reinterpret_cast<GridSync*>(base + best * GSYNC_STRIDE);
+  return MGCD_OK;
+}
+
 int mgcd::run_plan(mgcd_context* c, Plan& P)
 {
   if (!c) return MGCD_ERR_INVALID_ARG;
@@ -904,6 +911,11 @@ int mgcd::run_plan(mgcd_context* c, Plan& P)
     return MGCD_OK;
   }
   for (size_t k = 0; k < ng; ++k) P.eff_nq[k] = P.descs[k].nq;
+  for (uint32_t k : P.grid_pairs)
+    if (c->gsync == nullptr && on_grid(c, P.descs[k].nq)) {
+      const int rc = calibrate_exchange(c, P.stream);
+      if (rc != MGCD_OK) return rc;
+    }
   if (c->use_graph && P.graphable && !P.plain) {
     if (!P.graph) {
       // Record the run once (the results' reset, the chained bucket kernels, the

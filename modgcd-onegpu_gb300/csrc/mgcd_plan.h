@@ -147,7 +147,7 @@ struct mgcd_context {
   mgcd::DevBuf d_invtab;               // pairwise inverse table (InvTab)
   uint32_t invtab_n = 0;
   mgcd::DevBuf d_xchg;                 // GSYNC_PLACES places for the grid exchange's lines
-  mgcd::GridSync* gsync = nullptr;     // the fastest of them (calibrate_exchange)
+  mgcd::GridSync* gsync = nullptr;     // the fastest of them (calibrate_exchange), from the first grid pair on
   mgcd::Plan main;                     // the plan of the context's own calls
   bool serving = false;                // a request server runs on this context
 
