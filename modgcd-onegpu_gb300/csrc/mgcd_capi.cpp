@@ -486,7 +486,7 @@ static SmallShape small_batch_shape(const mgcd_context* c, size_t n, uint32_t nq
       const size_t smem = cluster_batch_smem_bytes(cs, nq_max, k);
       int nc = 0;
       if (smem > c->smem_optin - 24576 ||
-          cluster_batch_max_clusters(threads, k, c->L <= 30, cs, smem, &nc) != cudaSuccess || nc < 1)
+          cluster_batch_max_clusters(threads, k, c->L <= NARROW_MAX_L, cs, smem, &nc) != cudaSuccess || nc < 1)
         continue;
       nc = std::min(nc, budget / cs);
       if (nc < 1 || (!clusters_only && (size_t)nc < need)) continue;
@@ -528,7 +528,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
     bk.csize = cs;
     bk.smem = cluster_batch_smem_bytes(cs, bk.nq_max, 1);
     int nc = 0;
-    if (bk.smem > room || cluster_batch_max_clusters(bk.threads, 1, c->L <= 30, cs, bk.smem, &nc) != cudaSuccess || nc < 1)
+    if (bk.smem > room || cluster_batch_max_clusters(bk.threads, 1, c->L <= NARROW_MAX_L, cs, bk.smem, &nc) != cudaSuccess || nc < 1)
       return MGCD_ERR_GRID;
     bk.grid = (int)std::min<size_t>(v.size(), (size_t)nc);
     scratch += (size_t)bk.grid * 4 * bk.nq_max;
@@ -622,7 +622,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       bk.csize = cs;
       bk.smem = cluster_batch_smem_bytes(cs, bk.nq_max, bk.k);
       int nc = 0;
-      if (bk.smem > room || cluster_batch_max_clusters(bk.threads, bk.k, c->L <= 30, cs, bk.smem, &nc) != cudaSuccess || nc < 1)
+      if (bk.smem > room || cluster_batch_max_clusters(bk.threads, bk.k, c->L <= NARROW_MAX_L, cs, bk.smem, &nc) != cudaSuccess || nc < 1)
         return MGCD_ERR_GRID;
       bk.grid = (int)std::min<size_t>((v.size() + bk.k - 1) / bk.k, (size_t)nc);
       scratch += (size_t)bk.grid * 4 * bk.k * bk.nq_max;
@@ -673,7 +673,7 @@ static int schedule(mgcd_context* c, Plan& P, std::vector<PairDesc>& descs, cons
       while (bk.k > 1 && batch_smem_bytes(bk.threads, bk.k, bk.nq_max) > c->smem_optin - 16384) bk.k /= 2;
       bk.smem = batch_smem_bytes(bk.threads, bk.k, bk.nq_max);
       int bps = 0;
-      if (batch_max_blocks_per_sm(bk.threads, bk.k, c->L <= 30, bk.smem, &bps) != cudaSuccess || bps < 1)
+      if (batch_max_blocks_per_sm(bk.threads, bk.k, c->L <= NARROW_MAX_L, bk.smem, &bps) != cudaSuccess || bps < 1)
         return MGCD_ERR_GRID;
       bk.grid = (int)std::min<size_t>((v.size() + bk.k - 1) / bk.k, (size_t)c->sms * bps);
       scratch += (size_t)bk.grid * batch_scratch_words(bk.k, bk.nq_max);

@@ -333,7 +333,7 @@ __device__ __forceinline__ void t_key_min(uint32_t t, uint32_t q, uint32_t& kh, 
 // gives INF, INF gives 0) are settled behind one vote, and keys are kept without a branch.
 // 2,400 positions, four slots, half of them live, 1,024 threads: 12,485 -> 10,800 cycles
 // against computing every slot in every warp, with the same inverse.
-//   NARROW  moduli below 2^30.  Every modulus of a width-L table is an L-bit prime, so
+//   NARROW  moduli of at most NARROW_MAX_L bits.  Every modulus of a width-L table is an L-bit prime, so
 //           |b| <= p / 2 < q puts t - b in (-q, 2q): one conditional add of q makes it lazy,
 //           0 mod q exactly at 0 and q.  A pivot p < 2^32 enters a product as it is either
 //           way (p y < q 2^32 for a canonical y; p < 2q, y < 2q when lazy).

@@ -24,6 +24,10 @@ struct PairDesc {
                      // count; <= nq: no growth)
 };
 
+// Widest moduli whose products are kept lazily reduced and whose residues take four limbs a
+// step (horner_tile, which sets the limit; lazy products alone would allow 30 bits).
+constexpr int NARROW_MAX_L = 29;
+
 // Largest moduli count of a pair that runs on one CTA (size classes 0-2).
 constexpr uint32_t CTA_MAX_NQ = 16384;
 
@@ -161,8 +165,8 @@ constexpr uint32_t EPOCH_WITHHELD = 2u;
 
 // Launch helpers (mgcd_kernels.cu).
 // k = pairs per CTA run in lockstep (1: batch_kernel; 2, 4: batchk_kernel).  Scratch per
-// CTA: batch_scratch_words(k, nq_max).  Moduli below 2^30 (a.L <= 30; `narrow` for the occupancy
-// query) select the kernels with lazily reduced Montgomery products.
+// CTA: batch_scratch_words(k, nq_max).  Moduli of at most NARROW_MAX_L bits (`narrow` for the
+// occupancy query) select the kernels with lazily reduced Montgomery products.
 size_t batch_smem_bytes(int threads, int k, uint32_t nq_max);
 size_t batch_scratch_words(int k, uint32_t nq_max);
 cudaError_t batch_max_blocks_per_sm(int threads, int k, bool narrow, size_t smem, int* blocks);

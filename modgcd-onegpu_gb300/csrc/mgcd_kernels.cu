@@ -271,7 +271,7 @@ __device__ __forceinline__ uint32_t grow_step_for(uint32_t cap, uint32_t permill
 // and a newly loaded pair's states, computed in modulus order, are taken in by the next
 // re-layout (`fresh`).
 //
-// NARROW: moduli below 2^30 (widths up to 30 bits), lazily reduced Montgomery products.
+// NARROW: moduli of at most NARROW_MAX_L bits, lazily reduced Montgomery products.
 // RING: continuous serving -- pairs come from a.ring instead of the batch queue, empty
 // slots take newly published entries while the others run, and a CTA whose slots stay
 // empty for a.idle_ns leaves.
@@ -879,7 +879,7 @@ __device__ __forceinline__ bool cluster_min_keys(uint32_t (&kh)[K], uint32_t (&k
   return cs.failed == 0u;
 }
 
-// NARROW: moduli below 2^30, as in batchk_kernel.
+// NARROW: as in batchk_kernel.
 template <int T, int K, bool NARROW>
 __global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
 {
@@ -952,8 +952,8 @@ __global__ void __launch_bounds__(T, 1) cluster_batchk_kernel(const BatchArgs a)
       uint32_t* ts = tS + (size_t)s * per;
       uint32_t* u0 = scr + (size_t)s * 4 * NQS;
       const ModConst* my = a.mods + j0;
-      const bool staged = residues<T>(a.limbs + d.u_off, d.u_len, my, nloc, ts, stg, L <= 30);
-      const bool ok = residues<T>(a.limbs + d.v_off, d.v_len, my, nloc, acc2, stg, L <= 30) && staged;
+      const bool staged = residues<T>(a.limbs + d.u_off, d.u_len, my, nloc, ts, stg, L <= NARROW_MAX_L);
+      const bool ok = residues<T>(a.limbs + d.v_off, d.v_len, my, nloc, acc2, stg, L <= NARROW_MAX_L) && staged;
       h0 = 0xFFFFFFFFu;
       l0 = 0xFFFFFFFFu;
       for (uint32_t j = threadIdx.x; j < nloc; j += T) {
@@ -1350,7 +1350,7 @@ static const void* batchk_fn_for(int threads, int k)
   return nullptr;
 }
 
-// narrow: the context's moduli are below 2^30 (width <= 30)
+// narrow: the context's moduli are narrow (NARROW_MAX_L)
 static const void* batch_fn_for(int threads, int k, bool narrow)
 {
   if (k == 1) return reinterpret_cast<const void*>(&batch_kernel);
@@ -1385,7 +1385,7 @@ static const void* ring_fn_for(int threads, int k, bool narrow)
 
 cudaError_t launch_ring(const BatchArgs& a, int threads, int k, int grid, size_t smem, cudaStream_t s)
 {
-  const void* fn = ring_fn_for(threads, k, a.L <= 30);
+  const void* fn = ring_fn_for(threads, k, a.L <= NARROW_MAX_L);
   if (!fn || !a.ring) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -1395,7 +1395,7 @@ cudaError_t launch_ring(const BatchArgs& a, int threads, int k, int grid, size_t
 
 cudaError_t launch_batch(const BatchArgs& a, int threads, int k, int grid, size_t smem, cudaStream_t s, bool after)
 {
-  const void* fn = batch_fn_for(threads, k, a.L <= 30);
+  const void* fn = batch_fn_for(threads, k, a.L <= NARROW_MAX_L);
   if (!fn) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -1460,7 +1460,7 @@ static const void* cluster_batchk_fn_for(int threads, int k)
   return nullptr;
 }
 
-// narrow: the context's moduli are below 2^30 (width <= 30)
+// narrow: the context's moduli are narrow (NARROW_MAX_L)
 static const void* cluster_batch_fn_for(int threads, int k, bool narrow)
 {
   if (k == 1) return reinterpret_cast<const void*>(&cluster_batch_kernel);
@@ -1497,7 +1497,7 @@ cudaError_t launch_cluster(const GridArgs& a, int threads, int ctas, size_t smem
 cudaError_t launch_cluster_batch(const BatchArgs& a, int threads, int k, int csize, int clusters, size_t smem,
                                  cudaStream_t s, bool after)
 {
-  const void* fn = cluster_batch_fn_for(threads, k, a.L <= 30);
+  const void* fn = cluster_batch_fn_for(threads, k, a.L <= NARROW_MAX_L);
   cudaError_t e = prepare_cluster_fn(fn, csize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[2];

@@ -496,13 +496,16 @@ __device__ __forceinline__ void stage_issue(const uint32_t* x, int lo, int hi, S
 // One tile of Horner steps, most significant limb last in `chunk`: z = y / R for the value y
 // of the limbs so far (R = 2^32), so a limb is z' = REDC(z R^2 + l) and n limbs at once
 // REDC(z R^(n+1) + l_(n-1) R^(n-1) + ... + l_1 R + l_0), the powers mod q.
-//   narrow (moduli below 2^29: widths 22 and 27)  four limbs a step; z stays lazily below
-//            4.6 q, which the reduction keeps: (4.6 q^2 + 3 q R + R) / R + q < 4.6 q;
+//   narrow (moduli q < 2^NARROW_MAX_L)  four limbs a step; z stays lazily below 4.6 q, which
+//            the reduction keeps: (4.6 q^2 + 3 q R + R) / R + q < 4.6 q;
 //   else     two limbs a step (32-bit moduli: R mod q = R - q, so the sum stays below 2^64 and
 //            its reduction below 2 q).
 // What bounds it is the multiplier pipe (a product and its reduction per limb) and, with few
 // warps, the chain through z: four limbs take four products and one reduction, one link of
 // the chain.  Cycles per limb, 12 warps on an SM: 45 -> 23, and two limbs at 32 bits 59 -> 44.
+constexpr double NARROW_Q = (double)(1ull << NARROW_MAX_L), RADIX = 4294967296.0;
+static_assert(4.6 * NARROW_Q * NARROW_Q + 3.0 * NARROW_Q * RADIX + RADIX < RADIX * RADIX, "the sum of four limbs fits");
+static_assert(4.6 * NARROW_Q / RADIX + 4.0 + 1.0 / 4096.0 < 4.6 && 4.6 * NARROW_Q < RADIX, "z stays below 4.6 q");
 __device__ __forceinline__ uint32_t horner_tile(uint32_t z, const uint32_t* chunk, int len, const ModConst& c,
                                                 bool narrow)
 {
@@ -530,7 +533,7 @@ __device__ __forceinline__ uint32_t horner_tile(uint32_t z, const uint32_t* chun
 
 // x mod q_j for the nloc moduli mods[0..nloc), into acc[] (shared).  Limbs are staged
 // most-significant tile first; Horner in Montgomery form keeps z = y * 2^-32 where y is the
-// residue of the limbs consumed so far (horner_tile).  narrow: the moduli are below 2^29 (z
+// residue of the limbs consumed so far (horner_tile).  narrow: as there (z
 // lazy until the final conversion, which is canonical: 4.6 q r2 < q 2^32).  Returns
 // false if a staging wait ran out (after waiting, bounded, for the copy still in flight).
 template <int T>
@@ -638,8 +641,8 @@ __device__ void run_pair(const uint32_t* __restrict__ limbs, const PairDesc& d, 
   uint32_t parity = 0;
 
   // ---- MGCD2: residues
-  const bool staged = residues<T>(limbs + d.u_off, d.u_len, my, nloc, st, stg, L <= 30);
-  const bool ok = residues<T>(limbs + d.v_off, d.v_len, my, nloc, acc2, stg, L <= 30) && staged;
+  const bool staged = residues<T>(limbs + d.u_off, d.u_len, my, nloc, st, stg, L <= NARROW_MAX_L);
+  const bool ok = residues<T>(limbs + d.v_off, d.v_len, my, nloc, acc2, stg, L <= NARROW_MAX_L) && staged;
 
   uint32_t kh = 0xFFFFFFFFu, kl = 0xFFFFFFFFu;
   for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
@@ -689,13 +692,13 @@ __device__ void run_pair(const uint32_t* __restrict__ limbs, const PairDesc& d, 
     kl = 0xFFFFFFFFu;
     if (one) {
       if (have) {
-        t1 = t_update(t1, c1, p, b, L <= 30);
+        t1 = t_update(t1, c1, p, b, L <= NARROW_MAX_L);
         t_key(t1, c1.q, kh, kl);
       }
     } else {
       for (uint32_t j = threadIdx.x; j < nloc; j += TT) {
         const ModConst c = my[j];
-        const uint32_t t = t_update(st[j], c, p, b, L <= 30);
+        const uint32_t t = t_update(st[j], c, p, b, L <= NARROW_MAX_L);
         st[j] = t;
         uint32_t h, l;
         t_key(t, c.q, h, l);
@@ -1103,13 +1106,13 @@ __device__ void finish_pair(const ModConst* __restrict__ mods, const PairDesc& d
 
   // ---- replay: u mod q of the surviving moduli from (u0, v0) and the (p, b) history.
   // Invariant (U, V) = s * (u_i, v_i) mod q; each step (U, V, s) <- (V p, U - b V, s p) / R.
-  // Moduli below 2^30 keep U, V, s lazily in [0, 2q) (bn V + U < 4q^2 + 2q < q 2^32, as
+  // Narrow moduli keep U, V, s lazily in [0, 2q) (bn V + U < 4q^2 + 2q < q 2^32, as
   // redc_lazy asks).  The surviving moduli are first listed in ibuf (shared, nloc words), in
   // table order, so that thread t replays survivors t, t + T, ... with every lane busy; the
   // history is read in chunks of REPLAY_CHUNK entries that the whole CTA stages into shared
   // memory (hbuf), so every step reads a broadcast from shared memory instead of waiting on a
   // global load.
-  const bool narrow = L <= 30;
+  const bool narrow = L <= NARROW_MAX_L;
   uint32_t ns;                                         // survivors, listed in ibuf
   {
     // warp w lists a contiguous range of the moduli, after the counts of the warps before it
