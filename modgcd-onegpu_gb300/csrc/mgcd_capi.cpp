@@ -465,6 +465,18 @@ int mgcd::plan_batch(mgcd_context* c, Plan& P, size_t np, const uint32_t* limbs,
 // warp more for the pair's bookkeeping (run_pair), while they fit.
 static int single_threads(uint32_t per) { return (int)std::min<uint32_t>(1024, (per + 31) / 32 * 32 + 32); }
 
+// Clusters of a shape that fit the GPU at once; 0 if none does.
+static int clusters_at_once(mgcd_context* c, int threads, int k, int csize, size_t smem)
+{
+  for (const auto& f : c->fits)
+    if (f.threads == threads && f.k == k && f.csize == csize && f.smem == smem) return f.clusters;
+  int nc = 0;
+  if (cluster_batch_max_clusters(threads, k, c->L <= NARROW_MAX_L, csize, smem, &nc) != cudaSuccess) nc = 0;
+  if (c->fits.size() >= mgcd_context::FITS) c->fits.clear();
+  c->fits.push_back({threads, k, csize, smem, nc});
+  return nc;
+}
+
 // Launch shape of a class's n pairs in a batch too small to fill the GPU: CTAs per cluster, pairs
 // per cluster and clusters within `budget` SMs, or {} to keep the class's K pairs per CTA.  The
 // pairs' loops then bound the batch, so the shape is the one with the shortest iterations,
@@ -473,7 +485,7 @@ static int single_threads(uint32_t per) { return (int)std::min<uint32_t>(1024, (
 // 32 bits and 16.5 at 27, instead of 2 x 1, 10.3 and 9.7), at least a chain of ~1,500 cycles,
 // and the exchange 900 and 150 per slot; clusters that do not fit at once run one after another.
 struct SmallShape { int cs = 0, k = 0, clusters = 0; };
-static SmallShape small_batch_shape(const mgcd_context* c, size_t n, uint32_t nq_max, int budget, bool clusters_only)
+static SmallShape small_batch_shape(mgcd_context* c, size_t n, uint32_t nq_max, int budget, bool clusters_only)
 {
   SmallShape best;
   double best_cost = 1e30;
@@ -484,11 +496,8 @@ static SmallShape small_batch_shape(const mgcd_context* c, size_t n, uint32_t nq
       const size_t need = (n + k - 1) / k;
       const int threads = k == 1 ? single_threads(per) : per <= 256 ? 256 : per <= 512 ? 512 : 1024;
       const size_t smem = cluster_batch_smem_bytes(cs, nq_max, k);
-      int nc = 0;
-      if (smem > c->smem_optin - 24576 ||
-          cluster_batch_max_clusters(threads, k, c->L <= NARROW_MAX_L, cs, smem, &nc) != cudaSuccess || nc < 1)
-        continue;
-      nc = std::min(nc, budget / cs);
+      if (smem > c->smem_optin - 24576) continue;
+      const int nc = std::min(clusters_at_once(c, threads, k, cs, smem), budget / cs);
       if (nc < 1 || (!clusters_only && (size_t)nc < need)) continue;
       const double waves = (double)((need + nc - 1) / nc);
       const double update = std::max(1500.0, std::ceil(((per + 31) / 32) / 4.0) * (k == 4 ? 564.0 : 230.0 + 60.0 * k));

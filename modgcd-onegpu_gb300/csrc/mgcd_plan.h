@@ -159,6 +159,11 @@ struct mgcd_context {
                                        // caller sets a shape, fraction or growth (mgcd_set_spread)
   bool shaped[mgcd::NSTREAMS] = {};    // classes whose shape the caller has set (mgcd_set_size_class)
   bool use_graph = false;
+  // How many clusters of a shape fit at once, as the runtime answered (it takes ~1 us a shape
+  // and a small batch asks for up to twelve per class); at most FITS of them.
+  static constexpr size_t FITS = 256;
+  struct Fit { int threads, k, csize; size_t smem; int clusters; };
+  std::vector<Fit> fits;
   int single_policy = MGCD_SINGLE_AUTO;  // launch shape of pairs that span several CTAs
   unsigned long long wait_timeout_ns = 2000000000ull;   // bound of every cross-CTA wait
   uint32_t withhold_cta = 0xFFFFFFFFu;                  // test hook (mgcd_test_withhold_cta)

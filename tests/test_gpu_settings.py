@@ -145,3 +145,16 @@ def test_small_batch_fits_the_sms(mgcd, bits):
     us, vs = _pairs(random.Random(7), bits)
     with mgcd.Device(0, 27) as dev:
         assert sum(_run(dev, us, vs)[0]) <= torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def test_shapes_do_not_depend_on_earlier_batches(mgcd):
+    """A small batch takes the same shapes and gives the same results after many uploads of
+    other sizes (the context keeps a bounded number of the runtime's answers)."""
+    rng = random.Random(8)
+    us, vs = _pairs(rng, [30000] * 5 + [9000] * 7 + [2000] * 9)
+    with mgcd.Device(0, 32) as dev:
+        first = _run(dev, us, vs)
+        for nb in range(2000, 62000, 1500):
+            a, b = _pairs(rng, [nb] * 3)
+            dev.batch_upload(*mgcd.pack_pairs(a, b))
+        assert _run(dev, us, vs) == first
