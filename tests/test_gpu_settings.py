@@ -4,6 +4,7 @@ and reruns, with exact gcds."""
 import math
 import random
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -158,3 +159,31 @@ def test_shapes_do_not_depend_on_earlier_batches(mgcd):
             a, b = _pairs(rng, [nb] * 3)
             dev.batch_upload(*mgcd.pack_pairs(a, b))
         assert _run(dev, us, vs) == first
+
+
+@pytest.mark.parametrize("L,k", [(32, 1), (32, 2), (27, 4)])
+def test_operand_alignment_several_pairs_per_cta(mgcd, L, k):
+    """Operands that start at every limb of a 16-byte line, of lengths around a staging tile's
+    1,024 limbs, on the kernels with k pairs per CTA."""
+    rng = random.Random(9)
+    us = [rng.getrandbits(32 * n) | 1 << (32 * n - 1) | 1 for n in (1, 3, 4, 5, 1023, 1024, 1025, 2049)]
+    vs = [rng.getrandbits(u.bit_length() - 5) | 1 for u in us]
+    with mgcd.Device(0, L) as dev:
+        for c in (0, 1, 2):
+            dev.set_size_class(c, 512, k, 1.0)
+        dev.set_cta_trace(True)
+        for shift in range(4):
+            gap, parts, off, places = np.zeros(shift, dtype=np.uint32), [], 0, []
+            for x in [x for p in zip(us, vs) for x in p]:
+                parts += [gap, mgcd.to_limbs(x)]
+                places.append((off + shift, len(parts[-1])))
+                off += shift + len(parts[-1])
+            o = np.array([p[0] for p in places], dtype=np.uint64)
+            n = np.array([p[1] for p in places], dtype=np.uint32)
+            g, g_off, g_len, st = dev.gcd_batch_packed(np.concatenate(parts).astype(np.uint32), o[0::2].copy(),
+                                                       n[0::2].copy(), o[1::2].copy(), n[1::2].copy())
+            assert (st == 0).all()
+            assert ((dev.batch_cta_trace()["iterations"] > 0) == (k > 1)).any()
+            for i, (u, v) in enumerate(zip(us, vs)):
+                a = int(g_off[i])
+                assert mgcd.from_limbs(g[a: a + int(g_len[i])]) == math.gcd(u, v), (shift, i)
