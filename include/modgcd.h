@@ -219,11 +219,12 @@ int mgcd_get_class_cluster(const mgcd_context *ctx, int cls, int *ctas);
 /* Tuning table (the autotuner's output, modgcd-onegpu_gb300/tune.py): a text file with one
    line per size class, "class threads k nq_scale cluster_ctas" (cluster_ctas 0 except for
    class 3), '#' comments.  Load checks every line before applying any (MGCD_ERR_INVALID_ARG
-   for a missing file or a bad line); save writes the context's current table. */
+   for a missing file or a bad line) and leaves mgcd_set_spread as it is; save writes the
+   context's current table. */
 int mgcd_load_tuning(mgcd_context *ctx, const char *path);
 int mgcd_save_tuning(const mgcd_context *ctx, const char *path);
-/* Records the GPU work of a batch (status reset, queue resets, one persistent kernel per
-   size class on its own stream) into a CUDA graph at the first mgcd_batch_run after an
+/* Records the GPU work of a batch (the results' reset, one persistent kernel per size class,
+   chained on one stream) into a CUDA graph at the first mgcd_batch_run after an
    upload; every later mgcd_batch_run of the same upload is one graph launch.  The graph
    is rebuilt after the next upload (or a change of the wait bound); enable = 0 returns to
    direct launches.  Per-kernel times (mgcd_batch_kernel_stats) exist only for direct
@@ -251,11 +252,12 @@ int mgcd_batch_transfer_bytes(const mgcd_context *ctx, uint64_t *h2d, uint64_t *
 int mgcd_int_peak(mgcd_context *ctx, double *int_ops_per_s);
 /* Certifies, on this device, the float-reciprocal quotient steps of the modular inverse
    for every operand pair they can see (replaces certifyQuoRemQuasi.cu:25-48, which checks
-   the reference's quoRem<QUASI> per device): the estimate must be the true quotient or one
-   less, so that the single exact correction step is always right.  The estimate is
-   monotone in the dividend for a fixed divisor, so checking both ends of every quotient
-   interval of every divisor covers all pairs: *checked end points (about 6e10), *failures
-   of them (0 on a certified device), the first failing (r0, r1). */
+   the reference's quoRem<QUASI> per device): the estimate must be the quotient's floor or one
+   more (the quotient itself at multiples of the divisor) and the signed remainder exact, so
+   that every step shrinks the larger operand.  The estimate is monotone in the dividend for
+   a fixed divisor, so checking both ends of every quotient interval of every divisor covers
+   all pairs: *checked end points (about 1.4e11), *failures of them (0 on a certified
+   device), the first failing (r0, r1). */
 int mgcd_certify_inverse(mgcd_context *ctx, uint64_t *checked, uint64_t *failures, uint32_t *first_r0,
                          uint32_t *first_r1);
 

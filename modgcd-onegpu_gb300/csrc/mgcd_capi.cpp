@@ -703,7 +703,7 @@ static bool on_grid(const mgcd_context* c, uint32_t nq)
   return c->single_policy == MGCD_SINGLE_REFERENCE_SHAPE || nq > (uint32_t)MAX_CLUSTER * 1024;
 }
 
-// Launches the buckets (one stream each, joined back into P.stream) and then the
+// Launches the buckets (chained on P.stream, side by side) and then the
 // single-pair launches.  `pairs` is the descriptor array on the device, `queue_base` the
 // first of the bucket work counters (zeroed by the caller).
 static int launch_set(mgcd_context* c, Plan& P, const std::vector<Bucket>& buckets,

@@ -661,7 +661,8 @@ __global__ void __launch_bounds__(T, K < 8 ? 1024 / T : 1) batchk_kernel(const B
                               ss.lu[s], ss.lv[s], 0u, a.digits, a.count + pi, a.status + pi, a.inv, smem, acc2,
                               a.phases ? &phs[PH_REPLAY] : nullptr);
       }
-      if (RING && threadIdx.x == 0) stream_done(a, ss.seq[s]);   // results written by this thread
+      // (the digits are other lanes', ordered before this by the barrier that ends a finish)
+      if (RING && threadIdx.x == 0) stream_done(a, ss.seq[s]);
       __syncthreads();
       valid &= ~(1u << s);
       redux &= ~(1u << s);
@@ -727,8 +728,8 @@ __global__ void __launch_bounds__(T, K < 8 ? 1024 / T : 1) batchk_kernel(const B
     }
     // with K <= MGCD_PREFETCH_MAX_K, each position's constants are loaded one round ahead (a
     // global load from a table that the shared memory leaves little L1 for: its latency
-    // overlaps a round's update); the K = 4 loop has no registers to spare for them (mixed
-    // batch: none 72.6 ms, K <= 2 72.1, every K 75.6: the K = 4 loop's spills double)
+    // overlaps a round's update); with K = 4 the registers they take cost more (mixed batch:
+    // K <= 2 49.7 ms, every K 50.5)
     constexpr bool PREFETCH = K <= MGCD_PREFETCH_MAX_K;
     ModConst cn{};
     if constexpr (PREFETCH) cn = a.mods[pmod[threadIdx.x < npos ? threadIdx.x : 0u]];
